@@ -36,10 +36,10 @@ constexpr int kBatchWarps = kBatchBlock / 32;
 constexpr int kBatchMinBlocks = 3;  // 256 threads x 3 CTAs: at most 85 registers
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;
 
-// Resident 256-thread CTAs per SM the phased face kernel is compiled for (5: at most 51
-// registers; its shared memory, 15 KB per CTA, allows more).
+// Resident 128-thread CTAs per SM the phased face kernel is compiled for (8: at most 64
+// registers; its shared memory, 13 KB per CTA, allows more).
 #ifndef AXR_FACE_MIN_BLOCKS
-#define AXR_FACE_MIN_BLOCKS 5
+#define AXR_FACE_MIN_BLOCKS 8
 #endif
 
 // Resident 256-thread CTAs per SM the phased tile kernel is compiled for (4: at most 64
@@ -293,16 +293,6 @@ __device__ __forceinline__ void vertex_unit(const DrawParams& p, const UnitInfo&
     if (i < p.mesh.num_vertices) vertex_one<S>(p, i);
 }
 
-// kCoherent: the vertex cache was written earlier in the same launch
-template <bool kCoherent>
-__device__ __forceinline__ void face_unit(const DrawParams& p, const UnitInfo& ui, DevCounters* c, bool stats) {
-    GeomStats st = {0, 0, 0, 0};
-    uint32_t single_tile = kNoTile;
-    const uint32_t o = ui.local * kFaceUnit + threadIdx.x;
-    if (o < p.mesh.num_drawn) geometry_one<kCoherent>(p, o, st, single_tile);
-    geometry_warp_tail(p.target, c, stats, st, single_tile);
-}
-
 // Large-triangle tile items of all draws, strided over every warp of the grid (items are
 // alike, 256 pixels each, so a static split balances without a shared counter).
 __device__ __forceinline__ void large_items(const BatchParams& bp, bool stats) {
@@ -397,6 +387,7 @@ __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) batch_kernel(con
     __shared__ UnitInfo s_u[2];
     __shared__ __align__(128) uint32_t s_stage[kBatchWarps][2 * 512];  // warp: 2 x (colour | depth)
     __shared__ uint8_t s_list[kBatchWarps][256];
+    __shared__ __align__(16) FaceSmem<kBatchBlock> s_face;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool stats = bp.collect_stats != 0;
     BatchProfile* prof = bp.prof;
@@ -412,7 +403,7 @@ __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) batch_kernel(con
     for (uint32_t u = blockIdx.x; u < bp.face_units; u += gridDim.x, buf ^= 1) {
         stage_unit(bp, face_base + u, &s_p[buf], &s_u[buf]);
         __syncthreads();
-        face_unit<true>(s_p[buf], s_u[buf], bp.counters, stats);
+        face_cta<true>(s_p[buf], s_u[buf].local * kFaceUnit, kFaceUnit, bp.counters, stats, s_face);
     }
     if (!grid_barrier(bp.counters, prof, 1)) return;
     large_items(bp, stats);
@@ -437,16 +428,13 @@ __global__ void __launch_bounds__(kBatchBlock) batch_vertex_kernel(const __grid_
     vertex_unit<S>(s_p, s_u);
 }
 
-__global__ void __launch_bounds__(kBatchBlock, AXR_FACE_MIN_BLOCKS) batch_face_kernel(const __grid_constant__ BatchParams bp) {
+__global__ void __launch_bounds__(kPhasedFaceUnit, AXR_FACE_MIN_BLOCKS) batch_face_kernel(const __grid_constant__ BatchParams bp) {
     __shared__ __align__(16) DrawParams s_p;
     __shared__ UnitInfo s_u;
-    __shared__ FaceJob s_jobs[kBatchBlock];
-    __shared__ uint32_t s_count;
-    if (threadIdx.x == 0) s_count = 0u;
+    __shared__ __align__(16) FaceSmem<(int)kPhasedFaceUnit> s_face;
     stage_unit(bp, bp.vert_units + blockIdx.x, &s_p, &s_u);
     __syncthreads();
-    geometry_compacted(s_p, s_u.local * kFaceUnit + threadIdx.x, bp.counters, bp.collect_stats != 0, s_jobs,
-                       &s_count);
+    face_cta<false>(s_p, s_u.local * bp.face_unit, bp.face_unit, bp.counters, bp.collect_stats != 0, s_face);
 }
 
 __global__ void __launch_bounds__(kBatchBlock) batch_large_kernel(const __grid_constant__ BatchParams bp) {
@@ -643,7 +631,7 @@ cudaError_t launch_batch_s(const BatchParams& bp, int form, int num_sms, cudaStr
         if ((e = mark(1)) != cudaSuccess) return e;
         if (bp.vert_units) batch_vertex_kernel<S><<<bp.vert_units, kBatchBlock, 0, stream>>>(bp);
         if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(2)) != cudaSuccess) return e;
-        if (bp.face_units) batch_face_kernel<<<bp.face_units, kBatchBlock, 0, stream>>>(bp);
+        if (bp.face_units) batch_face_kernel<<<bp.face_units, kPhasedFaceUnit, 0, stream>>>(bp);
         if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(3)) != cudaSuccess) return e;
         // 16 CTAs per SM, about three waves of the 5 resident: the items are strided over
         // all warps of the grid, and the later waves even out the first waves' tails (5 per SM

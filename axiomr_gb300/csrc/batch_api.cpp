@@ -174,11 +174,12 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
     const int form = ctx->batch_form;
     const uint32_t tiles_per_warp = form == kFormPersistent ? kPersistentTilesPerWarp : kPhasedTilesPerWarp;
     const uint32_t tile_unit = kUnitWarps * tiles_per_warp;
+    const uint32_t face_unit = form == kFormPhased ? face_share(faces, ctx->cfg.num_sms) : kFaceUnit;
     size_t total_units = 0;
     for (int32_t i = 0; i < count; ++i) {
         const axr_draw_desc& d = draws[i];
         const bool drawn = d.mesh->num_drawn > 0;
-        total_units += (drawn ? ceil_div(d.mesh->num_vertices, kVertUnit) : 0u) + ceil_div(d.mesh->num_drawn, kFaceUnit);
+        total_units += (drawn ? ceil_div(d.mesh->num_vertices, kVertUnit) : 0u) + ceil_div(d.mesh->num_drawn, face_unit);
         if (binned)
             total_units += (uint64_t)bplan[(size_t)i].bins_x * bplan[(size_t)i].bins_y;
         else if (drawn || (d.clear_flags & (AXR_DRAW_CLEAR_COLOR | AXR_DRAW_CLEAR_DEPTH)))
@@ -298,7 +299,7 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
             bd.clear_depth = d.clear_depth;
             const bool drawn = m->num_drawn > 0;
             const uint32_t nv = drawn ? ceil_div(m->num_vertices, kVertUnit) : 0u;
-            const uint32_t nf = ceil_div(m->num_drawn, kFaceUnit);
+            const uint32_t nf = ceil_div(m->num_drawn, face_unit);
             const uint32_t nt = binned ? (uint32_t)p.bins.bins_x * p.bins.bins_y
                                 : (drawn || bd.flags & (kBatchClearColor | kBatchClearDepth))
                                     ? ceil_div((uint64_t)fb->tiles_x * fb->tiles_y, tile_unit)
@@ -340,6 +341,7 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
             bp.large_cap = large_cap;
             bp.item_cap = item_cap;
             bp.tiles_per_warp = tiles_per_warp;
+            bp.face_unit = face_unit;
             if (binned)
                 bp.bins = BinSet{d_bin_counters[set],
                                  reinterpret_cast<uint32_t*>(d_bin_counters[set] + 1) + group_bin_at[set], d_crec[set],

@@ -10,7 +10,7 @@
 //   vertex caches         per draw: vscreen[V] float4 + vattr[n*V] float4 (n = VAttr<S>::n)
 //                         + shading records (kRecFloat4 float4 per face in draw order)
 //   LargeTri[large_cap], large_draw[large_cap], LargeItem[item_cap]: shared by all draws
-// Work units: 256 vertices (vertex phase), 256 faces in draw order (geometry phase),
+// Work units: 256 vertices (vertex phase), up to 256 faces in draw order (geometry phase),
 // 8 x tiles_per_warp tiles of 16x16 (key-scan + shade phase); the large-triangle phase
 // takes items from the shared list.
 #pragma once
@@ -31,7 +31,9 @@ constexpr uint32_t kBatchTma = 4u;         // the tensor maps are valid (width %
 constexpr uint32_t kBatchClearedApart = 8u; // phased form: the clear kernel writes both planes
 
 constexpr uint32_t kVertUnit = 256;
-constexpr uint32_t kFaceUnit = 256;
+constexpr uint32_t kFaceUnit = 256;        // persistent and binned forms
+constexpr uint32_t kPhasedFaceUnit = 128;  // phased form (threads of its face kernel): at most this,
+                                           // fewer in a batch of few faces (face_share)
 constexpr uint32_t kUnitWarps = 8;  // warps of a 256-thread CTA
 constexpr uint32_t kClearUnit = 1u << 16;  // pixels per unit of the phased form's clear kernel
 
@@ -79,8 +81,21 @@ struct BatchParams {
     uint32_t large_cap, item_cap;
     int32_t collect_stats;
     uint32_t tiles_per_warp;      // tiles a warp takes per tile unit (unit = 8 warps x this)
+    uint32_t face_unit;           // faces per face unit
     BinSet bins;                  // binned form: the launch set's bin counts and clipped records
 };
+
+// Faces per CTA of a face launch over `faces` faces with CTAs of kPhasedFaceUnit threads: one
+// per thread where that gives every SM four CTAs or more; otherwise fewer, so that a small
+// draw's setup chains run side by side on all SMs and each CTA's threads share the pixels of
+// its few boxes (frames, us, at 16 / 128 faces per CTA: 4k-triangle sphere 30.8 / 36.9, 200k
+// triangles 148 / 119, 2M triangles 322 / 102).
+constexpr uint32_t kMinFaceShare = 16;
+inline uint32_t face_share(uint64_t faces, int num_sms) {
+    uint32_t n = kPhasedFaceUnit;
+    while (n > kMinFaceShare && faces < 4ull * (uint64_t)num_sms * n) n /= 2;
+    return n;
+}
 
 // Launch forms of a batch (chosen per batch by the autotuner):
 //   kFormPersistent  one cooperative launch: the four phases behind grid barriers

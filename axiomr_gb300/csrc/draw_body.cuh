@@ -46,7 +46,7 @@ struct GeomStats {
 // written. Walks the box the way the reference's tile raster does: per 16-pixel tile
 // column and row, the row start (a*(sx+0.5) + b*(py+0.5)) + c and its 8-pixel step are
 // computed once, then each pixel adds a*lane (eval_pixel gives the same bits per pixel).
-__device__ bool raster_box(const DevTarget& t, const Edges& e, uint32_t tag, GeomStats& st) {
+__device__ __forceinline__ bool raster_box(const DevTarget& t, const Edges& e, uint32_t tag, GeomStats& st) {
     bool wrote = false;
     for (int tx = e.x_lo >> 4; tx <= (e.x_hi - 1) >> 4; ++tx) {
         const int sx = max(tx * kTile, e.x_lo);
@@ -81,6 +81,11 @@ __device__ bool raster_box(const DevTarget& t, const Edges& e, uint32_t tag, Geo
         }
     }
     return wrote;
+}
+
+// The same out of line, for the rare paths.
+__device__ __noinline__ bool raster_box_call(const DevTarget& t, const Edges& e, uint32_t tag, GeomStats& st) {
+    return raster_box(t, e, tag, st);
 }
 
 __device__ __forceinline__ uint32_t tiles_of(const Edges& e, uint32_t& ntx) {
@@ -160,37 +165,16 @@ __device__ __forceinline__ uint32_t load_record(const DrawParams& p, uint32_t or
     return material;
 }
 
-// One triangle that survived clipping: cull, set up, then rasterise it here or queue its
-// tiles. *single_tile receives the one tile a small triangle wrote to (the caller marks
-// it after deduplicating across the warp); boxes spanning several tiles are marked here.
-// An unclipped triangle that can win a pixel leaves its shading record (face f, material).
-__device__ void emit_triangle(const DrawParams& p, const Screen& s, uint32_t tag, GeomStats& st,
-                              uint32_t* single_tile, const uint3& f, uint32_t material) {
-    if (is_backface(s)) return;
-    ++st.tris;
-    Edges e;
-    if (!edge_setup(s, p.target.width, p.target.height, e)) return;
-    const int npx = (e.x_hi - e.x_lo) * (e.y_hi - e.y_lo);
-    const bool record = (tag & 8u) == 0u && npx >= kRecMinPixels;
-    if (record) tag |= kRecTag;
+// A box that goes to the large-triangle pass: its setup record and one item per 16x16 tile
+// (or, with the lists full, its pixels in this thread). Unclipped triangles leave their
+// shading record at the caller.
+__device__ __forceinline__ void emit_large(const DrawParams& p, const Edges& e, uint32_t tag, GeomStats& st) {
     DevCounters* c = p.scratch.counters;
-    if (npx <= p.small_max_pixels) {
-        if (raster_box(p.target, e, tag, st)) {
-            if (record) store_record(p, tag >> 4, e, material, f);
-            uint32_t ntx;
-            if (tiles_of(e, ntx) == 1u && *single_tile == kNoTile)
-                *single_tile = tile_of(p.target, e.x_lo, e.y_lo);
-            else
-                mark_box(p.target, e);
-        }
-        return;
-    }
     uint32_t ntx;
     const uint32_t nt = tiles_of(e, ntx);
     const uint32_t slot = atomicAdd(&c->large_count, 1u);
     const uint32_t base = atomicAdd(&c->item_count, nt);
     const uint32_t icap = p.scratch.item_cap;
-    if (record) store_record(p, tag >> 4, e, material, f);
     if (slot < p.scratch.large_cap && base + nt <= icap && base + nt > base) {
         store_large(&p.scratch.large[slot], e, tag);
         if (p.scratch.large_draw) p.scratch.large_draw[slot] = p.draw;
@@ -199,10 +183,13 @@ __device__ void emit_triangle(const DrawParams& p, const Screen& s, uint32_t tag
     } else {
         // lists full: mark the reserved items empty and rasterise the triangle here
         for (uint32_t k = base; k < icap && k - base < nt; ++k) p.scratch.items[k] = LargeItem{kNoItem, 0u};
-        if (raster_box(p.target, e, tag, st)) mark_box(p.target, e);
+        GeomStats here = {0, 0, 0, 0};
+        const Edges copy = e;  // for the call: e itself stays in registers
+        if (raster_box_call(p.target, copy, tag, here)) mark_box(p.target, copy);
+        st.frags += here.frags;
+        st.tested += here.tested;
     }
 }
-
 
 // IShader::vertex of vertex i plus its screen position, NDC depth and clip-plane masks
 // (the per-vertex part of the reference's Triangle ctor, src/tiled_pipeline.cpp:53-72).
@@ -216,10 +203,13 @@ __device__ __forceinline__ void vertex_one(const DrawParams& p, uint32_t i) {
     pack_vsout<S>(vertex_shader<S>(p.u, v), &p.scratch.vattr[(size_t)VAttr<S>::n * i]);
 }
 
-// A face whose vertices straddle the clip volume: the clipper's output triangles, each
-// emitted with its clip index in the tag and its tile marked here.
-__device__ __noinline__ void geometry_clipped(const DrawParams& p, uint32_t o, const uint3 f, uint32_t material,
-                                              GeomStats& st) {
+// A face whose vertices straddle the clip volume: the clipper's output triangles, each culled,
+// set up and, with its clip index in the tag, rasterised here (boxes of at most
+// kClippedThreadPixels: such faces are few and far between) or sent to the large-triangle pass.
+constexpr int kClippedThreadPixels = 8;
+
+__device__ __noinline__ void geometry_clipped(const DrawParams& p, uint32_t o, GeomStats& st) {
+    const uint3 f = load_face(p.mesh, face_of(p.mesh, o).face);
     CVClip a[kMaxClipVerts], b[kMaxClipVerts];
     a[0].clip = load_clip(p.mesh, p.u.mvp, f.x);
     a[1].clip = load_clip(p.mesh, p.u.mvp, f.y);
@@ -229,99 +219,16 @@ __device__ __noinline__ void geometry_clipped(const DrawParams& p, uint32_t o, c
     for (int j = 0; 3 * j + 2 < n; ++j) {
         Screen s;
         screen_setup(out[3 * j].clip, out[3 * j + 1].clip, out[3 * j + 2].clip, p.target.width, p.target.height, s);
-        uint32_t tile = kNoTile;
-        emit_triangle(p, s, (o << 4) | 8u | (uint32_t)j, st, &tile, f, material);
-        if (tile != kNoTile) mark_tile(p.target, tile);
+        if (is_backface(s)) continue;
+        ++st.tris;
+        Edges e;
+        if (!edge_setup(s, p.target.width, p.target.height, e)) continue;
+        const uint32_t tag = (o << 4) | 8u | (uint32_t)j;
+        if ((e.x_hi - e.x_lo) * (e.y_hi - e.y_lo) > min(p.small_max_pixels, kClippedThreadPixels))
+            emit_large(p, e, tag, st);
+        else if (raster_box_call(p.target, e, tag, st))
+            mark_box(p.target, e);
     }
-}
-
-// Face at draw-order position o (< num_drawn): clip classification, cull, setup and
-// raster or queueing (src/tiled_pipeline.cpp:195-240, 436-487).
-// kCoherent: the vertex cache was written earlier in the same launch (plain loads).
-template <bool kCoherent = false>
-__device__ __forceinline__ void geometry_one(const DrawParams& p, uint32_t o, GeomStats& st, uint32_t& single_tile) {
-    if (o > kMaxOrdinal) {
-        atomicOr(&p.scratch.counters->error, kErrOrdinal);
-        return;
-    }
-    const FaceRef fr = face_of(p.mesh, o);
-    const uint3 f = load_face(p.mesh, fr.face);
-    const uint32_t nv = p.mesh.num_vertices;
-    if (f.x >= nv || f.y >= nv || f.z >= nv) {
-        atomicOr(&p.scratch.counters->error, kErrIndex);
-        return;
-    }
-    const float4* vs = p.scratch.vscreen;
-    const float4 g0 = ld_cached<kCoherent>(&vs[f.x]), g1 = ld_cached<kCoherent>(&vs[f.y]),
-                 g2 = ld_cached<kCoherent>(&vs[f.z]);
-    const int cls = classify_masks(__float_as_uint(g0.w), __float_as_uint(g1.w), __float_as_uint(g2.w));
-    if (cls == 3) {
-        Screen s;
-        s.x[0] = g0.x; s.y[0] = g0.y; s.z[0] = g0.z;
-        s.x[1] = g1.x; s.y[1] = g1.y; s.z[1] = g1.z;
-        s.x[2] = g2.x; s.y[2] = g2.y; s.z[2] = g2.z;
-        screen_bbox(s);
-        emit_triangle(p, s, o << 4, st, &single_tile, f, fr.material);
-    } else if (cls < 0) {
-        geometry_clipped(p, o, f, fr.material, st);
-    }
-}
-
-// A front-facing face inside the clip volume, queued by geometry_front for the setup and
-// raster pass of the compacted face phase.
-struct FaceJob {
-    float x[3], y[3], z[3];
-    uint32_t o, material;
-    uint32_t f[3];
-};
-
-// The first half of geometry_one for the compacted face phase: the checks, the vertex-cache
-// gathers, clip classification and the back-face test. A face that straddles the clip
-// volume is finished here; one inside it that faces the camera is returned in *job (true)
-// for emit_triangle in a second pass, where every lane of a warp has such a face.
-template <bool kCoherent>
-__device__ __forceinline__ bool geometry_front(const DrawParams& p, uint32_t o, GeomStats& st, FaceJob& job) {
-    if (o > kMaxOrdinal) {
-        atomicOr(&p.scratch.counters->error, kErrOrdinal);
-        return false;
-    }
-    const FaceRef fr = face_of(p.mesh, o);
-    const uint3 f = load_face(p.mesh, fr.face);
-    const uint32_t nv = p.mesh.num_vertices;
-    if (f.x >= nv || f.y >= nv || f.z >= nv) {
-        atomicOr(&p.scratch.counters->error, kErrIndex);
-        return false;
-    }
-    const float4* vs = p.scratch.vscreen;
-    const float4 g0 = ld_cached<kCoherent>(&vs[f.x]), g1 = ld_cached<kCoherent>(&vs[f.y]),
-                 g2 = ld_cached<kCoherent>(&vs[f.z]);
-    const int cls = classify_masks(__float_as_uint(g0.w), __float_as_uint(g1.w), __float_as_uint(g2.w));
-    if (cls == 3) {
-        Screen s;
-        s.x[0] = g0.x; s.y[0] = g0.y; s.z[0] = g0.z;
-        s.x[1] = g1.x; s.y[1] = g1.y; s.z[1] = g1.z;
-        s.x[2] = g2.x; s.y[2] = g2.y; s.z[2] = g2.z;
-        if (is_backface(s)) return false;
-        job = FaceJob{{s.x[0], s.x[1], s.x[2]}, {s.y[0], s.y[1], s.y[2]}, {s.z[0], s.z[1], s.z[2]},
-                      o, fr.material, {f.x, f.y, f.z}};
-        return true;
-    }
-    if (cls < 0) geometry_clipped(p, o, f, fr.material, st);
-    return false;
-}
-
-// The second half: setup and raster (or queueing) of a queued face, as geometry_one does.
-__device__ __forceinline__ void geometry_job(const DrawParams& p, const FaceJob& j, GeomStats& st,
-                                             uint32_t& single_tile) {
-    Screen s;
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        s.x[k] = j.x[k];
-        s.y[k] = j.y[k];
-        s.z[k] = j.z[k];
-    }
-    screen_bbox(s);
-    emit_triangle(p, s, j.o << 4, st, &single_tile, make_uint3(j.f[0], j.f[1], j.f[2]), j.material);
 }
 
 // Warp-wide end of the geometry step: one mark per distinct single tile in the warp, and
@@ -343,35 +250,246 @@ __device__ __forceinline__ void geometry_warp_tail(const DevTarget& t, DevCounte
     }
 }
 
-// One CTA's faces in two passes (every thread calls it with its face o; *count is zero on
-// entry; `jobs` holds one entry per thread): geometry_front per face, then geometry_job on
-// the front-facing faces inside the clip volume. When fewer than three quarters of the
-// CTA's faces go on (a closed mesh turns about half of its faces away), they are first
-// compacted into `jobs` by warp ballots, so that the second pass runs with every lane
-// busy instead of idling the culled faces' lanes through their neighbours' raster loops;
-// otherwise each thread goes on with its own face (the shared-memory round trip would
-// cost more than the idle lanes).
-__device__ __forceinline__ void geometry_compacted(const DrawParams& p, uint32_t o, DevCounters* c, bool stats,
-                                                   FaceJob* jobs, uint32_t* count) {
+// ---- the face phase: setup by face, raster by pixel
+//
+// Each thread sets up a face and rasterises a box of at most kThreadPixels pixels itself. The
+// pixels of larger boxes (up to p.small_max_pixels) are numbered one box after another over
+// a group of threads, a warp or the CTA, and the group's threads share these (triangle, pixel)
+// pairs evenly. Boxes differ by two orders of magnitude within a warp and about half of a
+// closed mesh's faces are culled, so a thread per triangle left 8 to 18 of 32 lanes at work
+// (ncu: 8.4 on a 4k-triangle sphere, 8.6 on 200k small triangles, 12.3 on the mixed batch)
+// behind the warp's largest box. Bound: issue and the gathers' latency. Frames, before and
+// after: 4k-triangle sphere at 512x512 60 to 31 us, 2M-triangle terrain at 1920x1080 109 to
+// 103, 200k triangles at 3840x2160 133 to 127, 30 mixed draws in a batch 220 to 192; all pixels
+// by pairs instead (no box in its own thread) left the terrain, most of whose boxes hold 2 to 6
+// pixels, at 129.
+constexpr int kWarpPairs = 2048;     // pairs a warp's share of the tables holds; boxes past a
+                                     // group's tables go to the large-triangle list
+constexpr int kThreadPixels = 6;  // boxes a thread rasterises itself (at most 8)
+
+template <int kThreads>
+struct FaceSmem {
+    float4 job[kThreads][5];                         // store_job, 80 bytes: no bank conflicts
+    uint32_t start[kThreads / 32 * kWarpPairs / 32]; // bit k: pair k is the first of its box
+    uint16_t owner[kThreads / 32 * kWarpPairs / 32]; // the box that holds pair 32 w
+    uint32_t warp_sum[kThreads / 32];
+    uint32_t end;                                       // pairs to rasterise (when they exceed the tables)
+};
+
+// Small non-negative integers as floats without the conversion unit (2^23 + v has v in its
+// low mantissa bits): v, and v + 1/2 (2^23 - 1/2 is a float), both exact.
+__device__ __forceinline__ float small_float(int v) { return __int_as_float(0x4B000000 | v) - 8388608.0f; }
+__device__ __forceinline__ float small_centre(int v) { return __int_as_float(0x4B000000 | v) - 8388607.5f; }
+
+__device__ __forceinline__ void store_job(float4* j, const Edges& e, uint32_t tag, uint32_t first) {
+    const uint32_t w = (uint32_t)(e.x_hi - e.x_lo);
+    j[0] = make_float4(e.a[0], e.b[0], e.c[0], e.a[1]);
+    j[1] = make_float4(e.b[1], e.c[1], e.a[2], e.b[2]);
+    j[2] = make_float4(e.c[2], e.inv_area, e.z[0], e.z[1]);
+    j[3] = make_float4(e.z[2], __uint_as_float((uint32_t)e.x_lo | ((uint32_t)e.y_lo << 16)), __uint_as_float(tag),
+                       __uint_as_float(first | (w << 16)));
+}
+
+// A box of at most 8 pixels in this thread (the 8-pixel step of eval_pixel never comes up);
+// returns whether a key was written.
+__device__ __forceinline__ bool raster_tiny(const DevTarget& t, const Edges& e, uint32_t tag, uint32_t npx, GeomStats& st) {
+    bool wrote = false;
+    int px = e.x_lo, py = e.y_lo;
+    st.tested += npx;
+    for (uint32_t q = 0; q < npx; ++q) {
+        const int sx = max(px & ~(kTile - 1), e.x_lo);
+        const float fsx = small_centre(sx), fpy = small_centre(py), lane = small_float(px - sx);
+        float cov[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            cov[k] = fadd(fadd(fadd(fmul(e.a[k], fsx), fmul(e.b[k], fpy)), e.c[k]), fmul(e.a[k], lane));
+        if (cov[0] >= 0.f && cov[1] >= 0.f && cov[2] >= 0.f) {
+            ++st.frags;
+            const float al = fmul(cov[0], e.inv_area), be = fmul(cov[1], e.inv_area), ga = fmul(cov[2], e.inv_area);
+            wrote |= write_key(t, px, py, fadd(fadd(fmul(e.z[0], al), fmul(e.z[1], be)), fmul(e.z[2], ga)), tag);
+        }
+        if (++px == e.x_hi) {
+            px = e.x_lo;
+            ++py;
+        }
+    }
+    return wrote;
+}
+
+// Pair k: coverage and depth of one pixel of the box `j`, in eval_pixel's operations. first
+// and w (both at most 16384) share a word; the row is the floor of (q + 1/2) / w, q < 16384
+// pixels into the box: an approximate reciprocal is off by less than q / w * 2^-22, and no
+// exact value is nearer than 1 / (2 w) to an integer, so the truncation is the quotient.
+__device__ __forceinline__ void raster_pair(const DevTarget& t, const float4* j, uint32_t k, GeomStats& st) {
+    const float4 v0 = j[0], v1 = j[1], v2 = j[2], v3 = j[3];
+    const uint32_t xy = __float_as_uint(v3.y), fw = __float_as_uint(v3.w);
+    const uint32_t w = fw >> 16, q = k - (fw & 0xFFFFu);
+    const uint32_t row = (uint32_t)__float2int_rz(small_centre((int)q) * crcp(small_float((int)w)));
+    const int x_lo = (int)(xy & 0xFFFFu);
+    const int px = x_lo + (int)(q - row * w), py = (int)((xy >> 16) + row);
+    const int sx = max(px & ~(kTile - 1), x_lo), i = px - sx;
+    const float fsx = small_centre(sx), fpy = small_centre(py), lane = small_float(i & 7);
+    const float a[3] = {v0.x, v0.w, v1.z}, b[3] = {v0.y, v1.x, v1.w}, c[3] = {v0.z, v1.y, v2.x};
+    float cov[3];
+#pragma unroll
+    for (int n = 0; n < 3; ++n) {
+        float r = fadd(fadd(fmul(a[n], fsx), fmul(b[n], fpy)), c[n]);
+        if (i >= 8) r = fadd(r, fmul(a[n], 8.0f));
+        cov[n] = fadd(r, fmul(a[n], lane));
+    }
+    if (cov[0] >= 0.f && cov[1] >= 0.f && cov[2] >= 0.f) {
+        ++st.frags;
+        const float al = fmul(cov[0], v2.y), be = fmul(cov[1], v2.y), ga = fmul(cov[2], v2.y);
+        write_key(t, px, py, fadd(fadd(fmul(v2.z, al), fmul(v2.w, be)), fmul(v3.x, ga)), __float_as_uint(v3.z));
+    }
+}
+
+// Checks, vertex-cache gathers, clip classification, cull and setup of the face at draw-order
+// position o. One inside the clip volume that faces the camera and has a pixel box is returned
+// (true) with its depth-key tag, its shading record stored; `cut`: it straddles the volume (for
+// geometry_clipped). kCoherent: the vertex cache was written earlier in the same launch (plain loads).
+template <bool kCoherent>
+__device__ __forceinline__ bool face_setup(const DrawParams& p, uint32_t o, GeomStats& st, Edges& e, uint32_t& tag,
+                                           bool& cut) {
+    if (o > kMaxOrdinal) {
+        atomicOr(&p.scratch.counters->error, kErrOrdinal);
+        return false;
+    }
+    const FaceRef fr = face_of(p.mesh, o);
+    const uint3 f = load_face(p.mesh, fr.face);
+    const uint32_t nv = p.mesh.num_vertices;
+    if (f.x >= nv || f.y >= nv || f.z >= nv) {
+        atomicOr(&p.scratch.counters->error, kErrIndex);
+        return false;
+    }
+    const float4* vs = p.scratch.vscreen;
+    const float4 g0 = ld_cached<kCoherent>(&vs[f.x]), g1 = ld_cached<kCoherent>(&vs[f.y]),
+                 g2 = ld_cached<kCoherent>(&vs[f.z]);
+    const int cls = classify_masks(__float_as_uint(g0.w), __float_as_uint(g1.w), __float_as_uint(g2.w));
+    cut = cls < 0;
+    if (cls != 3) return false;
+    Screen s;
+    s.x[0] = g0.x; s.y[0] = g0.y; s.z[0] = g0.z;
+    s.x[1] = g1.x; s.y[1] = g1.y; s.z[1] = g1.z;
+    s.x[2] = g2.x; s.y[2] = g2.y; s.z[2] = g2.z;
+    if (is_backface(s)) return false;
+    ++st.tris;
+    screen_bbox(s);
+    if (!edge_setup(s, p.target.width, p.target.height, e)) return false;
+    tag = o << 4;
+    if ((e.x_hi - e.x_lo) * (e.y_hi - e.y_lo) >= kRecMinPixels) {
+        tag |= kRecTag;
+        store_record(p, o, e, fr.material, f);
+    }
+    return true;
+}
+
+// The faces of a CTA, thread t's at draw-order position o (valid: it has one); a group is a
+// warp (kWarp) or the CTA. The tiles of a shared box are flagged whether or not a pixel of it turns
+// out covered (a flagged tile without keys costs the tile pass its key reads).
+template <bool kCoherent, int kThreads, bool kWarp>
+__device__ __forceinline__ void face_group(const DrawParams& p, uint32_t o, bool valid, DevCounters* c, bool stats,
+                                           FaceSmem<kThreads>& sm) {
+    constexpr int kGroupWarps = kWarp ? 1 : kThreads / 32;
+    constexpr uint32_t kCap = kGroupWarps * kWarpPairs;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int gw = kWarp ? 0 : warp, gt = kWarp ? lane : tid;  // this warp and thread in the group
+    const uint32_t table = kWarp ? (uint32_t)warp * (kWarpPairs / 32) : 0u;
+    float4(*job)[5] = sm.job + (kWarp ? 32 * warp : 0);
+    uint32_t* start = sm.start + table;
+    uint16_t* owner = sm.owner + table;
     GeomStats st = {0, 0, 0, 0};
-    uint32_t single_tile = kNoTile;
-    FaceJob job;
-    const bool queued = o < p.mesh.num_drawn && geometry_front<false>(p, o, st, job);
-    const unsigned m = __ballot_sync(0xFFFFFFFFu, queued);
-    const int lane = threadIdx.x & 31;
-    uint32_t base = 0;
-    if (lane == 0 && m) base = atomicAdd(count, (uint32_t)__popc(m));
-    base = __shfl_sync(0xFFFFFFFFu, base, 0);
-    __syncthreads();
-    const uint32_t n = *count;
-    if (4u * n >= 3u * blockDim.x) {
-        if (queued) geometry_job(p, job, st, single_tile);
-    } else {
-        if (queued) jobs[base + (uint32_t)__popc(m & ((1u << lane) - 1u))] = job;
-        __syncthreads();
-        if (threadIdx.x < n) geometry_job(p, jobs[threadIdx.x], st, single_tile);
+    uint32_t single_tile = kNoTile, tag = 0;
+    Edges e;
+    bool cut = false;
+    bool has = valid && face_setup<kCoherent>(p, o, st, e, tag, cut);
+    const uint32_t npx = has ? (uint32_t)(e.x_hi - e.x_lo) * (uint32_t)(e.y_hi - e.y_lo) : 0u;
+    bool large = npx > (uint32_t)max(p.small_max_pixels, kThreadPixels);
+    has = has && !large;
+    if (has && npx <= (uint32_t)kThreadPixels) {
+        has = false;
+        if (raster_tiny(p.target, e, tag, npx, st)) {
+            uint32_t ntx;
+            if (tiles_of(e, ntx) == 1u) single_tile = tile_of(p.target, e.x_lo, e.y_lo);
+            else mark_box(p.target, e);
+        }
+    }
+    if (!kWarp || __any_sync(0xFFFFFFFFu, has)) {
+        for (int k = gt; k < (int)kCap / 32; k += 32 * kGroupWarps) start[k] = 0u;
+        // (boxes, pairs) before this thread's: boxes above bit 23, pairs below (at most 256 * 2^14)
+        const uint32_t mine = has ? (1u << 23) | min(npx, kCap + 1u) : 0u;
+        uint32_t incl = mine;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
+            if (lane >= d) incl += v;
+        }
+        uint32_t before = incl - mine, total = 0;
+        if (kWarp) {
+            total = __shfl_sync(0xFFFFFFFFu, incl, 31);
+            if (lane == 0) sm.warp_sum[warp] = 0u;
+            __syncwarp();
+        } else {
+            if (lane == 31) sm.warp_sum[warp] = incl;
+            if (tid == 0) sm.end = 0u;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < kGroupWarps; ++w) {
+                const uint32_t v = sm.warp_sum[w];
+                if (w < warp) before += v;
+                total += v;
+            }
+        }
+        uint32_t* end = kWarp ? &sm.warp_sum[warp] : &sm.end;
+        uint32_t pairs = total & 0x7FFFFFu;
+        const bool over = pairs > kCap;
+        if (has) {
+            const uint32_t at = before & 0x7FFFFFu, rank = before >> 23;
+            large = at + npx > kCap;
+            if (!large) {
+                store_job(job[rank], e, tag, at);
+                atomicOr(&start[at >> 5], 1u << (at & 31u));
+                for (uint32_t w = (at + 31u) >> 5; (w << 5) < at + npx; ++w) owner[w] = (uint16_t)rank;
+                if (over) atomicMax(end, at + npx);
+                uint32_t ntx;
+                if (tiles_of(e, ntx) == 1u) single_tile = tile_of(p.target, e.x_lo, e.y_lo);
+                else mark_box(p.target, e);
+            }
+        }
+        if (kWarp) __syncwarp();
+        else __syncthreads();
+        if (over) pairs = *reinterpret_cast<volatile uint32_t*>(end);
+        for (uint32_t w = (uint32_t)gw; (w << 5) < pairs; w += kGroupWarps) {
+            const uint32_t k = (w << 5) + (uint32_t)lane;
+            const uint32_t rank = owner[w] + (uint32_t)__popc(start[w] & ~1u & ((2u << lane) - 1u));
+            if (k < pairs) {
+                ++st.tested;
+                raster_pair(p.target, job[rank], k, st);
+            }
+        }
+    }
+    if (large) emit_large(p, e, tag, st);
+    if (cut) {  // last: the clipper is a long chain, and the group would wait for it
+        GeomStats clipped = {0, 0, 0, 0};  // its own: no pointer to st leaves this function
+        geometry_clipped(p, o, clipped);
+        st.tris += clipped.tris;
+        st.frags += clipped.frags;
+        st.large += clipped.large;
+        st.tested += clipped.tested;
     }
     geometry_warp_tail(p.target, c, stats, st, single_tile);
+}
+
+// The CTA's faces from draw-order position `first`: a face per thread and warp groups, or
+// (faces_of_cta < threads, a draw of few faces) the first threads a face each and the pairs shared
+// by the whole CTA.
+template <bool kCoherent, int kThreads>
+__device__ __forceinline__ void face_cta(const DrawParams& p, uint32_t first, uint32_t faces_of_cta, DevCounters* c,
+                                         bool stats, FaceSmem<kThreads>& sm) {
+    const uint32_t o = first + threadIdx.x;
+    const bool valid = threadIdx.x < faces_of_cta && o < p.mesh.num_drawn;
+    if (faces_of_cta == (uint32_t)kThreads) face_group<kCoherent, kThreads, true>(p, o, valid, c, stats, sm);
+    else face_group<kCoherent, kThreads, false>(p, o, valid, c, stats, sm);
 }
 
 // Whether no pixel of 16x16 tile (tx, ty) inside the triangle's box can test covered.

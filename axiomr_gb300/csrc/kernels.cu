@@ -31,6 +31,7 @@
 #include <cstddef>
 #include <cstring>
 
+#include "batch_types.h"
 #include "draw_body.cuh"
 #include "kernels.h"
 
@@ -40,11 +41,12 @@ namespace {
 
 constexpr int kBlock = 256;
 
-// Resident 256-thread CTAs per SM the geometry kernel is compiled for (register budget
-// 65536 / (256 * n)); 5 keeps it at 48 registers.
+// Resident 128-thread CTAs per SM the geometry kernel is compiled for (register budget
+// 65536 / (128 * n)): 64 registers.
 #ifndef AXR_GEOMETRY_MIN_BLOCKS
-#define AXR_GEOMETRY_MIN_BLOCKS 5
+#define AXR_GEOMETRY_MIN_BLOCKS 8
 #endif
+
 
 template <int S>
 __global__ void __launch_bounds__(kBlock) vertex_kernel(const __grid_constant__ DrawParams p) {
@@ -52,35 +54,26 @@ __global__ void __launch_bounds__(kBlock) vertex_kernel(const __grid_constant__ 
     if (i < p.mesh.num_vertices) vertex_one<S>(p, i);
 }
 
-__global__ void __launch_bounds__(kBlock, AXR_GEOMETRY_MIN_BLOCKS) geometry_kernel(const __grid_constant__ DrawParams p) {
-    GeomStats st = {0, 0, 0, 0};
-    uint32_t single_tile = kNoTile;
-    const uint32_t o = blockIdx.x * kBlock + threadIdx.x;
-    if (o < p.mesh.num_drawn) geometry_one(p, o, st, single_tile);
-    geometry_warp_tail(p.target, p.scratch.counters, p.scratch.collect_stats != 0, st, single_tile);
+__global__ void __launch_bounds__(kPhasedFaceUnit, AXR_GEOMETRY_MIN_BLOCKS)
+    geometry_kernel(const __grid_constant__ DrawParams p, uint32_t faces_per_cta) {
+    __shared__ __align__(16) FaceSmem<(int)kPhasedFaceUnit> sm;
+    face_cta<false>(p, blockIdx.x * faces_per_cta, faces_per_cta, p.scratch.counters, p.scratch.collect_stats != 0, sm);
 }
 
 __global__ void __launch_bounds__(kBlock) large_kernel(const __grid_constant__ DrawParams p) {
     DevCounters* c = p.scratch.counters;
     const uint32_t n_items = min(ld_volatile(&c->item_count), p.scratch.item_cap);
-    if (n_items == 0) return;
     const uint32_t n_tris = min(ld_volatile(&c->large_count), p.scratch.large_cap);
     const int lane = threadIdx.x & 31;
+    const uint32_t warps = gridDim.x * (kBlock / 32);
     uint32_t frags = 0, tested = 0;
-    for (;;) {
-        uint32_t first = 0;
-        if (lane == 0) first = atomicAdd(&c->item_head, kItemsPerGrab);
-        first = __shfl_sync(0xFFFFFFFFu, first, 0);
-        if (first >= n_items) break;
-        const uint32_t last = min(first + kItemsPerGrab, n_items);
-        for (uint32_t it = first; it < last; ++it) {
-            const LargeItem item = p.scratch.items[it];
-            if (item.tri >= n_tris) continue;  // reserved slot of a triangle rasterised elsewhere
-            Edges e;
-            uint32_t tag;
-            load_large(&p.scratch.large[item.tri], e, tag);
-            large_tile(p.target, e, tag, item.tile, frags, tested);
-        }
+    for (uint32_t it = blockIdx.x * (kBlock / 32) + (threadIdx.x >> 5); it < n_items; it += warps) {
+        const LargeItem item = p.scratch.items[it];
+        if (item.tri >= n_tris) continue;  // reserved slot of a triangle rasterised elsewhere
+        Edges e;
+        uint32_t tag;
+        load_large(&p.scratch.large[item.tri], e, tag);
+        large_tile(p.target, e, tag, item.tile, frags, tested);
     }
     if (p.scratch.collect_stats) {
         uint32_t f = __reduce_add_sync(0xFFFFFFFFu, frags);
@@ -310,7 +303,8 @@ cudaError_t launch_shaded(const DrawParams& p, const LaunchConfig& cfg, cudaStre
         vertex_kernel<S><<<grid_for(p.mesh.num_vertices, kBlock, 0x7FFFFFFFu), kBlock, 0, stream>>>(p);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         if ((e = mark(1)) != cudaSuccess) return e;
-        geometry_kernel<<<grid_for(p.mesh.num_drawn, kBlock, 0x7FFFFFFFu), kBlock, 0, stream>>>(p);
+        const uint32_t share = face_share(p.mesh.num_drawn, cfg.num_sms);
+        geometry_kernel<<<grid_for(p.mesh.num_drawn, (int)share, 0x7FFFFFFFu), kPhasedFaceUnit, 0, stream>>>(p, share);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
         *launches += 2;
     } else if ((e = mark(1)) != cudaSuccess) {

@@ -1,0 +1,54 @@
+"""The face phase's two rasterisers (a thread per box of at most 6 pixels, shared (triangle,
+pixel) pairs above) and its limits against the CPU oracle: box sizes around the limits, face
+counts around a CTA's share, pair tables that overflow into the large-triangle pass."""
+import numpy as np
+import pytest
+
+from axiomr_gb300 import api
+from axiomr_gb300 import workloads as W
+from helpers import assert_parity
+
+pytestmark = pytest.mark.gpu
+
+
+def soup(count, edge, width=331, height=213, seed=21):
+    return W.soup_scene(count=count, width=width, height=height, seed=seed, edge_min=edge, edge_max=edge + 0.01,
+                        depth_min=1.0, depth_max=50.0)
+
+
+def check(ctx, port, sc, what):
+    vp = port.camera(sc.camera)[2]
+    assert_parity(api.render_scene(ctx, sc, view_proj=vp), port.draw(sc, vp), what)
+
+
+# edges from below a pixel to boxes past the 64-pixel limit, wider than an 8-pixel step and
+# than a 16-pixel tile
+@pytest.mark.parametrize("edge", [0.3, 1.0, 1.8, 3.0, 6.0, 7.0, 8.5, 17.0, 40.0])
+def test_box_sizes(ctx, port, edge):
+    check(ctx, port, soup(3000, edge), f"edge {edge}")
+
+
+# one face, around the smallest share of a CTA (16), a warp, a CTA; and past 4 CTAs of 128 on
+# each of 152 SMs, where a thread takes a face and each warp shares its own pairs
+@pytest.mark.parametrize("count", [1, 15, 16, 17, 31, 33, 127, 128, 129, 77_823, 77_825, 80_001])
+def test_face_counts(ctx, port, count):
+    check(ctx, port, soup(count, 4.0), f"{count} faces")
+
+
+# pixel-box limits whose boxes overflow a warp's table (2,048 pairs) or a CTA's (8,192)
+@pytest.mark.parametrize("limit", [0, 6, 7, 256, 1024, 65536])
+@pytest.mark.parametrize("count,edge", [(40, 60.0), (2000, 24.0), (80_000, 14.0)])
+def test_pair_tables_overflow(port, limit, count, edge):
+    ctx = api.Context(0)
+    ctx.set_tuning([limit] * 6)
+    sc = soup(count, edge)
+    vp = port.camera(sc.camera)[2]
+    draws = api.batch_draws(ctx, [sc])
+    draws[0].camera = api.Camera.from_matrices(vp, sc.camera.position, sc.camera.viewport)
+    for form in (api.BATCH_PHASED, api.BATCH_PERSISTENT):
+        ctx.batch_form = form
+        api.draw_batch(ctx, draws)
+        got = draws[0].framebuffer.read()
+        ctx.sync()
+        assert_parity(got, port.draw(sc, vp), f"limit {limit} form {form}")
+    ctx.close()
