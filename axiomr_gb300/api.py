@@ -90,7 +90,7 @@ class Context:
 
     def tuning(self) -> list:
         """The batched form's tuning table: per density class, the largest triangle pixel
-        box rasterised by one thread."""
+        box rasterised in the face phase."""
         out = (C.c_int32 * AXR_TUNE_CLASSES)()
         check(self.lib.axr_batch_get_tuning(self.handle, out), self.handle)
         return list(out)

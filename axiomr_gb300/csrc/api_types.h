@@ -69,10 +69,11 @@ struct axr_framebuffer {
 };
 
 // A planned batch (batch_api.cpp): the draw table and scratch in one device allocation,
-// and one launch description per shader kind present.
+// and one launch description per shader kind present (phased form: per launch set, its kinds
+// together).
 struct axr_batch {
     struct Launch {
-        int shader;
+        int shader;  // kMixedShaders: a phased set of several kinds
         int set;  // launch set: 0 on the context stream, 1 on the batch side stream
         axr::BatchParams params;
     };
@@ -80,6 +81,7 @@ struct axr_batch {
     void* dev = nullptr;
     size_t bytes = 0;
     std::vector<Launch> launches;
+    uint32_t kind_sets = 0;  // (shader kind, launch set) pairs with draws
     int sets = 1;                               // launch sets (phased form of a large batch: 2)
     axr::DevCounters* set_counters = nullptr;  // counters of launch set 1 (in `dev`)
     int form = 0;  // axr::kForm*
@@ -130,9 +132,10 @@ struct axr_context {
     uint32_t large_cap = 0, item_cap = 0, vcap = 0, px_cap = 0, rec_cap = 0;
     int collect_stats = 0;
     int small_max_pixels = 64;
-    // batched form: per density class, the largest pixel box rasterised per thread
-    // (autotuned), and the reusable plan of axr_draw_batch
-    int32_t tune_small[AXR_TUNE_CLASSES] = {64, 64, 64, 64, 64, 64};
+    // batched form: per density class, the largest pixel box rasterised in the face phase
+    // (autotuned; face_pixels bounds it in smaller batches), and the reusable plan of
+    // axr_draw_batch
+    int32_t tune_small[AXR_TUNE_CLASSES] = {256, 256, 256, 256, 256, 256};
     // binned batched form: bin parameters per density class (autotuned)
     axr_bin_params tune_bin[AXR_TUNE_CLASSES] = {{256, 4, 64, 2}, {256, 4, 64, 2}, {256, 4, 64, 2},
                                                  {256, 4, 64, 2}, {256, 4, 64, 2}, {256, 4, 64, 2}};

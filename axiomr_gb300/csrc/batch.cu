@@ -116,35 +116,44 @@ __device__ void profile_exit(BatchProfile* prof) {
 }
 
 // ---- the tile pass, in three steps over one 16x16 tile of draw `p`:
-//   tile_scan    (warp) keys -> pixel lists in shared memory: unclipped winners from the
-//                front of `list`, clipped ones from the back, their tags parked in the
-//                colour staging slots; keys and flag reset; pixels without a key get the
-//                requested clear (staged when both planes are cleared, else written)
-//   shade_winner (thread) one unclipped winner: fragment, merged into the staging slots
-//                or written to the framebuffer
-//   tile_finish  (warp) the clipped winners (rare), then the staged tile out with two
-//                TMA tensor stores (or plain stores when the pitch has no tensor map)
+//   tile_scan    (warp) keys -> entries (slot << 8 | pixel) in a list in shared memory:
+//                unclipped winners from its front, clipped ones from its back, their tags
+//                parked in the colour staging slots; keys and flag reset; pixels without a key
+//                get the requested clear (staged when both planes are cleared, else written)
+//   shade_winner (thread) one winner: fragment, merged into the staging slots or written to
+//                the framebuffer
+//   tile_store   (warp) the staged tile out with two TMA tensor stores (or plain stores when
+//                the pitch has no tensor map)
 // `stage` is the tile's staging buffer: colour plane [256] then depth plane [256].
+constexpr int kAnyShader = kMixedShaders;  // template argument: the draw's own shader kind, looked up per CTA
+
 struct TileCtx {
     uint32_t tile;
     int tx, ty;
     bool clear_c, clear_d, full;
 };
 
-__device__ __forceinline__ TileCtx tile_ctx(const DevTarget& t, const UnitInfo& ui, uint32_t tile) {
+__device__ __forceinline__ TileCtx tile_ctx_at(const UnitInfo& ui, uint32_t tile, int tx, int ty) {
     TileCtx c;
     c.tile = tile;
-    c.tx = (int)(tile % (uint32_t)t.tiles_x);
-    c.ty = (int)(tile / (uint32_t)t.tiles_x);
+    c.tx = tx;
+    c.ty = ty;
     c.clear_c = (ui.flags & kBatchClearColor) != 0u;
     c.clear_d = (ui.flags & kBatchClearDepth) != 0u;
     c.full = c.clear_c && c.clear_d;
     return c;
 }
 
-// Returns nwin | nclip << 16 (lane-uniform).
-__device__ uint32_t tile_scan(const DrawParams& p, const UnitInfo& ui, const TileCtx& c, bool dirty, uint32_t* stage,
-                              uint8_t* list, DevCounters* counters, bool stats) {
+__device__ __forceinline__ TileCtx tile_ctx(const DevTarget& t, const UnitInfo& ui, uint32_t tile) {
+    return tile_ctx_at(ui, tile, (int)(tile % (uint32_t)t.tiles_x), (int)(tile / (uint32_t)t.tiles_x));
+}
+
+// `cap`: entries of the list; `fill` (NULL: an empty list of the warp's own): the list's fill,
+// unclipped | clipped << 16, advanced by this tile's. Returns the tile's own counts, packed the
+// same way (lane-uniform).
+__device__ __forceinline__ uint32_t tile_scan(const DrawParams& p, const UnitInfo& ui, const TileCtx& c, bool dirty,
+                                              uint32_t* stage, uint32_t slot, uint16_t* list, uint32_t cap,
+                                              uint32_t* fill, DevCounters* counters, bool stats) {
     const DevTarget& t = p.target;
     const int lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
@@ -152,9 +161,6 @@ __device__ uint32_t tile_scan(const DrawParams& p, const UnitInfo& ui, const Til
     const int px = c.tx * kTile + lx;
     uint32_t* s_col = stage;
     float* s_dep = reinterpret_cast<float*>(stage + 256);
-    const float cd = ui.clear_depth;
-    const uint32_t cc = ui.clear_bgra;
-    uint32_t nwin = 0, nclip = 0;
     // all eight keys first: the resets below would otherwise keep the compiler from
     // issuing a row's load before the previous row's store (one load in flight)
     unsigned long long keys[8];
@@ -163,6 +169,18 @@ __device__ uint32_t tile_scan(const DrawParams& p, const UnitInfo& ui, const Til
         const int py = c.ty * kTile + ly0 + 2 * r;
         const bool in = px < t.width && py < t.height;
         keys[r] = (dirty && in) ? __ldcg(t.key + (size_t)py * (size_t)t.width + (size_t)px) : kEmptyKey;
+    }
+    uint32_t count = 0;
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const bool has = keys[r] != kEmptyKey, clipped = has && (((uint32_t)keys[r]) & 8u) != 0u;
+        count += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, has && !clipped)) +
+                 ((uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, clipped)) << 16);
+    }
+    uint32_t at = 0;  // the list's fill before this tile
+    if (fill) {
+        if (lane == 0 && count) at = atomicAdd(fill, count);
+        at = __shfl_sync(0xFFFFFFFFu, at, 0);
     }
 #pragma unroll
     for (int r = 0; r < 8; ++r) {
@@ -177,28 +195,26 @@ __device__ uint32_t tile_scan(const DrawParams& p, const UnitInfo& ui, const Til
         if (has) {
             t.key[idx] = kEmptyKey;  // reset for the next draw into this framebuffer
             s_col[pix] = (uint32_t)key;
-            if (clipped)
-                list[255u - (nclip + (uint32_t)__popc(mc & below))] = (uint8_t)pix;
-            else
-                list[nwin + (uint32_t)__popc(mw & below)] = (uint8_t)pix;
+            const uint32_t k = clipped ? cap - 1u - ((at >> 16) + (uint32_t)__popc(mc & below))
+                                       : (at & 0xFFFFu) + (uint32_t)__popc(mw & below);
+            list[k] = (uint16_t)((slot << 8) | (uint32_t)pix);
         } else if (c.full) {
-            s_col[pix] = cc;
-            s_dep[pix] = cd;
+            s_col[pix] = ui.clear_bgra;
+            s_dep[pix] = ui.clear_depth;
         } else if (in) {
-            if (c.clear_c) t.color[idx] = cc;
-            if (c.clear_d) t.depth[idx] = cd;
+            if (c.clear_c) t.color[idx] = ui.clear_bgra;
+            if (c.clear_d) t.depth[idx] = ui.clear_depth;
         }
-        nwin += (uint32_t)__popc(mw);
-        nclip += (uint32_t)__popc(mc);
+        at += (uint32_t)__popc(mw) + ((uint32_t)__popc(mc) << 16);
     }
     if (dirty && lane == 0) {
         t.tile_flag[c.tile] = 0u;
         if (stats) {
             atomicAdd(&counters->stat_tiles, 1ull);
-            atomicAdd(&counters->stat_shaded, (unsigned long long)(nwin + nclip));
+            atomicAdd(&counters->stat_shaded, (unsigned long long)((count & 0xFFFFu) + (count >> 16)));
         }
     }
-    return nwin | (nclip << 16);
+    return count;
 }
 
 // Merge one shaded (or rejected) fragment of pixel `pix` of the tile.
@@ -216,7 +232,7 @@ __device__ __forceinline__ void tile_put(const DevTarget& t, const UnitInfo& ui,
     }
 }
 
-template <int S>
+template <int S, bool kClipped>
 __device__ __forceinline__ void shade_winner(const DrawParams& p, const UnitInfo& ui, const TileCtx& c, uint32_t* stage,
                                              uint32_t pix) {
     const DevTarget& t = p.target;
@@ -226,28 +242,16 @@ __device__ __forceinline__ void shade_winner(const DrawParams& p, const UnitInfo
     const float old = c.clear_d ? ui.clear_depth : t.depth[idx];
     uint32_t bgra = 0u;
     float z = 0.0f;
-    const bool ok = shade_unclipped<S, true>(p, tag, gx, gy, old, bgra, z);
+    const bool ok = kClipped ? shade_clipped_px<S>(p, tag, gx, gy, old, &bgra, &z)
+                             : shade_unclipped<S, true>(p, tag, gx, gy, old, bgra, z);
     tile_put(t, ui, c, stage, pix, idx, ok, bgra, z);
 }
 
 // Returns whether a TMA store was committed.
-template <int S>
-__device__ bool tile_finish(const DrawParams& p, const UnitInfo& ui, const BatchDraw* bd, const TileCtx& c,
-                            uint32_t* stage, const uint8_t* list, uint32_t nclip) {
+__device__ __forceinline__ bool tile_store(const DrawParams& p, const UnitInfo& ui, const BatchDraw* bd, const TileCtx& c,
+                                           uint32_t* stage) {
     const DevTarget& t = p.target;
     const int lane = threadIdx.x & 31;
-#pragma unroll 1
-    for (uint32_t q = (uint32_t)lane; q < nclip; q += 32) {
-        const uint32_t pix = list[255u - q];
-        const uint32_t tag = stage[pix];
-        const int gx = c.tx * kTile + (int)(pix & 15u), gy = c.ty * kTile + (int)(pix >> 4);
-        const size_t idx = (size_t)gy * (size_t)t.width + (size_t)gx;
-        const float old = c.clear_d ? ui.clear_depth : t.depth[idx];
-        uint32_t bgra = 0u;
-        float z = 0.0f;
-        const bool ok = shade_clipped_px<S>(p, tag, gx, gy, old, &bgra, &z);
-        tile_put(t, ui, c, stage, pix, idx, ok, bgra, z);
-    }
     if (!c.full) return false;
     __syncwarp();
     if (ui.flags & kBatchTma) {
@@ -275,15 +279,17 @@ __device__ bool tile_finish(const DrawParams& p, const UnitInfo& ui, const Batch
 // The whole tile pass by one warp (persistent form). Returns whether a TMA store was committed.
 template <int S>
 __device__ bool tile_pass(const DrawParams& p, const UnitInfo& ui, const BatchDraw* bd, uint32_t tile, bool dirty,
-                          uint32_t* stage, uint8_t* list, DevCounters* counters, bool stats) {
+                          uint32_t* stage, uint16_t* list, DevCounters* counters, bool stats) {
     const TileCtx c = tile_ctx(p.target, ui, tile);
-    const uint32_t n = tile_scan(p, ui, c, dirty, stage, list, counters, stats);
-    const uint32_t nwin = n & 0xFFFFu, nclip = n >> 16;
+    const uint32_t n = tile_scan(p, ui, c, dirty, stage, 0u, list, 256u, nullptr, counters, stats);
+    const uint32_t lane = threadIdx.x & 31u;
     __syncwarp();
 #pragma unroll 1
-    for (uint32_t q = threadIdx.x & 31u; q < nwin; q += 32) shade_winner<S>(p, ui, c, stage, list[q]);
+    for (uint32_t q = lane; q < (n & 0xFFFFu); q += 32) shade_winner<S, false>(p, ui, c, stage, list[q]);
+#pragma unroll 1
+    for (uint32_t q = lane; q < n >> 16; q += 32) shade_winner<S, true>(p, ui, c, stage, list[255u - q]);
     __syncwarp();
-    return tile_finish<S>(p, ui, bd, c, stage, list, nclip);
+    return tile_store(p, ui, bd, c, stage);
 }
 
 // ---- phase bodies, shared by the persistent and the phased forms
@@ -353,7 +359,7 @@ __device__ __forceinline__ void clear_tile(const DevTarget& t, uint32_t tile, ui
 // tile that is dirty or to be cleared. *sbuf alternates the warp's two staging buffers.
 template <int S>
 __device__ __forceinline__ void tile_unit(const BatchParams& bp, const DrawParams& p, const UnitInfo& ui,
-                                          uint32_t* stage2, uint8_t* list, int* sbuf, bool stats) {
+                                          uint32_t* stage2, uint16_t* list, int* sbuf, bool stats) {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t tpw = bp.tiles_per_warp;
     const uint32_t ntiles = (uint32_t)p.target.tiles_x * (uint32_t)p.target.tiles_y;
@@ -386,7 +392,7 @@ __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) batch_kernel(con
     __shared__ __align__(16) DrawParams s_p[2];
     __shared__ UnitInfo s_u[2];
     __shared__ __align__(128) uint32_t s_stage[kBatchWarps][2 * 512];  // warp: 2 x (colour | depth)
-    __shared__ uint8_t s_list[kBatchWarps][256];
+    __shared__ uint16_t s_list[kBatchWarps][256];
     __shared__ __align__(16) FaceSmem<kBatchBlock> s_face;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool stats = bp.collect_stats != 0;
@@ -403,7 +409,7 @@ __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) batch_kernel(con
     for (uint32_t u = blockIdx.x; u < bp.face_units; u += gridDim.x, buf ^= 1) {
         stage_unit(bp, face_base + u, &s_p[buf], &s_u[buf]);
         __syncthreads();
-        face_cta<true>(s_p[buf], s_u[buf].local * kFaceUnit, kFaceUnit, bp.counters, stats, s_face);
+        face_cta<true, false>(s_p[buf], s_u[buf].local * kFaceUnit, kFaceUnit, bp.counters, stats, s_face);
     }
     if (!grid_barrier(bp.counters, prof, 1)) return;
     large_items(bp, stats);
@@ -419,13 +425,19 @@ __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) batch_kernel(con
 }
 
 // ---- phased form: one launch per phase, one CTA per work unit (large: persistent warps)
-template <int S>
+// (the vertices, faces and large triangles of every shader kind of a launch set together)
 __global__ void __launch_bounds__(kBatchBlock) batch_vertex_kernel(const __grid_constant__ BatchParams bp) {
     __shared__ __align__(16) DrawParams s_p;
     __shared__ UnitInfo s_u;
     stage_unit(bp, blockIdx.x, &s_p, &s_u);
     __syncthreads();
-    vertex_unit<S>(s_p, s_u);
+    switch (s_p.u.shader) {
+        case kFlat: vertex_unit<kFlat>(s_p, s_u); break;
+        case kPhong: vertex_unit<kPhong>(s_p, s_u); break;
+        case kPBR: vertex_unit<kPBR>(s_p, s_u); break;
+        case kBlinnPhong: vertex_unit<kBlinnPhong>(s_p, s_u); break;
+        default: vertex_unit<kGouraud>(s_p, s_u); break;
+    }
 }
 
 __global__ void __launch_bounds__(kPhasedFaceUnit, AXR_FACE_MIN_BLOCKS) batch_face_kernel(const __grid_constant__ BatchParams bp) {
@@ -434,57 +446,88 @@ __global__ void __launch_bounds__(kPhasedFaceUnit, AXR_FACE_MIN_BLOCKS) batch_fa
     __shared__ __align__(16) FaceSmem<(int)kPhasedFaceUnit> s_face;
     stage_unit(bp, bp.vert_units + blockIdx.x, &s_p, &s_u);
     __syncthreads();
-    face_cta<false>(s_p, s_u.local * bp.face_unit, bp.face_unit, bp.counters, bp.collect_stats != 0, s_face);
+    face_cta<false, false>(s_p, s_u.local * bp.face_unit, bp.face_unit, bp.counters, bp.collect_stats != 0, s_face);
 }
 
 __global__ void __launch_bounds__(kBatchBlock) batch_large_kernel(const __grid_constant__ BatchParams bp) {
     large_items(bp, bp.collect_stats != 0);
 }
 
-// Tile pass of the phased form: one CTA per unit of 8 x tiles_per_warp consecutive tiles
-// (at most 32). Warp 0 reads the unit's tile flags with one load per lane. Tiles without
-// keys whose two planes are to be cleared are cleared directly by the warps (no staging,
-// no barrier). The other tiles go through the staged pass in rounds of eight, one per
-// warp: each warp scans its tile, then all 256 threads shade the round's winners together
-// (balanced across the eight tiles), then each warp finishes its tile. A warp's two
-// staging buffers alternate after each committed TMA store, so a tile's store overlaps
-// the next round.
+// Shared memory of the phased tile kernel.
+struct TileSmem {
+    __align__(16) DrawParams p;
+    UnitInfo u;
+    __align__(128) uint32_t stage[kBatchWarps][2][512];
+    __align__(128) uint32_t clear[2][256];  // a cleared tile: colour, depth (TMA source)
+    uint16_t list[kBatchWarps * 256];       // a round's winners: unclipped from the front, clipped from the back
+    uint32_t buf[kBatchWarps];              // each slot's staging buffer and tile (x | y << 16)
+    uint32_t pos[kBatchWarps];
+    uint32_t fill[2];                       // the list's fill, by round parity
+    uint32_t dirty;
+};
+
+// Winner `v` of the round's list.
+template <int S, bool kClipped>
+__device__ __forceinline__ void shade_entry(TileSmem& sm, uint32_t v) {
+    const uint32_t w = v >> 8, pos = sm.pos[w];
+    const TileCtx c = tile_ctx_at(sm.u, 0u, (int)(pos & 0xFFFFu), (int)(pos >> 16));
+    shade_winner<S, kClipped>(sm.p, sm.u, c, sm.stage[w][sm.buf[w]], v & 255u);
+}
+
+// The clipped winners of a round, out of line (rare).
 template <int S>
-__global__ void __launch_bounds__(kBatchBlock, AXR_TILE_MIN_BLOCKS) batch_tile_kernel(const __grid_constant__ BatchParams bp) {
-    __shared__ __align__(16) DrawParams s_p;
-    __shared__ UnitInfo s_u;
-    __shared__ __align__(128) uint32_t s_stage[kBatchWarps][2][512];
-    __shared__ uint8_t s_list[kBatchWarps][256];
-    __shared__ uint32_t s_n[kBatchWarps], s_buf[kBatchWarps], s_tile[kBatchWarps];
-    __shared__ uint32_t s_dirty;
-    __shared__ __align__(128) uint32_t s_clear[2][256];  // a cleared tile: colour, depth (TMA source)
+__device__ __noinline__ void shade_clipped_list(TileSmem& sm, uint32_t n) {
+    for (uint32_t q = threadIdx.x; q < n; q += kBatchBlock)
+        shade_entry<S, true>(sm, sm.list[kBatchWarps * 256 - 1 - q]);
+}
+
+// A round's winners, shaded by the whole CTA.
+template <int S>
+__device__ __forceinline__ void shade_list(TileSmem& sm, uint32_t fill) {
+#pragma unroll 1
+    for (uint32_t q = threadIdx.x; q < (fill & 0xFFFFu); q += kBatchBlock) shade_entry<S, false>(sm, sm.list[q]);
+    if (fill >> 16) shade_clipped_list<S>(sm, fill >> 16);
+}
+
+// Tile pass of the phased form: one CTA per unit of bp.tile_unit consecutive tiles (at most
+// 32). Warp 0 reads the unit's tile flags with one load per lane. Tiles without keys whose two
+// planes are to be cleared are cleared directly by the warps (no staging, no barrier). The
+// other tiles go through the staged pass in rounds of eight, one per warp: each warp scans its
+// tile into the round's winner list, then all 256 threads shade the list (balanced across the
+// eight tiles), then each warp stores its tile. A warp's two staging buffers alternate after
+// each committed TMA store, so a tile's store overlaps the next round.
+template <int S>
+__global__ void __launch_bounds__(kBatchBlock, AXR_TILE_MIN_BLOCKS)
+    batch_tile_kernel(const __grid_constant__ BatchParams bp) {
+    __shared__ TileSmem sm;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const bool stats = bp.collect_stats != 0;
-    stage_unit(bp, bp.vert_units + bp.face_units + blockIdx.x, &s_p, &s_u);
+    stage_unit(bp, bp.vert_units + bp.face_units + blockIdx.x, &sm.p, &sm.u);
+    if (threadIdx.x == 0) sm.fill[0] = 0u;
     __syncthreads();
-    const DrawParams& p = s_p;
-    const UnitInfo& ui = s_u;
+    const DrawParams& p = sm.p;
+    const UnitInfo& ui = sm.u;
     // a fully cleared draw with tensor maps: its key-less tiles go out as TMA stores of one
     // cleared tile in shared memory (no clear kernel; every pixel of the frame written once)
     const bool tma_clear = (ui.flags & (kBatchClearColor | kBatchClearDepth)) == (kBatchClearColor | kBatchClearDepth) &&
                            (ui.flags & kBatchTma) && !(ui.flags & kBatchClearedApart);
     if (tma_clear) {
-        s_clear[0][threadIdx.x] = ui.clear_bgra;
-        s_clear[1][threadIdx.x] = __float_as_uint(ui.clear_depth);
+        sm.clear[0][threadIdx.x] = ui.clear_bgra;
+        sm.clear[1][threadIdx.x] = __float_as_uint(ui.clear_depth);
         tma_fence_smem();  // visible to the TMA unit after the barrier below
     }
     const uint32_t ntiles = (uint32_t)p.target.tiles_x * (uint32_t)p.target.tiles_y;
-    const uint32_t unit = kUnitWarps * bp.tiles_per_warp;  // <= 32
+    const uint32_t unit = bp.tile_unit;  // <= 32
     const uint32_t first = ui.local * unit;
     const uint32_t count = min(unit, ntiles - first);
     if (warp == 0) {
         const bool f = (uint32_t)lane < count && ld_volatile(&p.target.tile_flag[first + (uint32_t)lane]) != 0u;
         const unsigned m = __ballot_sync(0xFFFFFFFFu, f);
-        if (lane == 0) s_dirty = m;
+        if (lane == 0) sm.dirty = m;
     }
     __syncthreads();
     const unsigned all = count >= 32u ? 0xFFFFFFFFu : ((1u << count) - 1u);
-    const unsigned dirty = s_dirty;
+    const unsigned dirty = sm.dirty;
     const bool clears = (ui.flags & (kBatchClearColor | kBatchClearDepth)) != 0u;
     const bool full = (ui.flags & (kBatchClearColor | kBatchClearDepth)) == (kBatchClearColor | kBatchClearDepth);
     // key-less tiles with a full clear, spread over the warps (unless the clear kernel has
@@ -503,8 +546,8 @@ __global__ void __launch_bounds__(kBatchBlock, AXR_TILE_MIN_BLOCKS) batch_tile_k
                 if (lane == 0) {
                     const int x = (int)(tile % (uint32_t)p.target.tiles_x) * kTile;
                     const int y = (int)(tile / (uint32_t)p.target.tiles_x) * kTile;
-                    tma_store_tile(&bd->color_map, s_clear[0], x, y);
-                    tma_store_tile(&bd->depth_map, s_clear[1], x, y);
+                    tma_store_tile(&bd->color_map, sm.clear[0], x, y);
+                    tma_store_tile(&bd->depth_map, sm.clear[1], x, y);
                     tma_commit();
                 }
             } else {
@@ -515,7 +558,7 @@ __global__ void __launch_bounds__(kBatchBlock, AXR_TILE_MIN_BLOCKS) batch_tile_k
     // staged tiles: the dirty ones, plus the key-less ones when only one plane is cleared
     unsigned work = full ? dirty : (clears ? all : dirty);
     uint32_t sbuf = 0;  // the buffer this warp stages into; never the newest committed store's
-    while (work) {
+    for (uint32_t round = 0; work; ++round) {
         // this round: the next eight tiles of `work`, the w-th to warp w
         int mine = -1;
 #pragma unroll
@@ -526,40 +569,41 @@ __global__ void __launch_bounds__(kBatchBlock, AXR_TILE_MIN_BLOCKS) batch_tile_k
             if (w == warp) mine = t;
         }
         const uint32_t tile = first + (uint32_t)(mine < 0 ? 0 : mine);
-        uint32_t* stage = s_stage[warp][sbuf];
+        uint32_t* stage = sm.stage[warp][sbuf];
         const TileCtx c = tile_ctx(p.target, ui, tile);
-        uint32_t n = 0;
         if (mine >= 0) {
-            if (lane == 0) tma_wait_read_1();  // an older store from this buffer has read it
+            if (lane == 0) {
+                tma_wait_read_1();  // an older store from this buffer has read it
+                sm.buf[warp] = sbuf;
+                sm.pos[warp] = (uint32_t)c.tx | ((uint32_t)c.ty << 16);
+            }
             __syncwarp();
-            n = tile_scan(p, ui, c, (dirty >> mine) & 1u, stage, s_list[warp], bp.counters, stats);
-        }
-        if (lane == 0) {
-            s_n[warp] = n & 0xFFFFu;
-            s_buf[warp] = sbuf;
-            s_tile[warp] = tile;
+            tile_scan(p, ui, c, (dirty >> mine) & 1u, stage, (uint32_t)warp, sm.list, kBatchWarps * 256,
+                      &sm.fill[round & 1], bp.counters, stats);
         }
         __syncthreads();
-        uint32_t pre[kBatchWarps + 1];
-        pre[0] = 0;
-#pragma unroll
-        for (int w = 0; w < kBatchWarps; ++w) pre[w + 1] = pre[w] + s_n[w];
-        for (uint32_t q = threadIdx.x; q < pre[kBatchWarps]; q += kBatchBlock) {
-            int w = 0;
-#pragma unroll
-            for (int k = 1; k < kBatchWarps; ++k) w += q >= pre[k] ? 1 : 0;
-            shade_winner<S>(p, ui, tile_ctx(p.target, ui, s_tile[w]), s_stage[w][s_buf[w]], s_list[w][q - pre[w]]);
+        const uint32_t fill = sm.fill[round & 1];
+        if (threadIdx.x == 0) sm.fill[(round + 1) & 1] = 0u;  // its last reader passed the barrier above
+        if constexpr (S == kAnyShader) {
+            switch (p.u.shader) {
+                case kFlat: shade_list<kFlat>(sm, fill); break;
+                case kPhong: shade_list<kPhong>(sm, fill); break;
+                case kPBR: shade_list<kPBR>(sm, fill); break;
+                case kBlinnPhong: shade_list<kBlinnPhong>(sm, fill); break;
+                default: shade_list<kGouraud>(sm, fill); break;
+            }
+        } else {
+            shade_list<S>(sm, fill);
         }
         __syncthreads();
-        if (mine >= 0 && tile_finish<S>(p, ui, &bp.draws[ui.draw], c, stage, s_list[warp], n >> 16)) sbuf ^= 1u;
-        __syncthreads();  // s_list, s_n, s_buf and s_tile are rewritten by the next round
+        if (mine >= 0 && tile_store(p, ui, &bp.draws[ui.draw], c, stage)) sbuf ^= 1u;
     }
     // the staging buffers and the cleared tile must have been read before the CTA exits
     // (a thread that committed no store group passes at once)
     tma_wait_read_0();
 }
 
-// Clear of both planes of the phased form's fully cleared draws, in spans of kClearUnit
+// Clear of both planes of the phased form's fully cleared draws, in spans of bp.clear_unit
 // pixels of one draw with 16-byte stores (planes are 256-byte aligned and spans start at
 // multiples of 4 pixels). One CTA per SM walks the spans: 16-byte stores from 256 threads
 // per SM reach the HBM write rate.
@@ -573,7 +617,7 @@ __global__ void __launch_bounds__(kBatchBlock) batch_clear_kernel(const __grid_c
         const size_t n = (size_t)bd->p.target.width * (size_t)bd->p.target.height;
         const uint32_t cc = __ldg(&bd->clear_bgra);
         const float cd = __ldg(&bd->clear_depth);
-        const size_t lo = (size_t)r.y * kClearUnit, hi = min(n, lo + kClearUnit);
+        const size_t lo = (size_t)r.y * bp.clear_unit, hi = min(n, lo + (size_t)bp.clear_unit);
         const uint4 c4 = make_uint4(cc, cc, cc, cc);
         const float4 d4 = make_float4(cd, cd, cd, cd);
         const size_t v_hi = lo + ((hi - lo) & ~size_t(3));
@@ -608,43 +652,62 @@ __global__ void barrier_probe_kernel(DevCounters* c, unsigned long long timeout_
     grid_barrier(c, nullptr, 0, timeout_ns);
 }
 
-template <int S>
-cudaError_t launch_batch_s(const BatchParams& bp, int form, int num_sms, cudaStream_t stream, cudaEvent_t* ev,
-                           uint64_t* launches, bool clear_late) {
+cudaError_t launch_tiles(int shader, const BatchParams& bp, cudaStream_t stream) {
+    switch (shader) {
+        case kAnyShader: batch_tile_kernel<kAnyShader><<<bp.tile_units, kBatchBlock, 0, stream>>>(bp); break;
+        case kFlat: batch_tile_kernel<kFlat><<<bp.tile_units, kBatchBlock, 0, stream>>>(bp); break;
+        case kPhong: batch_tile_kernel<kPhong><<<bp.tile_units, kBatchBlock, 0, stream>>>(bp); break;
+        case kPBR: batch_tile_kernel<kPBR><<<bp.tile_units, kBatchBlock, 0, stream>>>(bp); break;
+        case kBlinnPhong: batch_tile_kernel<kBlinnPhong><<<bp.tile_units, kBatchBlock, 0, stream>>>(bp); break;
+        case kGouraud: batch_tile_kernel<kGouraud><<<bp.tile_units, kBatchBlock, 0, stream>>>(bp); break;
+        default: return cudaErrorInvalidValue;
+    }
+    return cudaGetLastError();
+}
+
+// One launch set of the phased form, all its shader kinds together.
+cudaError_t launch_phased(int shader, const BatchParams& bp, int num_sms, cudaStream_t stream, cudaEvent_t* ev,
+                          uint64_t* launches, bool clear_late) {
     cudaError_t e = cudaMemsetAsync(bp.counters, 0, kBatchCountersReset, stream);
     if (e != cudaSuccess) return e;
-    if (form == kFormPhased) {
-        auto mark = [&](int k) { return ev ? cudaEventRecord(ev[k], stream) : cudaSuccess; };
-        // at the HBM write rate; running it beside the vertex and face phases of the same
-        // draws (a side stream) measured no faster, since their key atomics then wait on its
-        // writes. The raster phases touch only keys and tile flags, so the clear may also
-        // run just before the tile pass (clear_late).
-        auto clear = [&]() -> cudaError_t {
-            if (!bp.clear_units) return cudaSuccess;
-            const unsigned g = min(bp.clear_units, (unsigned)num_sms);
-            batch_clear_kernel<<<g, kBatchBlock, 0, stream>>>(bp);
-            *launches += 1;
-            return cudaGetLastError();
-        };
-        if ((e = mark(0)) != cudaSuccess) return e;
-        if (!clear_late && (e = clear()) != cudaSuccess) return e;
-        if ((e = mark(1)) != cudaSuccess) return e;
-        if (bp.vert_units) batch_vertex_kernel<S><<<bp.vert_units, kBatchBlock, 0, stream>>>(bp);
-        if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(2)) != cudaSuccess) return e;
-        if (bp.face_units) batch_face_kernel<<<bp.face_units, kPhasedFaceUnit, 0, stream>>>(bp);
-        if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(3)) != cudaSuccess) return e;
-        // 16 CTAs per SM, about three waves of the 5 resident: the items are strided over
-        // all warps of the grid, and the later waves even out the first waves' tails (5 per SM
-        // measured 3.041 ms per 512-draw step, 8: 3.027, 10: 3.022, 16: 3.018, 32: 3.020)
-        if (bp.face_units) batch_large_kernel<<<(unsigned)num_sms * 16u, kBatchBlock, 0, stream>>>(bp);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if (clear_late && (e = clear()) != cudaSuccess) return e;
-        if ((e = mark(4)) != cudaSuccess) return e;
-        if (bp.tile_units) batch_tile_kernel<S><<<bp.tile_units, kBatchBlock, 0, stream>>>(bp);
-        if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(5)) != cudaSuccess) return e;
-        *launches += (bp.vert_units ? 1 : 0) + (bp.face_units ? 2 : 0) + (bp.tile_units ? 1 : 0);
-        return cudaSuccess;
-    }
+    auto mark = [&](int k) { return ev ? cudaEventRecord(ev[k], stream) : cudaSuccess; };
+    // at the HBM write rate; running it beside the vertex and face phases of the same
+    // draws (a side stream) measured no faster, since their key atomics then wait on its
+    // writes. The raster phases touch only keys and tile flags, so the clear may also
+    // run just before the tile pass (clear_late).
+    auto clear = [&]() -> cudaError_t {
+        if (!bp.clear_units) return cudaSuccess;
+        const unsigned g = min(bp.clear_units, (unsigned)num_sms);
+        batch_clear_kernel<<<g, kBatchBlock, 0, stream>>>(bp);
+        *launches += 1;
+        return cudaGetLastError();
+    };
+    if ((e = mark(0)) != cudaSuccess) return e;
+    if (!clear_late && (e = clear()) != cudaSuccess) return e;
+    if ((e = mark(1)) != cudaSuccess) return e;
+    if (bp.vert_units) batch_vertex_kernel<<<bp.vert_units, kBatchBlock, 0, stream>>>(bp);
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(2)) != cudaSuccess) return e;
+    if (bp.face_units) batch_face_kernel<<<bp.face_units, kPhasedFaceUnit, 0, stream>>>(bp);
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(3)) != cudaSuccess) return e;
+    // up to 16 CTAs per SM, about three waves of the 5 resident: the items are strided over
+    // all warps of the grid, and the later waves even out the first waves' tails (5 per SM
+    // measured 3.041 ms per 512-draw step, 8: 3.027, 10: 3.022, 16: 3.018, 32: 3.020); no more
+    // CTAs than a small batch has groups of 4 tiles, since CTAs without an item only cost
+    const unsigned large_ctas = max((unsigned)num_sms, min((unsigned)num_sms * 16u, bp.tile_units * bp.tile_unit / 4u));
+    if (bp.face_units) batch_large_kernel<<<large_ctas, kBatchBlock, 0, stream>>>(bp);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if (clear_late && (e = clear()) != cudaSuccess) return e;
+    if ((e = mark(4)) != cudaSuccess) return e;
+    if (bp.tile_units && (e = launch_tiles(shader, bp, stream)) != cudaSuccess) return e;
+    if ((e = mark(5)) != cudaSuccess) return e;
+    *launches += (bp.vert_units ? 1 : 0) + (bp.face_units ? 2 : 0) + (bp.tile_units ? 1 : 0);
+    return cudaSuccess;
+}
+
+template <int S>
+cudaError_t launch_persistent(const BatchParams& bp, int num_sms, cudaStream_t stream, uint64_t* launches) {
+    cudaError_t e = cudaMemsetAsync(bp.counters, 0, kBatchCountersReset, stream);
+    if (e != cudaSuccess) return e;
     // resident CTAs per SM of this instantiation, per device (a cooperative launch must not
     // exceed it)
     constexpr int kMaxDev = 64;
@@ -680,13 +743,13 @@ cudaError_t launch_batch_s(const BatchParams& bp, int form, int num_sms, cudaStr
 
 cudaError_t launch_batch(int shader, const BatchParams& bp, int form, int num_sms, cudaStream_t stream,
                          cudaEvent_t* phase_events, uint64_t* launches, bool clear_late) {
+    if (form == kFormPhased) return launch_phased(shader, bp, num_sms, stream, phase_events, launches, clear_late);
     switch (shader) {
-        case kFlat: return launch_batch_s<kFlat>(bp, form, num_sms, stream, phase_events, launches, clear_late);
-        case kPhong: return launch_batch_s<kPhong>(bp, form, num_sms, stream, phase_events, launches, clear_late);
-        case kPBR: return launch_batch_s<kPBR>(bp, form, num_sms, stream, phase_events, launches, clear_late);
-        case kBlinnPhong:
-            return launch_batch_s<kBlinnPhong>(bp, form, num_sms, stream, phase_events, launches, clear_late);
-        case kGouraud: return launch_batch_s<kGouraud>(bp, form, num_sms, stream, phase_events, launches, clear_late);
+        case kFlat: return launch_persistent<kFlat>(bp, num_sms, stream, launches);
+        case kPhong: return launch_persistent<kPhong>(bp, num_sms, stream, launches);
+        case kPBR: return launch_persistent<kPBR>(bp, num_sms, stream, launches);
+        case kBlinnPhong: return launch_persistent<kBlinnPhong>(bp, num_sms, stream, launches);
+        case kGouraud: return launch_persistent<kGouraud>(bp, num_sms, stream, launches);
         default: return cudaErrorInvalidValue;
     }
 }

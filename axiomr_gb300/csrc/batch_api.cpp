@@ -109,7 +109,8 @@ struct BinPlanD {
 axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t count, axr_batch* b, bool async) {
     axr_status st = check_draws(ctx, draws, count);
     if (st != AXR_OK) return st;
-    // draws grouped by shader kind (one launch each), batch order inside a group
+    // draws grouped by shader kind (one launch each; the phased form takes all kinds together,
+    // below), batch order inside a group
     std::vector<int32_t> order((size_t)count);
     for (int32_t i = 0; i < count; ++i) order[(size_t)i] = i;
     std::stable_sort(order.begin(), order.end(),
@@ -143,6 +144,13 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
     // other's tails and gaps, e.g. the issue-bound large-triangle phase beside the
     // latency-bound tile pass.
     const bool binned = ctx->batch_form == kFormBinned;
+    const std::vector<std::pair<int, std::pair<size_t, size_t>>> kinds = groups;
+    if (ctx->batch_form == kFormPhased && groups.size() > 1) {
+        // one launch set runs the vertices, faces, large triangles and tiles of every kind: a
+        // kind's own four launches would each wait for the kind before (20 small draws of four
+        // kinds: 356 to 65 us, with the tile units of tile_share)
+        groups.assign(1, {kMixedShaders, {0, order.size()}});
+    }
     const int nsets =
         ((ctx->batch_form == kFormPhased || binned) && count >= (int32_t)kSplitMinDraws) ? 2 : 1;
     // binned form: each draw's bin shape and capacity from its density class; per launch set
@@ -172,9 +180,16 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
     const uint32_t item_cap = std::max<uint32_t>(1u << 20, (item_cap_all + nsets - 1) / nsets);
     // work units of every draw (the same counts as the loop below assigns)
     const int form = ctx->batch_form;
-    const uint32_t tiles_per_warp = form == kFormPersistent ? kPersistentTilesPerWarp : kPhasedTilesPerWarp;
-    const uint32_t tile_unit = kUnitWarps * tiles_per_warp;
+    const uint32_t tile_unit = form == kFormPhased ? tile_share(tiles, ctx->cfg.num_sms) : kUnitWarps * kPersistentTilesPerWarp;
     const uint32_t face_unit = form == kFormPhased ? face_share(faces, ctx->cfg.num_sms) : kFaceUnit;
+    uint64_t apart = 0;  // pixels of the draws that the clear kernel writes
+    auto cleared_apart = [&](const axr_draw_desc& d) {
+        return form == kFormPhased && (d.clear_flags & AXR_DRAW_CLEAR_COLOR) && (d.clear_flags & AXR_DRAW_CLEAR_DEPTH) &&
+               !d.framebuffer->tma;
+    };
+    for (int32_t i = 0; i < count; ++i)
+        if (cleared_apart(draws[i])) apart += (uint64_t)draws[i].framebuffer->width * draws[i].framebuffer->height;
+    const uint32_t clear_unit = clear_share(apart, ctx->cfg.num_sms);
     size_t total_units = 0;
     for (int32_t i = 0; i < count; ++i) {
         const axr_draw_desc& d = draws[i];
@@ -184,9 +199,8 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
             total_units += (uint64_t)bplan[(size_t)i].bins_x * bplan[(size_t)i].bins_y;
         else if (drawn || (d.clear_flags & (AXR_DRAW_CLEAR_COLOR | AXR_DRAW_CLEAR_DEPTH)))
             total_units += ceil_div((uint64_t)d.framebuffer->tiles_x * d.framebuffer->tiles_y, tile_unit);
-        if (form == kFormPhased && (d.clear_flags & AXR_DRAW_CLEAR_COLOR) && (d.clear_flags & AXR_DRAW_CLEAR_DEPTH) &&
-            !d.framebuffer->tma)
-            total_units += ceil_div((uint64_t)d.framebuffer->width * d.framebuffer->height, kClearUnit);
+        if (cleared_apart(d))
+            total_units += ceil_div((uint64_t)d.framebuffer->width * d.framebuffer->height, clear_unit);
     }
     const size_t table_bytes = align256(sizeof(BatchDraw) * (size_t)std::max(count, 1));
     const size_t units_bytes = align256(sizeof(UnitRef) * std::max<size_t>(total_units, 1));
@@ -281,7 +295,7 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
                                             m->num_vertices, 0u, 0, 0, nullptr, rec}
                                : DevScratch{d_counters[set], d_large[set], d_items[set], vscreen, vattr, nullptr, nullptr,
                                             large_cap, item_cap, m->num_vertices, 0u, 0, 0, d_large_draw[set], rec};
-            p.small_max_pixels = ctx->tune_small[density_class(d)];
+            p.small_max_pixels = std::min(ctx->tune_small[density_class(d)], face_pixels(faces, ctx->cfg.num_sms));
             p.draw = (uint32_t)k;
             if (binned) {
                 const BinPlanD& bp = bplan[(size_t)order[first + k]];
@@ -310,9 +324,9 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
             // the phased form clears both planes of a fully cleared draw in its tile pass:
             // the key-less tiles with TMA stores of a cleared tile. A framebuffer without
             // tensor maps (width not a multiple of 4) is cleared by its own kernel first.
-            if (form == kFormPhased && (bd.flags & kBatchClearColor) && (bd.flags & kBatchClearDepth) && !fb->tma) {
+            if (cleared_apart(d)) {
                 bd.flags |= kBatchClearedApart;
-                const uint32_t nc = ceil_div((uint64_t)fb->width * fb->height, kClearUnit);
+                const uint32_t nc = ceil_div((uint64_t)fb->width * fb->height, clear_unit);
                 for (uint32_t j = 0; j < nc; ++j) uc.push_back(UnitRef{(uint32_t)k, j});
             }
         }
@@ -340,7 +354,9 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
             bp.clear_units = (uint32_t)uc.size();
             bp.large_cap = large_cap;
             bp.item_cap = item_cap;
-            bp.tiles_per_warp = tiles_per_warp;
+            bp.tiles_per_warp = kPersistentTilesPerWarp;
+            bp.tile_unit = tile_unit;
+            bp.clear_unit = clear_unit;
             bp.face_unit = face_unit;
             if (binned)
                 bp.bins = BinSet{d_bin_counters[set],
@@ -349,6 +365,8 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
             if (bp.vert_units + bp.face_units + bp.tile_units > 0) b->launches.push_back(L);
         }
     }
+    b->kind_sets = 0;
+    for (const auto& k : kinds) b->kind_sets += (uint32_t)std::min<size_t>(k.second.second - k.second.first, (size_t)nsets);
     if (async) {
         // through pinned staging, so that the copies are queued without waiting for the work
         // already on the stream
@@ -551,7 +569,7 @@ void axr_batch_destroy(axr_context* ctx, axr_batch* b) {
 axr_status axr_batch_get_info(const axr_batch* b, axr_batch_info* out) {
     if (!b || !out) return fail(nullptr, AXR_E_INVALID, "NULL argument");
     out->draws = b->count;
-    out->launches = (uint32_t)b->launches.size();
+    out->launches = b->launches.empty() ? 0u : b->kind_sets;
     out->form = b->form;
     out->vertices = b->vertices;
     out->faces = b->faces;

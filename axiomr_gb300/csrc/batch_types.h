@@ -11,8 +11,8 @@
 //                         + shading records (kRecFloat4 float4 per face in draw order)
 //   LargeTri[large_cap], large_draw[large_cap], LargeItem[item_cap]: shared by all draws
 // Work units: 256 vertices (vertex phase), up to 256 faces in draw order (geometry phase),
-// 8 x tiles_per_warp tiles of 16x16 (key-scan + shade phase); the large-triangle phase
-// takes items from the shared list.
+// up to 64 tiles of 16x16 (key-scan + shade phase); the large-triangle phase takes items
+// from the shared list.
 #pragma once
 #include <stdint.h>
 
@@ -32,10 +32,11 @@ constexpr uint32_t kBatchClearedApart = 8u; // phased form: the clear kernel wri
 
 constexpr uint32_t kVertUnit = 256;
 constexpr uint32_t kFaceUnit = 256;        // persistent and binned forms
-constexpr uint32_t kPhasedFaceUnit = 128;  // phased form (threads of its face kernel): at most this,
-                                           // fewer in a batch of few faces (face_share)
+constexpr uint32_t kPhasedFaceUnit = 128;  // phased form: at most this (the threads of its face
+                                           // kernel), fewer in a batch of few faces (face_share)
+constexpr uint32_t kPhasedTileUnit = 32;   // phased form: most tiles per tile unit (32-bit tile masks)
 constexpr uint32_t kUnitWarps = 8;  // warps of a 256-thread CTA
-constexpr uint32_t kClearUnit = 1u << 16;  // pixels per unit of the phased form's clear kernel
+constexpr uint32_t kClearUnit = 1u << 16;  // most pixels per unit of the phased form's clear kernel
 
 struct alignas(64) BatchDraw {
     TensorMap128 color_map;  // uint32 [height][width], 16x16 box
@@ -77,11 +78,13 @@ struct BatchParams {
     const uint32_t* large_draw;
     uint32_t count;
     uint32_t vert_units, face_units, tile_units;
-    uint32_t clear_units;         // phased form: kClearUnit-pixel spans of the full clears
+    uint32_t clear_units;         // phased form: clear_unit-pixel spans of the full clears
     uint32_t large_cap, item_cap;
     int32_t collect_stats;
-    uint32_t tiles_per_warp;      // tiles a warp takes per tile unit (unit = 8 warps x this)
+    uint32_t tiles_per_warp;      // persistent form: tiles a warp takes per tile unit (unit = 8 warps x this)
     uint32_t face_unit;           // faces per face unit
+    uint32_t tile_unit;           // tiles per tile unit
+    uint32_t clear_unit;          // pixels per clear unit
     BinSet bins;                  // binned form: the launch set's bin counts and clipped records
 };
 
@@ -90,11 +93,40 @@ struct BatchParams {
 // draw's setup chains run side by side on all SMs and each CTA's threads share the pixels of
 // its few boxes (frames, us, at 16 / 128 faces per CTA: 4k-triangle sphere 30.8 / 36.9, 200k
 // triangles 148 / 119, 2M triangles 322 / 102).
+constexpr uint32_t kTileShareCtas = 16;  // CTAs per SM that a tile pass should have
 constexpr uint32_t kMinFaceShare = 16;
 inline uint32_t face_share(uint64_t faces, int num_sms) {
     uint32_t n = kPhasedFaceUnit;
     while (n > kMinFaceShare && faces < 4ull * (uint64_t)num_sms * n) n /= 2;
     return n;
+}
+
+// Most pixels of a box that the face phase of a keyed batch of `faces` faces rasterises,
+// whatever the density classes allow: with few CTAs, those with large boxes outlast the others,
+// while the large-triangle pass spreads such boxes over all SMs (20 small draws, 30k faces: 63
+// us at 64 pixels, 73 at 256; 30 mixed draws, 320k faces: 159 us at 96, 180 at 256; 512 mixed
+// draws, 5.4M faces, with their PNG files: 5.91 ms at 64, 5.50 at 256).
+inline int32_t face_pixels(uint64_t faces, int num_sms) {
+    const uint64_t ctas = faces / kPhasedFaceUnit;
+    return ctas < 4ull * (uint64_t)num_sms ? 64 : ctas < 64ull * (uint64_t)num_sms ? 96 : INT32_MAX;
+}
+
+// Tiles per CTA of a phased tile pass over `tiles` tiles: 32 where that leaves enough CTAs for
+// every SM many times over; fewer in a smaller batch, whose tile pass would otherwise end with
+// a few CTAs that still shade their covered tiles one round of eight after another
+// (30 mixed draws, 57k tiles: tile pass 115 to 94 us at 16 tiles; fewer cost more in CTA starts,
+// 183 against 170 us a step at 4).
+inline uint32_t tile_share(uint64_t tiles, int num_sms) {
+    uint32_t n = kPhasedTileUnit;
+    while (n > 1 && tiles < (uint64_t)kTileShareCtas * (uint64_t)num_sms * n) n /= 2;
+    return n;
+}
+
+// Pixels per CTA of the phased form's clear kernel over `pixels` pixels: spread over all SMs,
+// in multiples of what 256 threads store at once.
+inline uint32_t clear_share(uint64_t pixels, int num_sms) {
+    const uint64_t n = (pixels / (uint64_t)num_sms + 1023) & ~uint64_t(1023);
+    return (uint32_t)(n < 4096 ? 4096 : n > kClearUnit ? kClearUnit : n);
 }
 
 // Launch forms of a batch (chosen per batch by the autotuner):
@@ -107,8 +139,10 @@ constexpr int kFormPersistent = 0;
 constexpr int kFormPhased = 1;
 constexpr int kFormBinned = 2;
 constexpr uint32_t kPersistentTilesPerWarp = 8;
-constexpr uint32_t kPhasedTilesPerWarp = 4;
 constexpr uint32_t kSplitMinDraws = 128;  // phased batches of this many draws run as two launch sets
-static_assert(kUnitWarps * kPhasedTilesPerWarp <= 32, "a phased tile unit is described by 32-bit tile masks");
+static_assert(kPhasedTileUnit <= 32, "a phased tile unit is described by 32-bit tile masks");
+
+// The shader argument of a phased launch set whose draws are of several kinds.
+constexpr int kMixedShaders = -1;
 
 }  // namespace axr

@@ -214,7 +214,7 @@ struct alignas(16) DrawParams {
     DevTarget target;
     DevUniforms u;
     DevScratch scratch;
-    int32_t small_max_pixels;  // triangles whose pixel box is at most this are rasterised per thread
+    int32_t small_max_pixels;  // triangles whose pixel box is at most this are rasterised in the face phase
     uint32_t draw;             // index of the draw in its batch (0 for a single draw)
     DevBins bins;              // binned form only
     uint32_t pad_[2];

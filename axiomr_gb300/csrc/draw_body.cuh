@@ -263,17 +263,16 @@ __device__ __forceinline__ void geometry_warp_tail(const DevTarget& t, DevCounte
 // 103, 200k triangles at 3840x2160 133 to 127, 30 mixed draws in a batch 220 to 192; all pixels
 // by pairs instead (no box in its own thread) left the terrain, most of whose boxes hold 2 to 6
 // pixels, at 129.
-constexpr int kWarpPairs = 2048;     // pairs a warp's share of the tables holds; boxes past a
-                                     // group's tables go to the large-triangle list
+constexpr int kWarpPairs = 8192;  // pairs that the 32 faces of a warp may share: 32 boxes of 256
+                                  // pixels; boxes past them go to the large-triangle pass
 constexpr int kThreadPixels = 6;  // boxes a thread rasterises itself (at most 8)
 
 template <int kThreads>
 struct FaceSmem {
     float4 job[kThreads][5];                         // store_job, 80 bytes: no bank conflicts
-    uint32_t start[kThreads / 32 * kWarpPairs / 32]; // bit k: pair k is the first of its box
+    __align__(16) uint32_t start[kThreads / 32 * kWarpPairs / 32]; // bit k: pair k is the first of its box
     uint16_t owner[kThreads / 32 * kWarpPairs / 32]; // the box that holds pair 32 w
     uint32_t warp_sum[kThreads / 32];
-    uint32_t end;                                       // pairs to rasterise (when they exceed the tables)
 };
 
 // Small non-negative integers as floats without the conversion unit (2^23 + v has v in its
@@ -317,8 +316,8 @@ __device__ __forceinline__ bool raster_tiny(const DevTarget& t, const Edges& e, 
 }
 
 // Pair k: coverage and depth of one pixel of the box `j`, in eval_pixel's operations. first
-// and w (both at most 16384) share a word; the row is the floor of (q + 1/2) / w, q < 16384
-// pixels into the box: an approximate reciprocal is off by less than q / w * 2^-22, and no
+// (below 65536) and w (at most 8192) share a word; the row is the floor of (q + 1/2) / w, q < 8192
+// pixels into the box: an approximate reciprocal leaves it off by less than q / w * 2^-22, and no
 // exact value is nearer than 1 / (2 w) to an integer, so the truncation is the quotient.
 __device__ __forceinline__ void raster_pair(const DevTarget& t, const float4* j, uint32_t k, GeomStats& st) {
     const float4 v0 = j[0], v1 = j[1], v2 = j[2], v3 = j[3];
@@ -415,50 +414,50 @@ __device__ __forceinline__ void face_group(const DrawParams& p, uint32_t o, bool
         }
     }
     if (!kWarp || __any_sync(0xFFFFFFFFu, has)) {
-        for (int k = gt; k < (int)kCap / 32; k += 32 * kGroupWarps) start[k] = 0u;
-        // (boxes, pairs) before this thread's: boxes above bit 23, pairs below (at most 256 * 2^14)
-        const uint32_t mine = has ? (1u << 23) | min(npx, kCap + 1u) : 0u;
+        for (int k = gt; k < (int)kCap / 128; k += 32 * kGroupWarps)
+            reinterpret_cast<uint4*>(start)[k] = make_uint4(0u, 0u, 0u, 0u);
+        // (boxes, pairs) before this thread's: boxes above bit 22, pairs below. A warp takes the
+        // boxes that its share of the tables holds, in face order.
+        const uint32_t mine = has ? (1u << 22) | min(npx, (uint32_t)kWarpPairs + 1u) : 0u;
         uint32_t incl = mine;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const uint32_t v = __shfl_up_sync(0xFFFFFFFFu, incl, d);
             if (lane >= d) incl += v;
         }
-        uint32_t before = incl - mine, total = 0;
-        if (kWarp) {
-            total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            if (lane == 0) sm.warp_sum[warp] = 0u;
-            __syncwarp();
-        } else {
-            if (lane == 31) sm.warp_sum[warp] = incl;
-            if (tid == 0) sm.end = 0u;
+        const unsigned past = __ballot_sync(0xFFFFFFFFu, (incl & 0x3FFFFFu) > (uint32_t)kWarpPairs);
+        uint32_t before = incl - mine;
+        uint32_t total = __shfl_sync(0xFFFFFFFFu, past ? before : incl, past ? __ffs(past) - 1 : 31);
+        if (past >> lane & 1u) {
+            large = large || has;
+            has = false;
+        }
+        if (!kWarp) {
+            if (lane == 31) sm.warp_sum[warp] = total;
             __syncthreads();
+            total = 0;
 #pragma unroll
             for (int w = 0; w < kGroupWarps; ++w) {
                 const uint32_t v = sm.warp_sum[w];
                 if (w < warp) before += v;
                 total += v;
             }
+        } else {
+            __syncwarp();  // the zeroed table
         }
-        uint32_t* end = kWarp ? &sm.warp_sum[warp] : &sm.end;
-        uint32_t pairs = total & 0x7FFFFFu;
-        const bool over = pairs > kCap;
+        const uint32_t pairs = total & 0x3FFFFFu;
         if (has) {
-            const uint32_t at = before & 0x7FFFFFu, rank = before >> 23;
-            large = at + npx > kCap;
-            if (!large) {
-                store_job(job[rank], e, tag, at);
-                atomicOr(&start[at >> 5], 1u << (at & 31u));
-                for (uint32_t w = (at + 31u) >> 5; (w << 5) < at + npx; ++w) owner[w] = (uint16_t)rank;
-                if (over) atomicMax(end, at + npx);
-                uint32_t ntx;
-                if (tiles_of(e, ntx) == 1u) single_tile = tile_of(p.target, e.x_lo, e.y_lo);
-                else mark_box(p.target, e);
-            }
+            const uint32_t at = before & 0x3FFFFFu, rank = before >> 22;
+            store_job(job[rank], e, tag, at);
+            atomicOr(&start[at >> 5], 1u << (at & 31u));
+            for (uint32_t w = (at + 31u) >> 5; (w << 5) < at + npx; ++w) owner[w] = (uint16_t)rank;
+            uint32_t ntx;
+            if (tiles_of(e, ntx) == 1u) single_tile = tile_of(p.target, e.x_lo, e.y_lo);
+            else mark_box(p.target, e);
         }
         if (kWarp) __syncwarp();
         else __syncthreads();
-        if (over) pairs = *reinterpret_cast<volatile uint32_t*>(end);
+#pragma unroll 2
         for (uint32_t w = (uint32_t)gw; (w << 5) < pairs; w += kGroupWarps) {
             const uint32_t k = (w << 5) + (uint32_t)lane;
             const uint32_t rank = owner[w] + (uint32_t)__popc(start[w] & ~1u & ((2u << lane) - 1u));
@@ -480,16 +479,20 @@ __device__ __forceinline__ void face_group(const DrawParams& p, uint32_t o, bool
     geometry_warp_tail(p.target, c, stats, st, single_tile);
 }
 
-// The CTA's faces from draw-order position `first`: a face per thread and warp groups, or
-// (faces_of_cta < threads, a draw of few faces) the first threads a face each and the pairs shared
-// by the whole CTA.
-template <bool kCoherent, int kThreads>
+// The CTA's faces from draw-order position `first`, one to each of its first threads. Pairs are
+// shared by the CTA, or (kWarpGroups, with a face for every thread) by each warp: one draw of
+// many faces, mostly tiny boxes, does without the two barriers (2M-triangle terrain 102 against
+// 133 us a frame), while a batch's draws of all densities gain more from the CTA's balance
+// (512 mixed draws, boxes up to 128 pixels: 5.77 against 5.84 ms with their PNG files).
+template <bool kCoherent, bool kWarpGroups, int kThreads>
 __device__ __forceinline__ void face_cta(const DrawParams& p, uint32_t first, uint32_t faces_of_cta, DevCounters* c,
                                          bool stats, FaceSmem<kThreads>& sm) {
     const uint32_t o = first + threadIdx.x;
     const bool valid = threadIdx.x < faces_of_cta && o < p.mesh.num_drawn;
-    if (faces_of_cta == (uint32_t)kThreads) face_group<kCoherent, kThreads, true>(p, o, valid, c, stats, sm);
-    else face_group<kCoherent, kThreads, false>(p, o, valid, c, stats, sm);
+    if (kWarpGroups && faces_of_cta == (uint32_t)kThreads)
+        face_group<kCoherent, kThreads, true>(p, o, valid, c, stats, sm);
+    else
+        face_group<kCoherent, kThreads, false>(p, o, valid, c, stats, sm);
 }
 
 // Whether no pixel of 16x16 tile (tx, ty) inside the triangle's box can test covered.

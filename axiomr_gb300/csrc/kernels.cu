@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kBlock) vertex_kernel(const __grid_constant__ 
 __global__ void __launch_bounds__(kPhasedFaceUnit, AXR_GEOMETRY_MIN_BLOCKS)
     geometry_kernel(const __grid_constant__ DrawParams p, uint32_t faces_per_cta) {
     __shared__ __align__(16) FaceSmem<(int)kPhasedFaceUnit> sm;
-    face_cta<false>(p, blockIdx.x * faces_per_cta, faces_per_cta, p.scratch.counters, p.scratch.collect_stats != 0, sm);
+    face_cta<false, true>(p, blockIdx.x * faces_per_cta, faces_per_cta, p.scratch.counters, p.scratch.collect_stats != 0, sm);
 }
 
 __global__ void __launch_bounds__(kBlock) large_kernel(const __grid_constant__ DrawParams p) {

@@ -376,18 +376,19 @@ typedef struct axr_batch axr_batch;
  * device scratch (vertex caches of all draws, shared large-triangle lists). Returns after
  * the upload. Meshes, framebuffers and textures must outlive the batch. */
 axr_status axr_batch_create(axr_context* ctx, const axr_draw_desc* draws, int32_t count, axr_batch** out);
-/* Enqueue the planned batch on the context stream (per shader kind: a counter reset and
- * the launches of its form). Allocates nothing and reads no host memory, so it can be
- * recorded into a CUDA graph (axr_graph_begin / axr_graph_end) and replayed. */
+/* Enqueue the planned batch on the context stream (per shader kind, or for all kinds
+ * together in the phased form: a counter reset and the launches of its form). Allocates
+ * nothing and reads no host memory, so it can be recorded into a CUDA graph
+ * (axr_graph_begin / axr_graph_end) and replayed. */
 axr_status axr_batch_launch(axr_context* ctx, axr_batch* batch);
 void axr_batch_destroy(axr_context* ctx, axr_batch* batch);
 
 /* Launch forms (the autotuner picks one per batch; batches planned afterwards use it):
  * PERSISTENT: one cooperative launch per shader kind, its four phases (vertices, faces,
- * large-triangle tiles, tile pass) behind grid barriers; PHASED: a clear kernel and four
- * launches per shader kind, one per phase, each over the work units of every draw. A
- * phased batch of 128 or more draws runs each shader kind as two launch sets of
- * alternating draws, the second on a side stream of the context (forked from and joined
+ * large-triangle tiles, tile pass) behind grid barriers; PHASED: a clear kernel (where
+ * needed) and four launches, one per phase, each over the work units of every draw. A
+ * phased batch of 128 or more draws runs as two launch sets of alternating draws, the
+ * second on a side stream of the context (forked from and joined
  * back into its stream, also inside a graph capture), so that the sets' phases overlap. */
 #define AXR_BATCH_PERSISTENT 0
 #define AXR_BATCH_PHASED 1
@@ -402,8 +403,8 @@ int32_t axr_batch_get_form(const axr_context* ctx);
 
 typedef struct axr_batch_info {
     uint32_t draws;
-    uint32_t launches;        /* launch sets per axr_batch_launch: one per shader kind, two for a
-                               * phased batch of 128+ draws */
+    uint32_t launches;        /* shader kinds times launch sets: one per shader kind, two for a
+                               * phased or binned batch of 128+ draws */
     int32_t form;             /* AXR_BATCH_* the batch was planned for */
     uint32_t pad_;
     uint64_t vertices;        /* vertices of all draws */
@@ -419,7 +420,7 @@ axr_status axr_batch_get_info(const axr_batch* batch, axr_batch_info* out);
 axr_status axr_draw_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t count);
 
 /* Autotuner. First the launch form, timing the whole batch in both forms. Then, per
- * density class, the largest triangle pixel box rasterised by one thread (larger boxes go
+ * density class, the largest triangle pixel box rasterised in the face phase (larger boxes go
  * to the warp-per-tile rasteriser), timing the sub-batch of the given draws in that class
  * with each candidate `repeats` times. A draw's density class is the estimated mean screen
  * area of its front-facing triangles, from the mesh's bounding sphere projected through

@@ -35,9 +35,10 @@ def test_face_counts(ctx, port, count):
     check(ctx, port, soup(count, 4.0), f"{count} faces")
 
 
-# pixel-box limits whose boxes overflow a warp's table (2,048 pairs) or a CTA's (8,192)
+# pixel-box limits below, at and above what the pair tables hold for a full CTA (256 pixels a
+# box: larger ones overflow into the large-triangle pass)
 @pytest.mark.parametrize("limit", [0, 6, 7, 256, 1024, 65536])
-@pytest.mark.parametrize("count,edge", [(40, 60.0), (2000, 24.0), (80_000, 14.0)])
+@pytest.mark.parametrize("count,edge", [(40, 60.0), (2000, 24.0), (80_000, 14.0), (1_250_000, 9.0)])
 def test_pair_tables_overflow(port, limit, count, edge):
     ctx = api.Context(0)
     ctx.set_tuning([limit] * 6)
@@ -45,12 +46,13 @@ def test_pair_tables_overflow(port, limit, count, edge):
     vp = port.camera(sc.camera)[2]
     draws = api.batch_draws(ctx, [sc])
     draws[0].camera = api.Camera.from_matrices(vp, sc.camera.position, sc.camera.viewport)
+    expected = port.draw(sc, vp)
     for form in (api.BATCH_PHASED, api.BATCH_PERSISTENT):
         ctx.batch_form = form
         api.draw_batch(ctx, draws)
         got = draws[0].framebuffer.read()
         ctx.sync()
-        assert_parity(got, port.draw(sc, vp), f"limit {limit} form {form}")
+        assert_parity(got, expected, f"limit {limit} form {form}")
     ctx.close()
 
 
