@@ -123,13 +123,16 @@ void free_scratch(axr_context* ctx) {
     dfree(ctx->items);
     dfree(ctx->vscreen);
     dfree(ctx->vattr);
+    dfree(ctx->cut);
+    dfree(ctx->crec);
     dfree(ctx->shade);
-    dfree(ctx->clip_px);
     dfree(ctx->rec);
     ctx->large = nullptr;
     ctx->items = nullptr;
     ctx->vscreen = ctx->vattr = nullptr;
-    ctx->shade = ctx->clip_px = nullptr;
+    ctx->cut = nullptr;
+    ctx->crec = nullptr;
+    ctx->shade = nullptr;
     ctx->rec = nullptr;
     ctx->large_cap = ctx->item_cap = ctx->vcap = ctx->px_cap = ctx->rec_cap = 0;
 }
@@ -145,16 +148,17 @@ void free_bins(axr_context* ctx) {
     ctx->bin_entry_cap = 0;
 }
 
-axr_status grow_scratch(axr_context* ctx, uint32_t faces, uint32_t vertices, uint64_t pixels) {
+axr_status grow_scratch(axr_context* ctx, uint32_t faces, uint32_t vertices, int32_t width, int32_t height) {
     // Large-triangle setups and tile work items (a triangle that finds either list full is
     // rasterised by its own thread instead, so those two sizes trade memory for speed), the
-    // per-vertex cache of the vertex pass (one entry per vertex) and the clipped-winner
-    // pixel list (at most one entry per pixel).
+    // per-vertex cache of the vertex pass (one entry per vertex), per face a shading record and an
+    // entry of the list of faces to clip, and the covered pixels of a frame that the draw scans.
     uint32_t want_tris = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(65536, (uint64_t)faces), 1u << 25);
     uint32_t want_items = (uint32_t)std::min<uint64_t>(std::max<uint64_t>(1u << 20, 4ull * faces), 1u << 27);
     uint32_t want_verts = std::max<uint32_t>(4096, vertices);
-    uint32_t want_px = (uint32_t)std::max<uint64_t>(1u << 16, pixels);
     uint32_t want_rec = std::max<uint32_t>(4096, faces);  // one shading record per face
+    const uint32_t tiles = (uint32_t)((width + kTile - 1) / kTile) * (uint32_t)((height + kTile - 1) / kTile);
+    uint32_t want_px = scan_pass(tiles, ctx->cfg.num_sms) ? (uint32_t)width * (uint32_t)height : 0u;
     if (want_tris <= ctx->large_cap && want_items <= ctx->item_cap && want_verts <= ctx->vcap &&
         want_px <= ctx->px_cap && want_rec <= ctx->rec_cap)
         return AXR_OK;
@@ -173,13 +177,14 @@ axr_status grow_scratch(axr_context* ctx, uint32_t faces, uint32_t vertices, uin
     AXR_CUDA(ctx, dmalloc(&ctx->vscreen, want_verts));
     AXR_CUDA(ctx, dmalloc(&ctx->vattr, 4ull * want_verts));
     AXR_CUDA(ctx, dmalloc(&ctx->shade, want_px));
-    AXR_CUDA(ctx, dmalloc(&ctx->clip_px, want_px));
+    ctx->px_cap = want_px;
+    AXR_CUDA(ctx, dmalloc(&ctx->cut, want_rec));
+    AXR_CUDA(ctx, dmalloc(&ctx->crec, (size_t)kClipRecFloat4 * axr_context::kClipRecs));
     AXR_CUDA(ctx, dmalloc(&ctx->rec, (size_t)kRecFloat4 * want_rec));
     ctx->rec_cap = want_rec;
     ctx->large_cap = want_tris;
     ctx->item_cap = want_items;
     ctx->vcap = want_verts;
-    ctx->px_cap = want_px;
     return AXR_OK;
 }
 
@@ -306,8 +311,8 @@ DrawParams make_params(axr_context* ctx, const axr_mesh* m, const axr_framebuffe
                          fb->width, fb->height, fb->tiles_x, fb->tiles_y};
     p.u = u;
     p.scratch = DevScratch{ctx->counters, ctx->large, ctx->items, ctx->vscreen, ctx->vattr,
-                           ctx->shade, ctx->clip_px, ctx->large_cap, ctx->item_cap, ctx->vcap, ctx->px_cap,
-                           ctx->collect_stats, 0, nullptr, ctx->rec};
+                           ctx->cut, ctx->shade, ctx->crec, ctx->large_cap, ctx->item_cap, ctx->vcap,
+                           axr_context::kClipRecs, ctx->px_cap, ctx->collect_stats, 0, nullptr, ctx->rec};
     p.small_max_pixels = ctx->small_max_pixels;
     return p;
 }
@@ -338,13 +343,6 @@ axr_status axr_context_create(int32_t device, axr_context** out) {
                     prop.major, prop.minor);
     }
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking);
-    // the side stream runs work that fills gaps beside the main stream's (the clipped-winner
-    // pass, the batched form's clears): lowest priority, so the main stream's CTAs go first
-    int prio_low = 0, prio_high = 0;
-    if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high);
-    if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&ctx->aux.stream, cudaStreamNonBlocking, prio_low);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->aux.fork, cudaEventDisableTiming);
-    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->aux.join, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&ctx->batch_side.stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->batch_side.fork, cudaEventDisableTiming);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&ctx->batch_side.join, cudaEventDisableTiming);
@@ -355,9 +353,6 @@ axr_status axr_context_create(int32_t device, axr_context** out) {
     if (e != cudaSuccess) {
         axr_status st = cuda_fail(nullptr, e, "context setup");
         if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
-        if (ctx->aux.stream) cudaStreamDestroy(ctx->aux.stream);
-        if (ctx->aux.fork) cudaEventDestroy(ctx->aux.fork);
-        if (ctx->aux.join) cudaEventDestroy(ctx->aux.join);
         if (ctx->batch_side.stream) cudaStreamDestroy(ctx->batch_side.stream);
         if (ctx->batch_side.fork) cudaEventDestroy(ctx->batch_side.fork);
         if (ctx->batch_side.join) cudaEventDestroy(ctx->batch_side.join);
@@ -368,8 +363,7 @@ axr_status axr_context_create(int32_t device, axr_context** out) {
     }
     ctx->stream = ctx->own_stream;
     ctx->cfg.num_sms = prop.multiProcessorCount;
-    ctx->cfg.large_ctas_per_sm = 2;
-    ctx->cfg.resolve_ctas_per_sm = 4;
+    ctx->cfg.large_ctas_per_sm = 4;
     *out = ctx;
     return AXR_OK;
 }
@@ -390,8 +384,6 @@ void axr_context_destroy(axr_context* ctx) {
     free_scratch(ctx);
     free_bins(ctx);
     free_png(ctx);
-    if (ctx->aux.stream) cudaStreamSynchronize(ctx->aux.stream);
-    if (ctx->aux.stream) cudaStreamDestroy(ctx->aux.stream);
     for (int k = 0; k < axr_context::kCopyStreams; ++k) {
         if (ctx->copy_stream[k]) {
             cudaStreamSynchronize(ctx->copy_stream[k]);
@@ -400,8 +392,6 @@ void axr_context_destroy(axr_context* ctx) {
         if (ctx->copy_join[k]) cudaEventDestroy(ctx->copy_join[k]);
     }
     if (ctx->copy_fork) cudaEventDestroy(ctx->copy_fork);
-    if (ctx->aux.fork) cudaEventDestroy(ctx->aux.fork);
-    if (ctx->aux.join) cudaEventDestroy(ctx->aux.join);
     if (ctx->batch_side.stream) {
         cudaStreamSynchronize(ctx->batch_side.stream);
         cudaStreamDestroy(ctx->batch_side.stream);
@@ -458,7 +448,7 @@ axr_status axr_reserve(axr_context* ctx, uint32_t max_faces) {
     if (!ctx) return fail(nullptr, AXR_E_INVALID, "context is NULL");
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard g(ctx->device);
-    axr_status st = grow_scratch(ctx, max_faces, max_faces * 3u, 3840ull * 2160ull);
+    axr_status st = grow_scratch(ctx, max_faces, max_faces * 3u, 3840, 2160);
     if (st != AXR_OK) return st;
     // the binned form's bins for a 3840x2160 framebuffer in the smallest-bin shape
     axr_framebuffer probe{};
@@ -978,8 +968,7 @@ axr_status axr_draw_mesh(axr_context* ctx, const axr_mesh* mesh, const float mod
     std::lock_guard<std::mutex> lk(ctx->mu);
     if (!ctx->has_shader || !ctx->has_camera || !ctx->fb) return AXR_OK;  // src/tiled_pipeline.cpp:146
     DeviceGuard g(ctx->device);
-    axr_status st = grow_scratch(ctx, mesh->num_drawn, mesh->num_vertices,
-                                 (uint64_t)ctx->fb->width * (uint64_t)ctx->fb->height);
+    axr_status st = grow_scratch(ctx, mesh->num_drawn, mesh->num_vertices, ctx->fb->width, ctx->fb->height);
     if (st != AXR_OK) return st;
     DevUniforms u = make_uniforms(ctx->camera, ctx->shader, model);
     DrawParams p = make_params(ctx, mesh, ctx->fb, u);
@@ -1002,7 +991,7 @@ axr_status axr_draw_mesh(axr_context* ctx, const axr_mesh* mesh, const float mod
     if (ctx->draw_form != AXR_DRAW_BINNED) {
         LaunchConfig cfg = ctx->cfg;
         cfg.clip_free = mesh_clip_free(mesh, u.mvp);
-        AXR_CUDA(ctx, launch_draw(p, cfg, ctx->stream, &ctx->aux, ev, &ctx->launches));
+        AXR_CUDA(ctx, launch_draw(p, cfg, ctx->stream, ev, &ctx->launches));
         return AXR_OK;
     }
     SoloBinned sb{};
@@ -1151,7 +1140,7 @@ axr_status axr_profile_read(axr_context* ctx, axr_profile* out) {
     AXR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     axr_profile r{};
     for (size_t k = 0; k + kStageEvents <= ctx->events_used; k += kStageEvents) {
-        double* out[6] = {&r.vertex_ms, &r.geometry_ms, &r.large_ms, &r.scan_ms, &r.shade_ms, &r.clipped_ms};
+        double* out[6] = {&r.vertex_ms, &r.geometry_ms, &r.clipped_ms, &r.large_ms, &r.shade_ms, &r.scan_ms};
         for (int j = 0; j < 6; ++j) {
             float ms = 0.f;
             AXR_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->event_pool[k + j], ctx->event_pool[k + j + 1]));

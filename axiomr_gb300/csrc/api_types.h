@@ -104,7 +104,6 @@ struct axr_context {
     int device = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t stream = nullptr;
-    axr::AuxStream aux{};  // side stream + fork/join events for the clipped-winner pass
     axr::AuxStream batch_side{};  // second launch set of a split batch (normal priority)
     // read-back streams of axr_framebuffers_read_async (created on first use): copies of many
     // framebuffers are spread over them so that several copy engines run at once
@@ -126,8 +125,10 @@ struct axr_context {
     LargeItem* items = nullptr;
     float4* vscreen = nullptr;
     float4* vattr = nullptr;
-    uint2* shade = nullptr;
-    uint2* clip_px = nullptr;
+    uint32_t* cut = nullptr;  // faces that straddle the clip volume (rec_cap entries)
+    uint2* shade = nullptr;   // covered pixels of larger frames (px_cap entries)
+    float4* crec = nullptr;   // clipped-triangle records (kClipRecFloat4 per entry)
+    static constexpr uint32_t kClipRecs = 1u << 16;
     float4* rec = nullptr;  // shading records (kRecFloat4 per face in draw order)
     uint32_t large_cap = 0, item_cap = 0, vcap = 0, px_cap = 0, rec_cap = 0;
     int collect_stats = 0;

@@ -291,10 +291,11 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
             cache += align256(16 * (size_t)m->num_vertices * (size_t)vattr_float4s(d.shader.kind));
             float4* rec = reinterpret_cast<float4*>(cache);
             cache += align256(16 * (size_t)kRecFloat4 * m->num_drawn);
-            p.scratch = binned ? DevScratch{d_counters[set], nullptr, nullptr, vscreen, vattr, nullptr, nullptr, 0u, 0u,
-                                            m->num_vertices, 0u, 0, 0, nullptr, rec}
-                               : DevScratch{d_counters[set], d_large[set], d_items[set], vscreen, vattr, nullptr, nullptr,
-                                            large_cap, item_cap, m->num_vertices, 0u, 0, 0, d_large_draw[set], rec};
+            p.scratch = binned ? DevScratch{d_counters[set], nullptr, nullptr, vscreen, vattr, nullptr, nullptr,
+                                            nullptr, 0u, 0u, m->num_vertices, 0u, 0u, 0, 0, nullptr, rec}
+                               : DevScratch{d_counters[set], d_large[set], d_items[set], vscreen, vattr, nullptr,
+                                            nullptr, nullptr, large_cap, item_cap, m->num_vertices, 0u, 0u, 0, 0,
+                                            d_large_draw[set], rec};
             p.small_max_pixels = std::min(ctx->tune_small[density_class(d)], face_pixels(faces, ctx->cfg.num_sms));
             p.draw = (uint32_t)k;
             if (binned) {

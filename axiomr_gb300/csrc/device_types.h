@@ -96,7 +96,6 @@ struct LargeItem {
     uint32_t tile;       // tile index inside the triangle's tile box (row-major)
 };
 constexpr uint32_t kNoItem = 0xFFFFFFFFu;
-constexpr uint32_t kItemsPerGrab = 4;  // tiles a warp takes per atomic
 
 // Bounding box and squared bounding-sphere radius of a mesh's positions, computed on the
 // device after an update: lo/hi as order-preserving integers (see kernels.cu), r2 the
@@ -106,14 +105,14 @@ struct MeshBounds {
     unsigned long long r2;  // bits of a non-negative double
 };
 
-// Work counters of one draw: the first kCountersReset bytes are zeroed (a memset on
-// the stream) before every draw.
+// Work counters of one draw: the first kCountersReset bytes are zeroed before every draw (by the
+// per-draw path's vertex kernel, a memset in the others).
 struct DevCounters {
     uint32_t large_count;     // LargeTri slots reserved (may exceed the capacity)
     uint32_t item_count;      // LargeItem slots reserved (may exceed the capacity)
-    uint32_t item_head;       // next LargeItem to hand out
-    uint32_t shade_count;     // covered pixels (unclipped winners) found by the key scan
-    uint32_t clip_count;      // covered pixels whose winner is a clipped triangle
+    uint32_t cut_count;       // faces that straddle the clip volume (per-draw path)
+    uint32_t crec_count;      // clipped-triangle records reserved (per-draw path; may exceed the capacity)
+    uint32_t shade_count;     // covered pixels listed by the scan kernel
     uint32_t bar_count;       // batched kernel: CTAs arrived at the current grid barrier
     uint32_t bar_gen;         // batched kernel: grid barriers completed
     uint32_t error;           // sticky error bits (kErr*), cleared by axr_sync
@@ -136,21 +135,21 @@ constexpr uint32_t kErrTma = 8u;      // a tile load of the binned form did not 
 // Per-vertex cache written by the vertex pass of each draw:
 //   vscreen[i] = (screen x, screen y, NDC z, clip-plane masks as uint bits)
 //   vattr[n*i ...] = the shader's vertex outputs (n = VAttr<S>::n float4s)
-// Resolve work lists written by the key scan: shade[k] = (pixel index, depth-key tag) of a
-// covered pixel whose winner is an unclipped triangle; clip_px[k] = the same pair when the
-// winner came out of the clipper.
+// cut[k] (per-draw path): draw-order position of a face that straddles the clip volume.
 struct DevScratch {
     DevCounters* counters;
     LargeTri* large;
     LargeItem* items;
     float4* vscreen;
     float4* vattr;
-    uint2* shade;
-    uint2* clip_px;
+    uint32_t* cut;            // >= num_drawn entries; NULL: such faces are clipped where they are found
+    uint2* shade;             // covered pixels (pixel x | y << 16, tag) listed by the scan kernel
+    float4* crec;             // clipped-triangle records: raster record + 3 packed vertex outputs each
     uint32_t large_cap;
     uint32_t item_cap;
     uint32_t vcap;
-    uint32_t px_cap;          // >= pixels of the target (shade and clip_px capacity)
+    uint32_t crec_cap;
+    uint32_t px_cap;          // entries of shade: >= pixels of the target where the scan kernel runs
     int32_t collect_stats;
     int32_t pad_;
     uint32_t* large_draw;     // batched draws: draw index of each LargeTri slot (NULL per draw)
@@ -162,7 +161,12 @@ struct DevScratch {
 // setup from the face: the raster record (edge terms, 1/area, vertex depths, pixel range,
 // material; x_lo gives the row-start rule of eval_pixel) and the three vertex indices (for
 // the cached vertex outputs).
+// A face that straddles the clip volume has none; with scratch.cut its position's first word
+// holds the number of its first clipped-triangle record (kNoClipRec: the list was full, its winners
+// re-run the clipper).
 constexpr int kRecFloat4 = 5;
+constexpr uint32_t kNoClipRec = 0xFFFFFFFFu;
+constexpr int kClipRecFloat4 = 16;  // most float4 per clipped-triangle record (4 + 3 * 4)
 
 // Binned form: the framebuffer is cut into bins of 8 tiles of 16x16 (tw x th tiles: 8x1,
 // 4x2 or 2x4). The face kernel appends each set-up triangle to the entry list of every bin

@@ -384,9 +384,10 @@ __device__ __forceinline__ bool face_setup(const DrawParams& p, uint32_t o, Geom
 }
 
 // The faces of a CTA, thread t's at draw-order position o (valid: it has one); a group is a
-// warp (kWarp) or the CTA. The tiles of a shared box are flagged whether or not a pixel of it turns
+// warp (kWarp) or the CTA. Faces that straddle the clip volume go to scratch.cut (kCutList) or
+// through the clipper here. The tiles of a shared box are flagged whether or not a pixel of it turns
 // out covered (a flagged tile without keys costs the tile pass its key reads).
-template <bool kCoherent, int kThreads, bool kWarp>
+template <bool kCoherent, bool kCutList, int kThreads, bool kWarp>
 __device__ __forceinline__ void face_group(const DrawParams& p, uint32_t o, bool valid, DevCounters* c, bool stats,
                                            FaceSmem<kThreads>& sm) {
     constexpr int kGroupWarps = kWarp ? 1 : kThreads / 32;
@@ -468,7 +469,15 @@ __device__ __forceinline__ void face_group(const DrawParams& p, uint32_t o, bool
         }
     }
     if (large) emit_large(p, e, tag, st);
-    if (cut) {  // last: the clipper is a long chain, and the group would wait for it
+    if (kCutList) {  // to the clip kernel
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, cut);
+        if (m) {
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&c->cut_count, (uint32_t)__popc(m));
+            at = __shfl_sync(0xFFFFFFFFu, at, 0);
+            if (cut) p.scratch.cut[at + (uint32_t)__popc(m & ((1u << lane) - 1u))] = o;
+        }
+    } else if (cut) {  // last: the clipper is a long chain, and the group would wait for it
         GeomStats clipped = {0, 0, 0, 0};  // its own: no pointer to st leaves this function
         geometry_clipped(p, o, clipped);
         st.tris += clipped.tris;
@@ -480,19 +489,19 @@ __device__ __forceinline__ void face_group(const DrawParams& p, uint32_t o, bool
 }
 
 // The CTA's faces from draw-order position `first`, one to each of its first threads. Pairs are
-// shared by the CTA, or (kWarpGroups, with a face for every thread) by each warp: one draw of
+// shared by the CTA, or (kSolo, the per-draw path, with a face for every thread) by each warp: one draw of
 // many faces, mostly tiny boxes, does without the two barriers (2M-triangle terrain 102 against
 // 133 us a frame), while a batch's draws of all densities gain more from the CTA's balance
 // (512 mixed draws, boxes up to 128 pixels: 5.77 against 5.84 ms with their PNG files).
-template <bool kCoherent, bool kWarpGroups, int kThreads>
+template <bool kCoherent, bool kSolo, int kThreads>
 __device__ __forceinline__ void face_cta(const DrawParams& p, uint32_t first, uint32_t faces_of_cta, DevCounters* c,
                                          bool stats, FaceSmem<kThreads>& sm) {
     const uint32_t o = first + threadIdx.x;
     const bool valid = threadIdx.x < faces_of_cta && o < p.mesh.num_drawn;
-    if (kWarpGroups && faces_of_cta == (uint32_t)kThreads)
-        face_group<kCoherent, kThreads, true>(p, o, valid, c, stats, sm);
+    if (kSolo && faces_of_cta == (uint32_t)kThreads)
+        face_group<kCoherent, kSolo, kThreads, true>(p, o, valid, c, stats, sm);
     else
-        face_group<kCoherent, kThreads, false>(p, o, valid, c, stats, sm);
+        face_group<kCoherent, kSolo, kThreads, false>(p, o, valid, c, stats, sm);
 }
 
 // Whether no pixel of 16x16 tile (tx, ty) inside the triangle's box can test covered.
@@ -599,6 +608,52 @@ __device__ bool clipped_inputs(const DrawParams& p, uint32_t tag, Screen& s, VSO
     return true;
 }
 
+// The clip pass of a listed face: geometry_clipped with the attributes carried along, and each
+// output triangle's setup and vertex-shader outputs stored for the tile pass, which would
+// otherwise re-run the clipper for every pixel it wins (a chain of 10 us that a CTA waits for).
+template <int S>
+__device__ void clip_listed(const DrawParams& p, uint32_t o, GeomStats& st) {
+    constexpr int A = ShaderAttrs<S>::mask;
+    constexpr uint32_t kStride = 4 + 3 * VAttr<S>::n;
+    static_assert(kStride <= (uint32_t)kClipRecFloat4, "clipped-triangle record size");
+    const FaceRef fr = face_of(p.mesh, o);
+    const uint3 f = load_face(p.mesh, fr.face);
+    CVFull a[kMaxClipVerts], b[kMaxClipVerts];
+    a[0] = load_vertex<A>(p.mesh, f.x);
+    a[1] = load_vertex<A>(p.mesh, f.y);
+    a[2] = load_vertex<A>(p.mesh, f.z);
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        const float4 q = __ldg(&p.mesh.pos[k == 0 ? f.x : k == 1 ? f.y : f.z]);
+        a[k].clip = mat4_mul(p.u.mvp, q.x, q.y, q.z, 1.0f);
+    }
+    CVFull* out;
+    const int n = clip_triangle<A>(a, b, &out);
+    const uint32_t nt = (uint32_t)n / 3u;
+    uint32_t base = nt ? atomicAdd(&p.scratch.counters->crec_count, nt) : 0u;
+    if (base + nt > p.scratch.crec_cap) base = kNoClipRec;
+    p.scratch.rec[(size_t)kRecFloat4 * o] = make_float4(__uint_as_float(base), 0.f, 0.f, 0.f);
+    for (uint32_t j = 0; j < nt; ++j) {
+        const CVFull* v = out + 3 * j;
+        Screen s;
+        screen_setup(v[0].clip, v[1].clip, v[2].clip, p.target.width, p.target.height, s);
+        if (is_backface(s)) continue;
+        ++st.tris;
+        Edges e;
+        if (!edge_setup(s, p.target.width, p.target.height, e)) continue;
+        if (base != kNoClipRec) {
+            float4* r = p.scratch.crec + (size_t)kStride * (base + j);
+            store_raster(r, e, fr.material);
+            for (int k = 0; k < 3; ++k) pack_vsout<S>(vertex_shader<S>(p.u, v[k]), r + 4 + VAttr<S>::n * k);
+        }
+        const uint32_t tag = (o << 4) | 8u | j;
+        if ((e.x_hi - e.x_lo) * (e.y_hi - e.y_lo) > min(p.small_max_pixels, kClippedThreadPixels))
+            emit_large(p, e, tag, st);
+        else if (raster_box_call(p.target, e, tag, st))
+            mark_box(p.target, e);
+    }
+}
+
 // Fragment of the winner at (px, py): exact barycentrics and depth, the merge test against
 // `old_depth` (tile depth < framebuffer depth, strict; src/tiled_pipeline.cpp:1171-1174)
 // and the shader. Returns whether the fragment is written.
@@ -663,6 +718,37 @@ __device__ __noinline__ bool shade_clipped_px(const DrawParams& p, uint32_t tag,
     VSOut vo[3];
     uint32_t material;
     return clipped_inputs<S>(p, tag, s, vo, material) && shade_pixel<S>(p, px, py, material, s, vo, old_depth, *bgra, *z);
+}
+
+// Winner of the per-draw tile pass, clipped or not.
+template <int S, bool kClip>
+__device__ __forceinline__ bool shade_any(const DrawParams& p, uint32_t tag, int px, int py, float old_depth,
+                                          uint32_t& bgra, float& z) {
+    VSOut vo[3];
+    Edges e;
+    uint32_t material;
+    if (kClip && (tag & 8u)) {
+        const uint32_t base = __float_as_uint(p.scratch.rec[(size_t)kRecFloat4 * (tag >> 4)].x);
+        if (base == kNoClipRec) {
+            uint32_t c = 0u;
+            float d = 0.0f;
+            if (!shade_clipped_px<S>(p, tag, px, py, old_depth, &c, &d)) return false;
+            bgra = c;
+            z = d;
+            return true;
+        }
+        const float4* r = p.scratch.crec + (size_t)(4 + 3 * VAttr<S>::n) * (base + (tag & 7u));
+        material = unpack_raster(r[0], r[1], r[2], r[3], e);
+#pragma unroll
+        for (int k = 0; k < 3; ++k) vo[k] = unpack_vsout<S, true>(r + 4 + VAttr<S>::n * k);
+    } else if (tag & kRecTag) {
+        material = record_inputs<S, true>(p, tag, e, vo);
+    } else {
+        Screen s;
+        material = winner_inputs<S, true>(p, tag, s, vo);
+        if (!edge_setup(s, p.target.width, p.target.height, e)) return false;
+    }
+    return shade_from<S>(p, e, vo, material, px, py, old_depth, bgra, z);
 }
 
 }  // namespace

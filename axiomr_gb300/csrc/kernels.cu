@@ -1,6 +1,7 @@
 // Draw kernels for sm_103a.
 //
-// A draw is a counter reset (memset) and six launches on one stream:
+// A draw is four launches on one stream (one more when faces may be clipped, and one in a larger
+// frame), each set up while the one before drains (pdl.cuh):
 //   vertex_kernel    one thread per vertex: clip position (mvp * pos), screen position and
 //                    NDC depth (the per-vertex part of the reference's Triangle ctor,
 //                    src/tiled_pipeline.cpp:53-72), clip-plane masks, and the shader's
@@ -8,19 +9,22 @@
 //                    reference recomputes these for every face a vertex belongs to (clip
 //                    stage) and every tile a triangle touches (processTile, cpp:407-409);
 //                    they depend only on the vertex, so one evaluation gives the same bits.
-//   geometry_kernel  one thread per face in draw order: clip classification from the
-//                    vertex masks (exact clipper for faces that straddle a plane), backface
-//                    cull and edge setup (cpp:195-236, 436-487). Triangles whose pixel box
-//                    is small are rasterised by the same thread; larger ones get one setup
-//                    record and one work item per 16x16 tile of their box.
-//   large_kernel     warps take tile work items (4 per atomic) and evaluate 256 pixels
-//                    each, 8 per lane.
-//   scan_kernel      one warp per flagged 16x16 tile: compacts the tile's covered pixels
-//                    (non-empty depth keys) into the shade / clipped lists, resets the keys.
-//   shade_kernel     one thread per covered pixel: the winner is re-derived from its depth
-//                    key, shaded once, and merged into the framebuffer with the reference's
-//                    strict less-than test (winners that were clipped go to
-//                    resolve_clipped_kernel).
+//                    Its first thread zeroes the draw's counters.
+//   geometry_kernel  one thread per face in draw order: clip classification from the vertex
+//                    masks, backface cull and edge setup (cpp:195-236, 436-487), then the pixels
+//                    of the smaller boxes (face_group, draw_body.cuh); larger boxes get one
+//                    setup record and one work item per 16x16 tile, faces that straddle the
+//                    clip volume go to a list
+//   clip_kernel      one thread per listed face: the exact clipper, its output triangles
+//                    rasterised or queued as above; not launched when the mesh's bounding sphere
+//                    shows that no face can be clipped
+//   large_kernel     warps take tile work items and evaluate 256 pixels each, 8 per lane
+//   tile_kernel      a CTA per flagged tile: its covered pixels (non-empty depth keys) are
+//                    listed and their keys reset, then one thread per covered pixel re-derives
+//                    the winner from its key, shades it once and merges it into the framebuffer
+//                    with the reference's strict less-than test. A larger frame (scan_pass) does
+//                    it in two kernels, scan_kernel listing the covered pixels of all tiles in
+//                    memory and shade_kernel shading them
 // Visibility is order independent: every covered pixel does a fire-and-forget 64-bit
 // atomicMin of (depth, draw-order position), so the surviving key is the reference's
 // early-Z winner (minimum depth, earliest triangle on ties) whatever order the threads
@@ -34,12 +38,16 @@
 #include "batch_types.h"
 #include "draw_body.cuh"
 #include "kernels.h"
+#include "pdl.cuh"
 
 namespace axr {
 
 namespace {
 
 constexpr int kBlock = 256;
+constexpr int kClipBlock = 64;
+constexpr int kScanTiles = 2;  // tiles per warp and round of the scan kernel
+
 
 // Resident 128-thread CTAs per SM the geometry kernel is compiled for (register budget
 // 65536 / (128 * n)): 64 registers.
@@ -50,17 +58,47 @@ constexpr int kBlock = 256;
 
 template <int S>
 __global__ void __launch_bounds__(kBlock) vertex_kernel(const __grid_constant__ DrawParams p) {
+    pdl_release();
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
+    if (i == 0) {
+        p.scratch.counters->large_count = 0u;
+        p.scratch.counters->item_count = 0u;
+        p.scratch.counters->cut_count = 0u;
+        p.scratch.counters->crec_count = 0u;
+        p.scratch.counters->shade_count = 0u;
+    }
     if (i < p.mesh.num_vertices) vertex_one<S>(p, i);
 }
 
 __global__ void __launch_bounds__(kPhasedFaceUnit, AXR_GEOMETRY_MIN_BLOCKS)
     geometry_kernel(const __grid_constant__ DrawParams p, uint32_t faces_per_cta) {
     __shared__ __align__(16) FaceSmem<(int)kPhasedFaceUnit> sm;
-    face_cta<false, true>(p, blockIdx.x * faces_per_cta, faces_per_cta, p.scratch.counters, p.scratch.collect_stats != 0, sm);
+    pdl_wait();
+    pdl_release();
+    face_cta<true, true>(p, blockIdx.x * faces_per_cta, faces_per_cta, p.scratch.counters, p.scratch.collect_stats != 0,
+                         sm);
+}
+
+// The listed faces, spread over the warps of the grid first (lane 0 of each, then lane 1, ...):
+// the lanes of a warp would run different planes' chains one after another.
+template <int S>
+__global__ void __launch_bounds__(kClipBlock) clip_kernel(const __grid_constant__ DrawParams p) {
+    pdl_wait();
+    pdl_release();
+    DevCounters* c = p.scratch.counters;
+    const uint32_t n = min(ld_volatile(&c->cut_count), p.mesh.num_drawn);
+    const uint32_t warps = gridDim.x * (kClipBlock / 32);
+    GeomStats st = {0, 0, 0, 0};
+    for (uint32_t k = blockIdx.x * (kClipBlock / 32) + (threadIdx.x >> 5) + (threadIdx.x & 31u) * warps; k < n;
+         k += 32 * warps)
+        clip_listed<S>(p, p.scratch.cut[k], st);
+    __syncwarp();
+    geometry_warp_tail(p.target, c, p.scratch.collect_stats != 0, st, kNoTile);
 }
 
 __global__ void __launch_bounds__(kBlock) large_kernel(const __grid_constant__ DrawParams p) {
+    pdl_wait();
+    pdl_release();
     DevCounters* c = p.scratch.counters;
     const uint32_t n_items = min(ld_volatile(&c->item_count), p.scratch.item_cap);
     const uint32_t n_tris = min(ld_volatile(&c->large_count), p.scratch.large_cap);
@@ -83,130 +121,152 @@ __global__ void __launch_bounds__(kBlock) large_kernel(const __grid_constant__ D
     }
 }
 
-// Key scan over every tile of the target, one warp per tile and 8 tiles per CTA round:
-// flagged tiles have their 256 keys read (8 per lane), every covered pixel is appended as
-// (pixel, tag) to the shade list, or to the clipped list when its winner came out of the
-// clipper, and the keys and the flag are reset. List space is taken once per CTA round
-// (shared-memory prefix over the 8 warps), so the global counters see few atomics.
-__global__ void __launch_bounds__(kBlock) scan_kernel(const __grid_constant__ DrawParams p) {
+// Resident 256-thread CTAs per SM the shading kernels are compiled for, by the shader's registers
+// (frames, us: PBR close-up 102.8 / 96.2 / 96.7 at 2 / 3 / 4 CTAs, Blinn-Phong terrain 96.3 / 94.9 / 96.7
+// at 3 / 4 / 5; without a bound PBR took 86 registers, so 2 CTAs).
+constexpr int tile_blocks(int shader) {
+    return shader == kPhong || shader == kPBR ? 3 : shader == kBlinnPhong ? 4 : 5;
+}
+
+// One covered pixel (x | y << 16) whose winner is `tag`: shaded and merged.
+template <int S, bool kClip>
+__device__ __forceinline__ void shade_listed(const DrawParams& p, uint2 w) {
+    const DevTarget& t = p.target;
+    const int px = (int)(w.x & 0xFFFFu), py = (int)(w.x >> 16);
+    const size_t idx = (size_t)py * (size_t)t.width + (size_t)px;
+    uint32_t bgra;
+    float z;
+    if (shade_any<S, kClip>(p, w.y, px, py, t.depth[idx], bgra, z)) {
+        t.color[idx] = bgra;
+        t.depth[idx] = z;
+    }
+}
+
+// Tile pass of a small frame: a CTA per flagged tile, a thread per pixel. The covered pixels are
+// listed in shared memory, so that a tile of few fills as few warps; a frame of this size is
+// bound by latency, and one kernel has one start and one chain.
+template <int S, bool kClip>
+__global__ void __launch_bounds__(kBlock, tile_blocks(S)) tile_kernel(const __grid_constant__ DrawParams p) {
+    __shared__ uint2 s_list[256];
+    __shared__ uint32_t s_fill;
+    const DevTarget& t = p.target;
+    const int tid = threadIdx.x, lane = tid & 31;
+    if (tid == 0) s_fill = 0u;
+    pdl_wait();
+    pdl_release();
+    const uint32_t tile = blockIdx.x;
+    if (ld_volatile(&t.tile_flag[tile]) == 0u) return;  // the same for every thread
+    const uint32_t px = tile % (uint32_t)t.tiles_x * kTile + (uint32_t)(tid & 15);
+    const uint32_t py = tile / (uint32_t)t.tiles_x * kTile + (uint32_t)(tid >> 4);
+    unsigned long long key = kEmptyKey;
+    const size_t idx = (size_t)py * (size_t)t.width + px;
+    if (px < (uint32_t)t.width && py < (uint32_t)t.height) key = __ldcg(t.key + idx);
+    const bool has = key != kEmptyKey;
+    const unsigned m = __ballot_sync(0xFFFFFFFFu, has);
+    __syncthreads();  // s_fill; and every thread has read the flag
+    if (tid == 0) t.tile_flag[tile] = 0u;
+    uint32_t at = 0;
+    if (lane == 0 && m) at = atomicAdd(&s_fill, (uint32_t)__popc(m));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0);
+    if (has) {
+        s_list[at + (uint32_t)__popc(m & ((1u << lane) - 1u))] = make_uint2(px | (py << 16), (uint32_t)key);
+        t.key[idx] = kEmptyKey;  // for the next draw
+    }
+    __syncthreads();
+    const uint32_t n = s_fill;
+    if (p.scratch.collect_stats && tid == 0) {
+        atomicAdd(&p.scratch.counters->stat_tiles, 1ull);
+        atomicAdd(&p.scratch.counters->stat_shaded, (unsigned long long)n);
+    }
+    if ((uint32_t)tid < n) shade_listed<S, kClip>(p, s_list[tid]);
+}
+
+// Key scan of a larger frame: kScanTiles tiles per warp and round, all their keys in flight at
+// once; the covered pixels are appended to the shade list, their keys and the tiles' flags
+// reset. List space is taken once per CTA round (a prefix over the warps), so the global counter
+// sees few atomics; the warps' counts are double-buffered, so that a round has two barriers.
+// Bound by the keys' reads.
+__global__ void __launch_bounds__(kBlock, 3) scan_kernel(const __grid_constant__ DrawParams p) {
     constexpr int kWarps = kBlock / 32;
-    __shared__ uint32_t s_count[2][kWarps];
-    __shared__ uint32_t s_base[2];
+    __shared__ uint32_t s_count[2][kWarps], s_base[2];
     DevCounters* c = p.scratch.counters;
     const DevTarget& t = p.target;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const uint32_t ntiles = (uint32_t)t.tiles_x * (uint32_t)t.tiles_y;
-    for (uint32_t first = blockIdx.x * kWarps; first < ntiles; first += gridDim.x * kWarps) {
-        const uint32_t tile = first + (uint32_t)warp;
-        const bool dirty = tile < ntiles && ld_volatile(&t.tile_flag[tile]) != 0u;
-        const int px = (int)(tile % (uint32_t)t.tiles_x) * kTile + (lane & 15);
-        const int py0 = (int)(tile / (uint32_t)t.tiles_x) * kTile + (lane >> 4);
-        unsigned long long keys[8];
-        unsigned ms[8], mc[8];
-        uint32_t ns = 0, nc = 0;
-        if (dirty) {
+    const uint32_t ntiles = (uint32_t)t.tiles_x * (uint32_t)t.tiles_y, per_round = kWarps * kScanTiles;
+    pdl_wait();
+    pdl_release();
+    int buf = 0;
+    for (uint32_t first = blockIdx.x * per_round; first < ntiles; first += gridDim.x * per_round, buf ^= 1) {
+        unsigned long long keys[kScanTiles][8];
+        uint32_t pos[kScanTiles], count = 0;
+        bool dirty[kScanTiles];
+#pragma unroll
+        for (int k = 0; k < kScanTiles; ++k) {
+            const uint32_t tile = first + (uint32_t)(warp * kScanTiles + k);
+            dirty[k] = tile < ntiles && ld_volatile(&t.tile_flag[tile]) != 0u;
+            pos[k] = (tile % (uint32_t)t.tiles_x * kTile + (uint32_t)(lane & 15)) |
+                     (tile / (uint32_t)t.tiles_x * kTile + (uint32_t)(lane >> 4)) << 16;
+        }
+#pragma unroll
+        for (int k = 0; k < kScanTiles; ++k) {
+            const uint32_t px = pos[k] & 0xFFFFu, py = pos[k] >> 16;
+            const unsigned long long* at = t.key + (size_t)py * (size_t)t.width + px;
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
-                const int py = py0 + 2 * r;
-                keys[r] = (px < t.width && py < t.height) ? t.key[(uint32_t)py * (uint32_t)t.width + (uint32_t)px]
-                                                          : kEmptyKey;
+                keys[k][r] = (dirty[k] && px < (uint32_t)t.width && py + 2 * r < (uint32_t)t.height) ? __ldcg(at) : kEmptyKey;
+                at += 2 * (size_t)t.width;
             }
+        }
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const bool has = keys[r] != kEmptyKey;
-                const bool clipped = has && (((uint32_t)keys[r]) & 8u) != 0u;
-                ms[r] = __ballot_sync(0xFFFFFFFFu, has && !clipped);
-                mc[r] = __ballot_sync(0xFFFFFFFFu, clipped);
-                ns += (uint32_t)__popc(ms[r]);
-                nc += (uint32_t)__popc(mc[r]);
+        for (int k = 0; k < kScanTiles; ++k)
+            if (dirty[k]) {
+#pragma unroll
+                for (int r = 0; r < 8; ++r) count += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, keys[k][r] != kEmptyKey));
             }
-        }
-        if (lane == 0) {
-            s_count[0][warp] = ns;
-            s_count[1][warp] = nc;
-        }
+        if (lane == 0) s_count[buf][warp] = count;
         __syncthreads();
-        if (threadIdx.x < 2) {
-            uint32_t total = 0;
-            for (int w = 0; w < kWarps; ++w) {
-                const uint32_t v = s_count[threadIdx.x][w];
-                s_count[threadIdx.x][w] = total;
-                total += v;
-            }
-            s_base[threadIdx.x] = total ? atomicAdd(threadIdx.x == 0 ? &c->shade_count : &c->clip_count, total) : 0u;
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (int w = 0; w < kWarps; ++w) {
+            const uint32_t v = s_count[buf][w];
+            if (w < warp) before += v;
+            total += v;
         }
+        if (threadIdx.x == 0 && total) s_base[buf] = atomicAdd(&c->shade_count, total);
         __syncthreads();
-        if (dirty) {
-            uint32_t bs = s_base[0] + s_count[0][warp], bc = s_base[1] + s_count[1][warp];
+        uint32_t at = s_base[buf] + before;
+#pragma unroll
+        for (int k = 0; k < kScanTiles; ++k) {
+            if (!dirty[k]) continue;
+            unsigned long long* key = t.key + (size_t)(pos[k] >> 16) * (size_t)t.width + (pos[k] & 0xFFFFu);
 #pragma unroll
             for (int r = 0; r < 8; ++r) {
-                if (keys[r] != kEmptyKey) {
-                    const uint32_t idx = (uint32_t)(py0 + 2 * r) * (uint32_t)t.width + (uint32_t)px;
-                    const uint2 entry = make_uint2(idx, (uint32_t)keys[r]);
-                    if ((uint32_t)keys[r] & 8u)
-                        p.scratch.clip_px[bc + (uint32_t)__popc(mc[r] & below)] = entry;
-                    else
-                        p.scratch.shade[bs + (uint32_t)__popc(ms[r] & below)] = entry;
-                    t.key[idx] = kEmptyKey;
+                const bool has = keys[k][r] != kEmptyKey;
+                const unsigned m = __ballot_sync(0xFFFFFFFFu, has);
+                if (has) {
+                    p.scratch.shade[at + (uint32_t)__popc(m & below)] = make_uint2(pos[k] + ((uint32_t)(2 * r) << 16), (uint32_t)keys[k][r]);
+                    key[(size_t)(2 * r) * (size_t)t.width] = kEmptyKey;  // for the next draw
                 }
-                bs += (uint32_t)__popc(ms[r]);
-                bc += (uint32_t)__popc(mc[r]);
+                at += (uint32_t)__popc(m);
             }
             if (lane == 0) {
-                t.tile_flag[tile] = 0u;
-                if (p.scratch.collect_stats) {
-                    atomicAdd(&c->stat_tiles, 1ull);
-                    atomicAdd(&c->stat_shaded, (unsigned long long)(ns + nc));
-                }
+                t.tile_flag[first + (uint32_t)(warp * kScanTiles + k)] = 0u;
+                if (p.scratch.collect_stats) atomicAdd(&c->stat_tiles, 1ull);
             }
         }
-        __syncthreads();
+        if (p.scratch.collect_stats && lane == 0) atomicAdd(&c->stat_shaded, (unsigned long long)count);
     }
 }
 
-// Dense shading of the covered pixels whose winner is unclipped: the winner's setup (from
-// its shading record, or re-derived from the face and the vertex cache) gives its exact
-// barycentrics and depth, and the fragment is shaded once.
-template <int S>
-__global__ void __launch_bounds__(kBlock) shade_kernel(const __grid_constant__ DrawParams p) {
-    DevCounters* c = p.scratch.counters;
-    const DevTarget& t = p.target;
-    const uint32_t n = min(ld_volatile(&c->shade_count), p.scratch.px_cap);
-    for (uint32_t q = blockIdx.x * kBlock + threadIdx.x; q < n; q += gridDim.x * kBlock) {
-        const uint2 w = p.scratch.shade[q];
-        const size_t idx = w.x;
-        const int px = (int)(idx % (size_t)t.width), py = (int)(idx / (size_t)t.width);
-        uint32_t bgra;
-        float z;
-        if (shade_unclipped<S>(p, w.y, px, py, t.depth[idx], bgra, z)) {
-            t.color[idx] = bgra;
-            t.depth[idx] = z;
-        }
-    }
-}
-
-// Pixels whose winner is a clipped triangle: the winner's inputs come from re-running the
-// clipper on the face.
-template <int S>
-__global__ void __launch_bounds__(kBlock) resolve_clipped_kernel(const __grid_constant__ DrawParams p) {
-    const uint32_t n = min(ld_volatile(&p.scratch.counters->clip_count), p.scratch.px_cap);
-    const DevTarget& t = p.target;
-    for (uint32_t q = blockIdx.x * kBlock + threadIdx.x; q < n; q += gridDim.x * kBlock) {
-        const uint2 w = p.scratch.clip_px[q];
-        const size_t idx = w.x;
-        const int px = (int)(idx % (size_t)t.width), py = (int)(idx / (size_t)t.width);
-        Screen s;
-        VSOut vo[3];
-        uint32_t material;
-        if (!clipped_inputs<S>(p, w.y, s, vo, material)) continue;
-        uint32_t bgra;
-        float z;
-        if (shade_pixel<S>(p, px, py, material, s, vo, t.depth[idx], bgra, z)) {
-            t.color[idx] = bgra;
-            t.depth[idx] = z;
-        }
-    }
+// The listed pixels, a thread each: covered areas are spread evenly over all SMs.
+template <int S, bool kClip>
+__global__ void __launch_bounds__(kBlock, tile_blocks(S)) shade_kernel(const __grid_constant__ DrawParams p) {
+    pdl_wait();
+    pdl_release();
+    const uint32_t n = min(ld_volatile(&p.scratch.counters->shade_count), p.scratch.px_cap);
+    const uint2* list = p.scratch.shade;
+    for (uint32_t q = blockIdx.x * kBlock + threadIdx.x; q < n; q += gridDim.x * kBlock) shade_listed<S, kClip>(p, list[q]);
 }
 
 // Colour and/or depth fill, 16-byte stores (the planes are 256-byte aligned allocations).
@@ -293,64 +353,67 @@ unsigned grid_for(size_t n, int block, unsigned cap = 65535u * 16u) {
 }
 
 template <int S>
-cudaError_t launch_shaded(const DrawParams& p, const LaunchConfig& cfg, cudaStream_t stream, const AuxStream* aux,
-                          cudaEvent_t* ev, uint64_t* launches) {
+cudaError_t launch_shaded(const DrawParams& p, const LaunchConfig& cfg, cudaStream_t stream, cudaEvent_t* ev,
+                          uint64_t* launches) {
     cudaError_t e;
     auto mark = [&](int k) { return ev ? cudaEventRecord(ev[k], stream) : cudaSuccess; };
-    if ((e = cudaMemsetAsync(p.scratch.counters, 0, kCountersReset, stream)) != cudaSuccess) return e;
     if ((e = mark(0)) != cudaSuccess) return e;
-    if (p.mesh.num_drawn > 0) {
-        vertex_kernel<S><<<grid_for(p.mesh.num_vertices, kBlock, 0x7FFFFFFFu), kBlock, 0, stream>>>(p);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        if ((e = mark(1)) != cudaSuccess) return e;
-        const uint32_t share = face_share(p.mesh.num_drawn, cfg.num_sms);
-        geometry_kernel<<<grid_for(p.mesh.num_drawn, (int)share, 0x7FFFFFFFu), kPhasedFaceUnit, 0, stream>>>(p, share);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        *launches += 2;
-    } else if ((e = mark(1)) != cudaSuccess) {
-        return e;
+    if (p.mesh.num_drawn == 0) {  // nothing to draw: the framebuffer stays as it is
+        for (int k = 1; k < kStageEvents; ++k)
+            if ((e = mark(k)) != cudaSuccess) return e;
+        return cudaSuccess;
     }
-    if ((e = mark(2)) != cudaSuccess) return e;
-    large_kernel<<<(unsigned)(cfg.num_sms * cfg.large_ctas_per_sm), kBlock, 0, stream>>>(p);
+    vertex_kernel<S><<<grid_for(p.mesh.num_vertices, kBlock, 0x7FFFFFFFu), kBlock, 0, stream>>>(p);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = mark(3)) != cudaSuccess) return e;
-    const unsigned tiles = (unsigned)(p.target.tiles_x * p.target.tiles_y);
-    scan_kernel<<<min((tiles + 7u) / 8u, (unsigned)(cfg.num_sms * 8)), kBlock, 0, stream>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = mark(4)) != cudaSuccess) return e;
-    // the clipped-winner pass is independent of the main shading pass: run it beside it
-    // (unless no triangle can have been clipped, when its list is empty)
+    if ((e = mark(1)) != cudaSuccess) return e;
+    const uint32_t share = face_share(p.mesh.num_drawn, cfg.num_sms);
+    e = launch_dependent(geometry_kernel, grid_for(p.mesh.num_drawn, (int)share, 0x7FFFFFFFu), kPhasedFaceUnit, stream, p,
+                         share);
+    if (e != cudaSuccess || (e = mark(2)) != cudaSuccess) return e;
     const bool clipped = !cfg.clip_free;
-    cudaStream_t side = aux ? aux->stream : stream;
-    if (clipped && aux) {
-        if ((e = cudaEventRecord(aux->fork, stream)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(aux->stream, aux->fork, 0)) != cudaSuccess) return e;
-    }
     if (clipped) {
-        resolve_clipped_kernel<S><<<(unsigned)cfg.num_sms / 2u + 1u, kBlock, 0, side>>>(p);
-        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+        // a warp for each of the first num_sms * 8 faces
+        e = launch_dependent(clip_kernel<S>, (unsigned)cfg.num_sms * 4u, (unsigned)kClipBlock, stream, p);
+        if (e != cudaSuccess) return e;
     }
-    shade_kernel<S><<<(unsigned)(cfg.num_sms * cfg.resolve_ctas_per_sm), kBlock, 0, stream>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = mark(5)) != cudaSuccess) return e;
-    if (clipped && aux) {
-        if ((e = cudaEventRecord(aux->join, aux->stream)) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(stream, aux->join, 0)) != cudaSuccess) return e;
+    if ((e = mark(3)) != cudaSuccess) return e;
+    e = launch_dependent(large_kernel, (unsigned)(cfg.num_sms * cfg.large_ctas_per_sm), (unsigned)kBlock, stream, p);
+    if (e != cudaSuccess || (e = mark(4)) != cudaSuccess) return e;
+    const uint32_t tiles = (uint32_t)(p.target.tiles_x * p.target.tiles_y);
+    if (!scan_pass(tiles, cfg.num_sms)) {
+        e = clipped ? launch_dependent(tile_kernel<S, true>, tiles, (unsigned)kBlock, stream, p)
+                    : launch_dependent(tile_kernel<S, false>, tiles, (unsigned)kBlock, stream, p);
+    } else {
+        const unsigned scan_ctas = (tiles + kBlock / 32 * kScanTiles - 1) / (kBlock / 32 * kScanTiles);
+        e = launch_dependent(scan_kernel, scan_ctas, (unsigned)kBlock, stream, p);
+        if (e != cudaSuccess) return e;
+        *launches += 1;
+        const unsigned shade_ctas = (unsigned)(cfg.num_sms * tile_blocks(S));
+        e = clipped ? launch_dependent(shade_kernel<S, true>, shade_ctas, (unsigned)kBlock, stream, p)
+                    : launch_dependent(shade_kernel<S, false>, shade_ctas, (unsigned)kBlock, stream, p);
     }
-    *launches += clipped ? 4 : 3;
+    if (e != cudaSuccess || (e = mark(5)) != cudaSuccess) return e;
+    *launches += clipped ? 5 : 4;
     return mark(6);
 }
 
 }  // namespace
 
-cudaError_t launch_draw(const DrawParams& p, const LaunchConfig& cfg, cudaStream_t stream, const AuxStream* aux,
-                        cudaEvent_t* stage_events, uint64_t* launches) {
+// Up to 30 tiles per SM one kernel is faster (frames, us, one kernel / scan and shade: 96x96 icon 19.5 /
+// 22.8, 512x512 sphere 22.6 / 26.2, 1365x767 close-up 93.6 / 96.2); in larger frames it is not, since it
+// shades a tile where its CTA runs while a list spreads the covered pixels evenly over all
+// threads, and its keys' reads wait for shading (1920x1080 terrain level; 200k small triangles at
+// 3840x2160 120 to 139 with 8 tiles per CTA / 106).
+bool scan_pass(uint32_t tiles, int num_sms) { return tiles > 30u * (uint32_t)num_sms; }
+
+cudaError_t launch_draw(const DrawParams& p, const LaunchConfig& cfg, cudaStream_t stream, cudaEvent_t* stage_events,
+                        uint64_t* launches) {
     switch (p.u.shader) {
-        case kFlat: return launch_shaded<kFlat>(p, cfg, stream, aux, stage_events, launches);
-        case kPhong: return launch_shaded<kPhong>(p, cfg, stream, aux, stage_events, launches);
-        case kPBR: return launch_shaded<kPBR>(p, cfg, stream, aux, stage_events, launches);
-        case kBlinnPhong: return launch_shaded<kBlinnPhong>(p, cfg, stream, aux, stage_events, launches);
-        case kGouraud: return launch_shaded<kGouraud>(p, cfg, stream, aux, stage_events, launches);
+        case kFlat: return launch_shaded<kFlat>(p, cfg, stream, stage_events, launches);
+        case kPhong: return launch_shaded<kPhong>(p, cfg, stream, stage_events, launches);
+        case kPBR: return launch_shaded<kPBR>(p, cfg, stream, stage_events, launches);
+        case kBlinnPhong: return launch_shaded<kBlinnPhong>(p, cfg, stream, stage_events, launches);
+        case kGouraud: return launch_shaded<kGouraud>(p, cfg, stream, stage_events, launches);
         default: return cudaErrorInvalidValue;
     }
 }

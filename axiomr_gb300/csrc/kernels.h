@@ -7,8 +7,8 @@
 
 namespace axr {
 
-// Side stream and events of a context: the clipped-winner resolve pass runs on the side
-// stream, concurrently with the main shading pass (fork after the key scan, join after).
+// Side stream and events of a context: the second launch set of a split batch (fork before its
+// first launch, join after its last).
 struct AuxStream {
     cudaStream_t stream;
     cudaEvent_t fork, join;
@@ -17,20 +17,22 @@ struct AuxStream {
 struct LaunchConfig {
     int num_sms;
     int large_ctas_per_sm;
-    int resolve_ctas_per_sm;
     // no vertex of the draw can lie outside or on a clip plane (checked on the host from the
-    // mesh's bounding sphere): no triangle is clipped, so the clipped-winner pass is not run
+    // mesh's bounding sphere): no triangle is clipped, so the clip pass is not run
     bool clip_free = false;
 };
 
-// One draw: geometry (transform, clip, cull, setup, small-triangle raster) -> large
-// triangle tile raster -> per-tile resolve and shading into the framebuffer.
-// `stage_events` (optional, kStageEvents events) are recorded before the first kernel and
-// after each of the six (vertex, geometry, large, scan, shade, clipped). Adds the number
-// of kernels launched to *launches.
+// One draw: vertices, faces (clip classification, cull, setup, raster of the smaller boxes), the
+// clip pass, large-triangle tiles, tile pass (key scan, shading, merge). `stage_events` (optional,
+// kStageEvents events) are recorded before the first kernel and after each of vertex, geometry,
+// clip, large, tile (and once more). Adds the number of kernels launched to *launches.
+// Whether a draw into a frame of so many tiles lists its covered pixels in scratch.shade (a scan
+// and a shade kernel) instead of tile by tile in shared memory.
+bool scan_pass(uint32_t tiles, int num_sms);
+
 constexpr int kStageEvents = 7;
-cudaError_t launch_draw(const DrawParams& p, const LaunchConfig& cfg, cudaStream_t stream, const AuxStream* aux,
-                        cudaEvent_t* stage_events, uint64_t* launches);
+cudaError_t launch_draw(const DrawParams& p, const LaunchConfig& cfg, cudaStream_t stream, cudaEvent_t* stage_events,
+                        uint64_t* launches);
 
 cudaError_t launch_clear(uint32_t* color, float* depth, size_t pixels, uint32_t bgra, float depth_value,
                          bool do_color, bool do_depth, cudaStream_t stream);

@@ -49,9 +49,11 @@ constexpr size_t kOffLarge = align256(kOffCounters + sizeof(axr::DevCounters));
 constexpr size_t kOffItems = align256(kOffLarge + sizeof(axr::LargeTri) * kNoAllocMaxFaces);
 constexpr size_t kOffVscreen = align256(kOffItems + sizeof(axr::LargeItem) * kNoAllocMaxItems);
 constexpr size_t kOffVattr = align256(kOffVscreen + sizeof(float4) * kNoAllocMaxVertices);
-constexpr size_t kOffShade = align256(kOffVattr + 4 * sizeof(float4) * kNoAllocMaxVertices);
-constexpr size_t kOffClip = align256(kOffShade + sizeof(uint2) * kNoAllocMaxPixels);
-constexpr size_t kOffRec = align256(kOffClip + sizeof(uint2) * kNoAllocMaxPixels);
+constexpr size_t kOffCut = align256(kOffVattr + 4 * sizeof(float4) * kNoAllocMaxVertices);
+constexpr uint32_t kNoAllocClipRecs = 1u << 14;
+constexpr size_t kOffCrec = align256(kOffCut + sizeof(uint32_t) * kNoAllocMaxFaces);
+constexpr size_t kOffShade = align256(kOffCrec + sizeof(float4) * axr::kClipRecFloat4 * kNoAllocClipRecs);
+constexpr size_t kOffRec = align256(kOffShade + sizeof(uint2) * kNoAllocMaxPixels);
 constexpr size_t kNoAllocBytes = align256(kOffRec + sizeof(float4) * axr::kRecFloat4 * kNoAllocMaxFaces);
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocBytes];
@@ -116,14 +118,15 @@ extern "C" axr_status axr_draw_mesh_noalloc(axr_context* ctx, const axr_mesh* me
                                reinterpret_cast<LargeItem*>(base + kOffItems),
                                reinterpret_cast<float4*>(base + kOffVscreen),
                                reinterpret_cast<float4*>(base + kOffVattr),
+                               reinterpret_cast<uint32_t*>(base + kOffCut),
                                reinterpret_cast<uint2*>(base + kOffShade),
-                               reinterpret_cast<uint2*>(base + kOffClip),
-                               kNoAllocMaxFaces, kNoAllocMaxItems, kNoAllocMaxVertices, kNoAllocMaxPixels,
-                               ctx->collect_stats, 0, nullptr, reinterpret_cast<float4*>(base + kOffRec)};
+                               reinterpret_cast<float4*>(base + kOffCrec),
+                               kNoAllocMaxFaces, kNoAllocMaxItems, kNoAllocMaxVertices, kNoAllocClipRecs,
+                               kNoAllocMaxPixels, ctx->collect_stats, 0, nullptr, reinterpret_cast<float4*>(base + kOffRec)};
         p.small_max_pixels = ctx->small_max_pixels;
         // the array keeps the previous call's contents: start from zeroed counters
         e = cudaMemsetAsync(counters, 0, sizeof(DevCounters), ctx->stream);
-        if (e == cudaSuccess) e = launch_draw(p, ctx->cfg, ctx->stream, &ctx->aux, nullptr, &ctx->launches);
+        if (e == cudaSuccess) e = launch_draw(p, ctx->cfg, ctx->stream, nullptr, &ctx->launches);
         // the array's error bits and statistics into the context's counters
         if (e == cudaSuccess) e = launch_merge_counters(ctx->counters, counters, ctx->stream);
         if (e == cudaSuccess) ctx->launches += 1;

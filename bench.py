@@ -437,15 +437,14 @@ def run_ours(args, dist: Dist):
         # depth-key write per covered fragment
         "geometry": 12.0 * F + 16.0 * V + 8.0 * frags,
         "large": 8.0 * frags,
-        # keys of the dirty tiles read, one 8-byte work entry per covered pixel written
-        "scan": 8.0 * scanned_px + 8.0 * frags,
-        # per covered pixel: work entry, indices, depth read, colour + depth write; the
-        # vertex cache read once
-        "shade": frags * (8.0 + 12.0 + 4.0 + 8.0) + float(V) * (16 + vattr),
+        "scan": 0.0,  # part of the shade stage
+        # keys of the dirty tiles read; per covered pixel: indices, depth read, colour + depth
+        # write; the vertex cache read once
+        "shade": 8.0 * scanned_px + frags * (12.0 + 4.0 + 8.0) + float(V) * (16 + vattr),
         "clipped": 0.0,
     }
     kernel_names = {k: k + "_kernel" for k in stages}
-    kernel_names["clipped"] = "resolve_clipped_kernel"
+    kernel_names["clipped"] = "clip_kernel"
     if args.draw_form == "binned":
         # three kernels: vertices, faces (setup and binning; the profile's geometry stage) and
         # bins (raster, shading and tile write-out; its shading stage). Algorithmic bytes: the

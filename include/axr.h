@@ -631,11 +631,11 @@ typedef struct axr_profile {
     uint32_t draws;          /* draws recorded */
     uint32_t pad_;
     double vertex_ms;        /* per-vertex transform and vertex shader */
-    double geometry_ms;      /* clip, cull, setup, small-triangle raster */
+    double geometry_ms;      /* cull, setup, raster of smaller boxes */
     double large_ms;         /* large-triangle tile raster */
-    double scan_ms;          /* dirty-tile key scan */
-    double shade_ms;         /* per-pixel resolve and shading */
-    double clipped_ms;       /* resolve of pixels won by clipped triangles */
+    double scan_ms;          /* 0: the key scan is part of shade_ms */
+    double shade_ms;         /* key scan, per-pixel resolve and shading */
+    double clipped_ms;       /* clipper on faces that straddle the view volume */
     uint64_t kernel_launches;/* all kernels launched on this context since creation */
     uint64_t batch_launches; /* batched launches timed (including graph replays) */
     double batch_vertex_ms;  /* batched kernel phases: vertices */

@@ -66,3 +66,30 @@ def test_clip_planes(ctx, port, target, distance, lon):
     sc = W.sphere_scene(width=241, height=163, lon=lon, lat=max(4, lon // 2), shader=W.SHADER_PHONG)
     sc.camera = W.Camera((0.0, 0.0, float(distance)), target, 60.0, float(np.float32(241 / 163)), (0, 0, 241, 163))
     check(ctx, port, sc, f"target {target} distance {distance}")
+
+
+# frames on both sides of the limit (30 tiles per SM: 4,560 on 152 SMs) between the one-kernel tile
+# pass and the scan and shade kernels, with ragged right and top edges, clipped and not
+@pytest.mark.parametrize("size", [(1, 1), (15, 17), (1216, 960), (1215, 961), (1301, 977)])
+@pytest.mark.parametrize("shader", [W.SHADER_FLAT, W.SHADER_PBR])
+@pytest.mark.parametrize("distance", [3.0, 1.3])
+def test_tile_passes(ctx, port, size, shader, distance):
+    sc = W.sphere_scene(width=size[0], height=size[1], lon=48, lat=24, tex_size=64, shader=shader, distance=distance)
+    check(ctx, port, sc, f"{size} shader {shader} distance {distance}")
+
+
+# more clipped triangles than their records hold (65,536, or 16,384 of the no-allocation draw): the
+# winners past them re-run the clipper
+@pytest.mark.parametrize("entry,count", [("axr_draw_mesh", 50_000), ("axr_draw_mesh_noalloc", 21_000)])
+def test_clipped_records_overflow(ctx, port, entry, count):
+    sc = W.soup_scene(count=count, width=96, height=64, seed=33, edge_min=60.0, edge_max=200.0, depth_min=0.12, depth_max=50.0)
+    sc.shader = W.Shader(W.SHADER_GOURAUD)
+    vp = port.camera(sc.camera)[2]
+    fb, mesh = api.Framebuffer(ctx, sc.width, sc.height), api.Mesh.from_workload(ctx, sc.mesh)
+    fb.clearColor(0, 0, 0, 255)
+    fb.clearDepth()
+    api.TiledPipeline(ctx, api.Camera.from_matrices(vp, sc.camera.position, sc.camera.viewport), fb).setShader(api.GouraudShader())
+    api.check(getattr(ctx.lib, entry)(ctx.handle, mesh.handle, np.ascontiguousarray(sc.model, np.float32).ctypes.data), ctx.handle)
+    got = fb.read()
+    ctx.sync()
+    assert_parity(got, port.draw(sc, vp), entry)
