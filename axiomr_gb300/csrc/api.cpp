@@ -95,9 +95,9 @@ void mesh_sync_bounds(const axr_mesh* m) {
     if (cudaEventSynchronize(m->bounds_ready) != cudaSuccess) return;  // keep the previous bounds
     const MeshBounds& b = *m->bounds_host;
     for (int k = 0; k < 3; ++k)
-        m->bound_center[k] = 0.5f * (mesh_bounds_float(b.lo[k]) + mesh_bounds_float(b.hi[k]));
-    double r2;
-    std::memcpy(&r2, &b.r2, sizeof(r2));
+        m->bound_center[k] = 0.5f * (b.lo[k] + b.hi[k]);
+    double r2 = 0.0;
+    for (uint32_t k = 0; k < b.blocks; ++k) r2 = std::max(r2, b.r2[k]);
     m->bound_radius = m->num_vertices ? (float)std::sqrt(r2) * 1.0001f : 0.f;
     m->bounds_pending = false;
 }
@@ -213,23 +213,32 @@ axr_status check_mesh_desc(axr_context* ctx, const axr_mesh_desc* d) {
     return AXR_OK;
 }
 
-// Upload float3 arrays via the staging buffer and widen them to float4.
-axr_status upload_vec3(axr_context* ctx, axr_mesh* m, const float* src, float4* dst) {
-    if (!src || !dst || m->num_vertices == 0) return AXR_OK;
-    AXR_CUDA(ctx, cudaMemcpyAsync(m->staging, src, 12ull * m->num_vertices, cudaMemcpyHostToDevice, ctx->stream));
-    AXR_CUDA(ctx, launch_pack3(m->staging, dst, m->num_vertices, ctx->stream));
-    ++ctx->launches;
-    return AXR_OK;
-}
-
-axr_status upload_mesh_arrays(axr_context* ctx, axr_mesh* m, const axr_mesh_desc* d) {
-    axr_status st;
-    if ((st = upload_vec3(ctx, m, d->positions, m->pos)) != AXR_OK) return st;
-    if ((st = upload_vec3(ctx, m, d->normals, m->nrm)) != AXR_OK) return st;
-    if ((st = upload_vec3(ctx, m, d->tangents, m->tan)) != AXR_OK) return st;
-    if ((st = upload_vec3(ctx, m, d->bitangents, m->bit)) != AXR_OK) return st;
-    if (m->num_vertices)
-        AXR_CUDA(ctx, cudaMemcpyAsync(m->uv, d->uvs, 8ull * m->num_vertices, cudaMemcpyHostToDevice, ctx->stream));
+// The arrays of a mesh on their way to the device: the float3 ones into the staging area and, as
+// many at a time as it holds, widened to float4 by one kernel, which with `bounds` also starts the
+// positions' bounds.
+axr_status upload_mesh_arrays(axr_context* ctx, axr_mesh* m, const axr_mesh_desc* d, axr::MeshBounds* bounds) {
+    const size_t V = m->num_vertices;
+    if (V) {
+        const float* src[4] = {d->positions, d->normals, d->tangents, d->bitangents};
+        float4* dst[4] = {m->pos, m->nrm, m->tan, m->bit};
+        MeshPack pack{};
+        pack.n = m->num_vertices;
+        for (int k = 0; k < 4; ++k) {
+            if (src[k] && dst[k]) {
+                float* at = m->staging + 3 * V * pack.arrays;
+                pack.src[pack.arrays] = at;
+                pack.dst[pack.arrays++] = dst[k];
+                AXR_CUDA(ctx, cudaMemcpyAsync(at, src[k], 12ull * V, cudaMemcpyHostToDevice, ctx->stream));
+            }
+            if (pack.arrays && (pack.arrays == m->staging_slots || k == 3)) {
+                AXR_CUDA(ctx, launch_mesh_pack(pack, bounds ? m->staging + 3 * V * m->staging_slots : nullptr, bounds,
+                                               ctx->stream, &ctx->launches));
+                bounds = nullptr;  // of the positions, which come first
+                pack.arrays = 0;
+            }
+        }
+        AXR_CUDA(ctx, cudaMemcpyAsync(m->uv, d->uvs, 8ull * V, cudaMemcpyHostToDevice, ctx->stream));
+    }
     if (m->num_faces)
         AXR_CUDA(ctx, cudaMemcpyAsync(m->idx, d->indices, 12ull * m->num_faces, cudaMemcpyHostToDevice, ctx->stream));
     return AXR_OK;
@@ -238,7 +247,7 @@ axr_status upload_mesh_arrays(axr_context* ctx, axr_mesh* m, const axr_mesh_desc
 void free_mesh(axr_mesh* m) {
     if (!m) return;
     dfree(m->pos); dfree(m->nrm); dfree(m->tan); dfree(m->bit); dfree(m->uv); dfree(m->idx);
-    dfree(m->groups); dfree(m->materials); dfree(m->staging); dfree(m->bounds_dev);
+    dfree(m->groups); dfree(m->materials); dfree(m->staging);
     if (m->bounds_ready) {
         cudaEventSynchronize(m->bounds_ready);
         cudaEventDestroy(m->bounds_ready);
@@ -541,7 +550,8 @@ axr_status axr_mesh_create(axr_context* ctx, const axr_mesh_desc* d, axr_mesh** 
     if (d->tangents) alloc(&m->tan, V);
     if (d->bitangents) alloc(&m->bit, V);
     alloc(&m->idx, 3ull * d->num_faces);
-    alloc(&m->staging, 3ull * V);
+    m->staging_slots = 2u + (d->tangents ? 1u : 0u) + (d->bitangents ? 1u : 0u);
+    alloc(&m->staging, m->staging_floats());
     alloc(&m->groups, std::max<uint32_t>(1, d->num_groups));
     alloc(&m->materials, std::max<uint32_t>(1, d->num_materials));
     if (e != cudaSuccess) {
@@ -568,7 +578,7 @@ axr_status axr_mesh_create(axr_context* ctx, const axr_mesh_desc* d, axr_mesh** 
         dm.ao = dev_texture(md.ao);
         dm.specular_exponent = md.specular_exponent;
     }
-    st = upload_mesh_arrays(ctx, m, d);
+    st = upload_mesh_arrays(ctx, m, d, nullptr);
     if (st == AXR_OK) {
         e = cudaMemcpyAsync(m->groups, groups.data(), groups.size() * sizeof(DevGroup), cudaMemcpyHostToDevice,
                             ctx->stream);
@@ -601,27 +611,22 @@ axr_status axr_mesh_update(axr_context* ctx, axr_mesh* m, const axr_mesh_desc* d
     if (d->num_faces && !d->indices) return fail(ctx, AXR_E_INVALID, "mesh update needs indices");
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard g(ctx->device);
-    axr_status st = upload_mesh_arrays(ctx, m, d);
-    if (st != AXR_OK) return st;
     // the bounding sphere of the new positions: a host pass for a small mesh (a few us);
     // for a large one on the device behind the upload (a host pass over a million vertices
     // takes milliseconds), which batch planning waits for if it must
     if (m->num_vertices <= kHostBoundsMaxVertices) {
+        axr_status st = upload_mesh_arrays(ctx, m, d, nullptr);
+        if (st != AXR_OK) return st;
         mesh_bounds(d->positions, d->num_vertices, m->bound_center, &m->bound_radius);
         m->bounds_pending = false;
         return AXR_OK;
     }
-    if (!m->bounds_dev) {
-        AXR_CUDA(ctx, cudaMalloc(&m->bounds_dev, sizeof(MeshBounds)));
-        AXR_CUDA(ctx, cudaMallocHost(&m->bounds_host, sizeof(MeshBounds)));
-        AXR_CUDA(ctx, cudaEventCreateWithFlags(&m->bounds_ready, cudaEventDisableTiming));
-    }
-    AXR_CUDA(ctx, launch_mesh_bounds(m->pos, m->num_vertices, m->bounds_dev, ctx->stream));
-    AXR_CUDA(ctx, cudaMemcpyAsync(m->bounds_host, m->bounds_dev, sizeof(MeshBounds), cudaMemcpyDeviceToHost,
-                                  ctx->stream));
+    if (!m->bounds_host) AXR_CUDA(ctx, cudaMallocHost(&m->bounds_host, sizeof(MeshBounds)));
+    if (!m->bounds_ready) AXR_CUDA(ctx, cudaEventCreateWithFlags(&m->bounds_ready, cudaEventDisableTiming));
+    axr_status st = upload_mesh_arrays(ctx, m, d, m->bounds_host);
+    if (st != AXR_OK) return st;
     AXR_CUDA(ctx, cudaEventRecord(m->bounds_ready, ctx->stream));
     m->bounds_pending = true;
-    ctx->launches += m->num_vertices ? 2 : 0;
     return AXR_OK;
 }
 

@@ -41,16 +41,20 @@ struct axr_mesh {
     uint32_t* idx = nullptr;
     DevGroup* groups = nullptr;
     DevMaterial* materials = nullptr;
-    float* staging = nullptr;  // packed float3 upload area for updates
+    // upload area: room for staging_slots packed float3 arrays, then the bounds' partial boxes
+    float* staging = nullptr;
+    uint32_t staging_slots = 1;
+    size_t staging_floats() const {
+        return 3 * (size_t)staging_slots * num_vertices + 6 * (size_t)axr::kBoundsBlocks;
+    }
     uint32_t num_vertices = 0, num_faces = 0, num_groups = 0, num_materials = 0, num_drawn = 0;
     int device = 0;
     // bounding sphere of the positions (batch planning): from the host arrays at creation;
-    // after axr_mesh_update computed on the device on the update's stream and copied into
-    // bounds_host behind bounds_ready (read through mesh_sync_bounds)
+    // after axr_mesh_update computed on the device on the update's stream, straight into
+    // bounds_host, which holds them behind bounds_ready (read through mesh_sync_bounds)
     mutable float bound_center[3] = {0.f, 0.f, 0.f};
     mutable float bound_radius = 0.f;
     mutable bool bounds_pending = false;
-    axr::MeshBounds* bounds_dev = nullptr;
     axr::MeshBounds* bounds_host = nullptr;  // pinned
     cudaEvent_t bounds_ready = nullptr;
 };

@@ -98,11 +98,13 @@ struct LargeItem {
 constexpr uint32_t kNoItem = 0xFFFFFFFFu;
 
 // Bounding box and squared bounding-sphere radius of a mesh's positions, computed on the
-// device after an update: lo/hi as order-preserving integers (see kernels.cu), r2 the
-// largest squared distance (double) from the box centre.
+// device after an update: lo/hi, and per block of the radius kernel the largest squared distance
+// (double) from the box centre.
+constexpr uint32_t kBoundsBlocks = 512;  // most blocks of the pack and radius kernels
 struct MeshBounds {
-    uint32_t lo[3], hi[3];
-    unsigned long long r2;  // bits of a non-negative double
+    float lo[3], hi[3];
+    uint32_t blocks, pad_;
+    double r2[kBoundsBlocks];
 };
 
 // Work counters of one draw: the first kCountersReset bytes are zeroed before every draw (by the

@@ -389,7 +389,7 @@ extern "C" axr_status axr_mesh_create_from_obj(axr_context* ctx, const axr_obj_d
     if (e == cudaSuccess) e = dmalloc(&m->bit, nv);
     if (e == cudaSuccess) e = dmalloc(&m->uv, nv);
     if (e == cudaSuccess) e = dmalloc(&m->idx, 3ull * nf);
-    if (e == cudaSuccess) e = dmalloc(&m->staging, 3ull * nv);
+    if (e == cudaSuccess) e = dmalloc(&m->staging, m->staging_floats());
     if (e == cudaSuccess) e = dmalloc(&m->groups, std::max<uint32_t>(1, d->num_groups));
     if (e == cudaSuccess) e = dmalloc(&m->materials, std::max<uint32_t>(1, d->num_materials));
     float4 *ft = nullptr, *fb = nullptr;

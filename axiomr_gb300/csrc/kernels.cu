@@ -291,12 +291,6 @@ __global__ void fill_u64_kernel(unsigned long long* dst, size_t n, unsigned long
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) dst[i] = v;
 }
 
-__global__ void pack3_kernel(const float* __restrict__ src, float4* __restrict__ dst, uint32_t n) {
-    uint32_t stride = gridDim.x * blockDim.x;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-        dst[i] = make_float4(src[3ull * i], src[3ull * i + 1], src[3ull * i + 2], 0.0f);
-}
-
 __device__ void debug_emit(float* out, uint32_t* count, uint32_t cap, const Screen& s, uint32_t tag) {
     if (is_backface(s)) return;
     uint32_t slot = atomicAdd(count, 1u);
@@ -430,46 +424,83 @@ cudaError_t launch_fill_u64(unsigned long long* dst, size_t n, unsigned long lon
     return cudaGetLastError();
 }
 
-// ---- mesh bounds after an update (batch planning's density classes)
-__device__ __forceinline__ uint32_t float_ord(float f) {
-    const uint32_t u = __float_as_uint(f);
-    return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
-}
-__device__ __forceinline__ float ord_float(uint32_t o) {
-    return __uint_as_float((o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o);
-}
+// ---- mesh uploads: float3 arrays widened to float4, with the positions' bounds after an update
+// (batch planning's density classes, clip-free draws). One kernel for all arrays, each block's box
+// in memory instead of atomics on a cleared word, and the result written to the host's memory: a
+// copy, a kernel and a memset each, one after another, cost more than their work (65k-vertex
+// mesh updated and drawn: 160 to 112 us).
+constexpr int kPackBlock = 256;
 
-__global__ void mesh_box_kernel(const float4* __restrict__ pos, uint32_t n, MeshBounds* out) {
+__global__ void __launch_bounds__(kPackBlock) mesh_pack_kernel(const __grid_constant__ MeshPack p, float* partial) {
+    pdl_release();
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p = __ldg(pos + i);
-        const float v[3] = {p.x, p.y, p.z};
+    for (uint32_t i = blockIdx.x * kPackBlock + threadIdx.x; i < p.n; i += gridDim.x * kPackBlock) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-            lo[k] = fminf(lo[k], v[k]);
-            hi[k] = fmaxf(hi[k], v[k]);
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (k >= p.arrays) break;
+            const float* s = p.src[k] + 3ull * i;
+            const float v[3] = {s[0], s[1], s[2]};
+            p.dst[k][i] = make_float4(v[0], v[1], v[2], 0.0f);
+            if (k == 0) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    lo[d] = fminf(lo[d], v[d]);
+                    hi[d] = fmaxf(hi[d], v[d]);
+                }
+            }
         }
     }
+    if (!partial) return;
+    __shared__ float s_box[kPackBlock / 32][6];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) {
+    for (int d = 0; d < 3; ++d) {
         for (int o = 16; o > 0; o >>= 1) {
-            lo[k] = fminf(lo[k], __shfl_xor_sync(0xFFFFFFFFu, lo[k], o));
-            hi[k] = fmaxf(hi[k], __shfl_xor_sync(0xFFFFFFFFu, hi[k], o));
+            lo[d] = fminf(lo[d], __shfl_xor_sync(0xFFFFFFFFu, lo[d], o));
+            hi[d] = fmaxf(hi[d], __shfl_xor_sync(0xFFFFFFFFu, hi[d], o));
         }
         if ((threadIdx.x & 31) == 0) {
-            atomicMin(&out->lo[k], float_ord(lo[k]));
-            atomicMax(&out->hi[k], float_ord(hi[k]));
+            s_box[threadIdx.x >> 5][d] = lo[d];
+            s_box[threadIdx.x >> 5][3 + d] = hi[d];
         }
+    }
+    __syncthreads();
+    if (threadIdx.x < 6) {
+        float v = s_box[0][threadIdx.x];
+        for (int w = 1; w < kPackBlock / 32; ++w)
+            v = threadIdx.x < 3 ? fminf(v, s_box[w][threadIdx.x]) : fmaxf(v, s_box[w][threadIdx.x]);
+        partial[6 * blockIdx.x + threadIdx.x] = v;
     }
 }
 
-__global__ void mesh_radius_kernel(const float4* __restrict__ pos, uint32_t n, MeshBounds* out) {
+// The box of all blocks, then each block's largest squared distance from its centre.
+__global__ void __launch_bounds__(kPackBlock) mesh_radius_kernel(const float4* pos, uint32_t n, const float* partial,
+                                                                 MeshBounds* out) {
+    __shared__ float s_box[6];
+    __shared__ double s_r2[kPackBlock / 32];
+    pdl_wait();
+    if (threadIdx.x < 192) {  // a warp per bound
+        const uint32_t d = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        float v = d < 3 ? INFINITY : -INFINITY;
+        for (uint32_t b = lane; b < gridDim.x; b += 32) {
+            const float w = partial[6 * b + d];
+            v = d < 3 ? fminf(v, w) : fmaxf(v, w);
+        }
+        for (int o = 16; o > 0; o >>= 1) {
+            const float w = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+            v = d < 3 ? fminf(v, w) : fmaxf(v, w);
+        }
+        if (lane == 0) {
+            s_box[d] = v;
+            if (blockIdx.x == 0) (d < 3 ? out->lo : out->hi)[d % 3] = v;
+        }
+    }
+    __syncthreads();
     float c[3];
 #pragma unroll
-    for (int k = 0; k < 3; ++k) c[k] = __fmul_rn(0.5f, __fadd_rn(ord_float(out->lo[k]), ord_float(out->hi[k])));
+    for (int k = 0; k < 3; ++k) c[k] = __fmul_rn(0.5f, __fadd_rn(s_box[k], s_box[3 + k]));
     double r2 = 0.0;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 p = __ldg(pos + i);
+    for (uint32_t i = blockIdx.x * kPackBlock + threadIdx.x; i < n; i += gridDim.x * kPackBlock) {
+        const float4 p = pos[i];
         const float v[3] = {p.x, p.y, p.z};
         double s = 0.0;
 #pragma unroll
@@ -480,30 +511,26 @@ __global__ void mesh_radius_kernel(const float4* __restrict__ pos, uint32_t n, M
         r2 = fmax(r2, s);
     }
     for (int o = 16; o > 0; o >>= 1) r2 = fmax(r2, __shfl_xor_sync(0xFFFFFFFFu, r2, o));
-    if ((threadIdx.x & 31) == 0) atomicMax(&out->r2, (unsigned long long)__double_as_longlong(r2));
+    if ((threadIdx.x & 31) == 0) s_r2[threadIdx.x >> 5] = r2;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < kPackBlock / 32; ++w) r2 = fmax(r2, s_r2[w]);
+        out->r2[blockIdx.x] = r2;
+        if (blockIdx.x == 0) out->blocks = gridDim.x;
+    }
 }
 
-cudaError_t launch_mesh_bounds(const float4* pos, uint32_t n, MeshBounds* out, cudaStream_t stream) {
-    cudaError_t e = cudaMemsetAsync(out->lo, 0xFF, sizeof(out->lo), stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(out->hi, 0, sizeof(out->hi) + sizeof(out->r2), stream);
-    if (e != cudaSuccess || n == 0) return e;
-    const unsigned g = grid_for(n, 256, 1024);
-    mesh_box_kernel<<<g, 256, 0, stream>>>(pos, n, out);
-    mesh_radius_kernel<<<g, 256, 0, stream>>>(pos, n, out);
-    return cudaGetLastError();
-}
-
-float mesh_bounds_float(uint32_t o) {
-    const uint32_t u = (o & 0x80000000u) ? (o & 0x7FFFFFFFu) : ~o;
-    float f;
-    std::memcpy(&f, &u, sizeof(f));
-    return f;
-}
-
-cudaError_t launch_pack3(const float* src, float4* dst, uint32_t n, cudaStream_t stream) {
-    if (n == 0) return cudaSuccess;
-    pack3_kernel<<<grid_for(n, 256, 4096), 256, 0, stream>>>(src, dst, n);
-    return cudaGetLastError();
+cudaError_t launch_mesh_pack(const MeshPack& p, float* partial, MeshBounds* bounds, cudaStream_t stream, uint64_t* launches) {
+    if (p.n == 0) return cudaSuccess;
+    const unsigned g = grid_for(p.n, kPackBlock, kBoundsBlocks);
+    mesh_pack_kernel<<<g, kPackBlock, 0, stream>>>(p, partial);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    *launches += 1;
+    if (!partial) return cudaSuccess;
+    *launches += 1;
+    return launch_dependent(mesh_radius_kernel, g, (unsigned)kPackBlock, stream, (const float4*)p.dst[0], p.n,
+                            (const float*)partial, bounds);
 }
 
 cudaError_t launch_debug_triangles(const DrawParams& p, float* out, uint32_t* count, uint32_t capacity,

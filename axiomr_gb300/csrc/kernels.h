@@ -37,14 +37,17 @@ cudaError_t launch_draw(const DrawParams& p, const LaunchConfig& cfg, cudaStream
 cudaError_t launch_clear(uint32_t* color, float* depth, size_t pixels, uint32_t bgra, float depth_value,
                          bool do_color, bool do_depth, cudaStream_t stream);
 cudaError_t launch_fill_u64(unsigned long long* dst, size_t n, unsigned long long v, cudaStream_t stream);
-// float3 (packed) -> float4 (x, y, z, 0)
-cudaError_t launch_pack3(const float* src, float4* dst, uint32_t n, cudaStream_t stream);
-// Bounds of pos[0, n) into *out (device); the box centre and squared radius follow the
-// host's mesh_bounds operation for operation.
-cudaError_t launch_mesh_bounds(const float4* pos, uint32_t n, MeshBounds* out, cudaStream_t stream);
-// The float an order-preserving integer of launch_mesh_bounds stands for.
-float mesh_bounds_float(uint32_t ord);
-// RGBA8 bytes of a uint32 array (no conversion needed; provided for symmetry)
+// The packed float3 arrays of a mesh upload -> float4 (x, y, z, 0), src[k] to dst[k] for the first
+// `arrays` (src[0]: positions). With `partial` (6 * kBoundsBlocks floats on the device) also the
+// positions' bounds into *bounds (pinned host memory, complete when the stream gets past); the
+// box centre and squared radius follow the host's mesh_bounds operation for operation. Adds the
+// number of kernels launched to *launches.
+struct MeshPack {
+    const float* src[4];
+    float4* dst[4];
+    uint32_t n, arrays;
+};
+cudaError_t launch_mesh_pack(const MeshPack& p, float* partial, MeshBounds* bounds, cudaStream_t stream, uint64_t* launches);
 
 // Stage dump for parity tests: every triangle that survives clip + cull, unordered, as
 // (tag, screen x0 y0 x1 y1 x2 y2, ndcZ0..2, minX, minY, maxX, maxY) = 14 words.
