@@ -87,18 +87,20 @@ bool mesh_clip_free(const axr_mesh* m, const float mvp[16]) {
     return true;
 }
 
+void take_bounds(const axr_mesh* m, const MeshBounds& b) {
+    double r2 = 0.0;
+    for (uint32_t k = 0; k < b.blocks; ++k) r2 = std::max(r2, b.r2[k]);
+    for (int k = 0; k < 3; ++k) m->bound_center[k] = b.blocks ? 0.5f * (b.lo[k] + b.hi[k]) : 0.f;
+    m->bound_radius = b.blocks ? (float)std::sqrt(r2) * 1.0001f : 0.f;
+}
+
 void mesh_sync_bounds(const axr_mesh* m) {
     static std::mutex mu;  // planners on several threads may share a mesh
     if (!m) return;
     std::lock_guard<std::mutex> lk(mu);
     if (!m->bounds_pending) return;
     if (cudaEventSynchronize(m->bounds_ready) != cudaSuccess) return;  // keep the previous bounds
-    const MeshBounds& b = *m->bounds_host;
-    for (int k = 0; k < 3; ++k)
-        m->bound_center[k] = 0.5f * (b.lo[k] + b.hi[k]);
-    double r2 = 0.0;
-    for (uint32_t k = 0; k < b.blocks; ++k) r2 = std::max(r2, b.r2[k]);
-    m->bound_radius = m->num_vertices ? (float)std::sqrt(r2) * 1.0001f : 0.f;
+    take_bounds(m, *m->bounds_host);
     m->bounds_pending = false;
 }
 
@@ -246,8 +248,13 @@ axr_status upload_mesh_arrays(axr_context* ctx, axr_mesh* m, const axr_mesh_desc
 
 void free_mesh(axr_mesh* m) {
     if (!m) return;
-    dfree(m->pos); dfree(m->nrm); dfree(m->tan); dfree(m->bit); dfree(m->uv); dfree(m->idx);
-    dfree(m->groups); dfree(m->materials); dfree(m->staging);
+    if (m->mem) {
+        dfree(m->groups);  // with the materials; waits for draws in flight, which freeing pool memory does not
+        cudaFree(m->mem);
+    } else {
+        dfree(m->pos); dfree(m->nrm); dfree(m->tan); dfree(m->bit); dfree(m->uv); dfree(m->idx);
+        dfree(m->groups); dfree(m->materials); dfree(m->staging);
+    }
     if (m->bounds_ready) {
         cudaEventSynchronize(m->bounds_ready);
         cudaEventDestroy(m->bounds_ready);
@@ -393,6 +400,8 @@ void axr_context_destroy(axr_context* ctx) {
     free_scratch(ctx);
     free_bins(ctx);
     free_png(ctx);
+    if (ctx->ingest_host) cudaFreeHost(ctx->ingest_host);
+    if (ctx->ingest_pool) cudaMemPoolDestroy(ctx->ingest_pool);  // its meshes may outlive it
     for (int k = 0; k < axr_context::kCopyStreams; ++k) {
         if (ctx->copy_stream[k]) {
             cudaStreamSynchronize(ctx->copy_stream[k]);

@@ -17,6 +17,14 @@
 
 namespace axr_internal {
 struct PngState;  // scratch of the PNG encoder (encode.cu)
+
+// What the OBJ ingest's kernels report to the host (pinned, one per context).
+struct IngestHost {
+    uint32_t vertices;   // distinct vertices
+    uint32_t first_bad;  // first corner that names no position; all-ones: none
+    axr::MeshBounds bounds;
+};
+constexpr uint64_t kIngestKept = 256ull << 20;  // most bytes a context's ingest pool keeps between calls
 }
 
 using axr::DevCounters;
@@ -33,6 +41,7 @@ struct axr_texture {
 };
 
 struct axr_mesh {
+    void* mem = nullptr;  // an ingested mesh: the pool allocation of its arrays (materials share the groups')
     float4* pos = nullptr;
     float4* nrm = nullptr;
     float4* tan = nullptr;
@@ -164,6 +173,8 @@ struct axr_context {
     size_t events_used = 0;
     uint64_t launches = 0;
     axr_internal::PngState* png = nullptr;
+    axr_internal::IngestHost* ingest_host = nullptr;
+    cudaMemPool_t ingest_pool = nullptr;
 };
 
 namespace axr {

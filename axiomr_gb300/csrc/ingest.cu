@@ -10,11 +10,17 @@
 //   insert          open-addressing hash table of corner indices; a slot keeps the smallest
 //                   corner index of its key (atomicMin), i.e. the key's first appearance
 //   first_flags     a corner is a vertex's first appearance when its slot holds itself
-//   scan            exclusive prefix sum of the flags: vertex numbers in appearance order
+//   scan            exclusive prefix sum of the flags: vertex numbers in appearance order (and
+//                   polygon offsets from their sizes)
 //   emit_vertices / fan_faces / face_frames / incidence + vertex_frames
 // The per-vertex sums run in face order (each vertex's incident (face, corner) entries are
 // sorted before summing), so every float is the reference's. The text itself is parsed on
-// the host (the reference's parser, or any other that produces the same pools).
+// the host (the reference's parser, or any other that produces the same pools). Of a
+// 65k-triangle model's call the kernels are 150 us; the rest was allocations (19 stream-ordered ones from
+// a pool that every synchronisation emptied, 9 plain ones and their frees) and host passes over
+// corners and positions. Now: one allocation for the scratch and one for the arrays, from a pool that
+// the context keeps, and those passes on the device (model ingested and its first 800x600 frame drawn:
+// 1070 to 264 us).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -61,12 +67,18 @@ __device__ __forceinline__ uint32_t key_hash(const Key& k) {
     return h;
 }
 
-__global__ void corner_keys_kernel(const float* __restrict__ pos, const float* __restrict__ uv, uint32_t n_uv,
+// A corner that names no position (the caller is told of the first) gets the pool's first one.
+__global__ void corner_keys_kernel(const float* __restrict__ pos, uint32_t n_pos, const float* __restrict__ uv, uint32_t n_uv,
                                    const float* __restrict__ nrm, uint32_t n_nrm, const int* __restrict__ corners,
-                                   uint32_t nc, Key* keys) {
+                                   uint32_t nc, Key* keys, uint32_t* first_bad) {
     const uint32_t c = blockIdx.x * kBlock + threadIdx.x;
     if (c >= nc) return;
-    const int v = corners[3 * (size_t)c], t = corners[3 * (size_t)c + 1], n = corners[3 * (size_t)c + 2];
+    int v = corners[3 * (size_t)c], t = corners[3 * (size_t)c + 1], n = corners[3 * (size_t)c + 2];
+    if (v < 0 || (uint32_t)v >= n_pos) {
+        atomicMin(first_bad, c);
+        if (n_pos == 0) return;  // no vertex comes of it: the call fails
+        v = 0;
+    }
     const bool tv = t >= 0 && (uint32_t)t < n_uv, nv = n >= 0 && (uint32_t)n < n_nrm;
     Key k;
     k.a = make_float4(pos[3 * (size_t)v], pos[3 * (size_t)v + 1], pos[3 * (size_t)v + 2], tv ? uv[2 * (size_t)t] : 0.0f);
@@ -114,61 +126,71 @@ __global__ void first_flags_kernel(const Key* keys, int* table, uint32_t mask, u
     first[c] = r == c ? 1u : 0u;
 }
 
-// ---- exclusive prefix sum (block scans + a scan of the block totals)
+// ---- exclusive prefix sum: block scans, then each block adds the totals of the blocks before it
 constexpr int kScanBlock = 1024;
 
-__global__ void scan_block_kernel(uint32_t* data, uint32_t n, uint32_t* block_sums) {
-    __shared__ uint32_t warp_sums[kScanBlock / 32];
-    const uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
-    const uint32_t x = i < n ? data[i] : 0u;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t incl = x;
+__device__ __forceinline__ uint32_t warp_inclusive(uint32_t x, int lane) {
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, incl, o);
-        if (lane >= o) incl += y;
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+        if (lane >= o) x += y;
     }
+    return x;
+}
+
+// dst (may be src): each block's own exclusive sums; the block's total to block_sums. kFan: the
+// elements are polygon sizes and count as their fan's triangles.
+template <bool kFan>
+__global__ void scan_block_kernel(const uint32_t* src, uint32_t* dst, uint32_t n, uint32_t* block_sums) {
+    __shared__ uint32_t warp_sums[kScanBlock / 32];
+    const uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
+    uint32_t x = i < n ? src[i] : 0u;
+    if (kFan) x = x >= 3u ? x - 2u : 0u;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t incl = warp_inclusive(x, lane);
     if (lane == 31) warp_sums[warp] = incl;
     __syncthreads();
-    if (warp == 0) {
-        uint32_t s = lane < kScanBlock / 32 ? warp_sums[lane] : 0u;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, s, o);
-            if (lane >= o) s += y;
-        }
-        if (lane < kScanBlock / 32) warp_sums[lane] = s;  // inclusive over warps
-    }
+    if (warp == 0) warp_sums[lane] = warp_inclusive(warp_sums[lane], lane);  // inclusive over warps
     __syncthreads();
-    const uint32_t before = (warp > 0 ? warp_sums[warp - 1] : 0u) + incl - x;
-    if (i < n) data[i] = before;
-    if (threadIdx.x == kScanBlock - 1 && block_sums) block_sums[blockIdx.x] = warp_sums[kScanBlock / 32 - 1];
+    if (i < n) dst[i] = (warp > 0 ? warp_sums[warp - 1] : 0u) + incl - x;
+    if (threadIdx.x == 0) block_sums[blockIdx.x] = warp_sums[kScanBlock / 32 - 1];
 }
 
-__global__ void scan_add_kernel(uint32_t* data, uint32_t n, const uint32_t* block_offsets) {
+// Block b adds the totals of the blocks before it (a model of 1M corners has 1000);
+// `host`: the total (the last element's prefix and `last`, the element itself) and *first_bad go
+// there.
+__global__ void scan_add_kernel(uint32_t* data, uint32_t n, const uint32_t* block_sums, const uint32_t* last,
+                                const uint32_t* first_bad, IngestHost* host) {
+    __shared__ uint32_t warp_sums[kScanBlock / 32];
+    uint32_t v = 0;
+    for (uint32_t b = threadIdx.x; b < blockIdx.x; b += kScanBlock) v += block_sums[b];
+    v = __reduce_add_sync(0xFFFFFFFFu, v);
+    if ((threadIdx.x & 31) == 0) warp_sums[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = __reduce_add_sync(0xFFFFFFFFu, warp_sums[threadIdx.x & 31]);
     const uint32_t i = blockIdx.x * kScanBlock + threadIdx.x;
-    if (i < n) data[i] += block_offsets[blockIdx.x];
+    if (i < n) {
+        const uint32_t p = data[i] + v;
+        data[i] = p;
+        if (host && i == n - 1) {
+            host->vertices = p + *last;
+            host->first_bad = *first_bad;
+        }
+    }
 }
 
-cudaError_t scan_exclusive(uint32_t* data, uint32_t n, cudaStream_t st) {
+uint32_t scan_blocks(size_t n) { return (uint32_t)((n + kScanBlock - 1) / kScanBlock); }
+
+// Exclusive sums of src[0, n) into dst; sums: scan_blocks(n) words of scratch.
+template <bool kFan = false>
+cudaError_t scan_exclusive(const uint32_t* src, uint32_t* dst, uint32_t n, uint32_t* sums, cudaStream_t st,
+                           const uint32_t* last = nullptr, const uint32_t* first_bad = nullptr,
+                           IngestHost* host = nullptr) {
     if (n == 0) return cudaSuccess;
-    const uint32_t blocks = (n + kScanBlock - 1) / kScanBlock;
-    if (blocks == 1) {
-        scan_block_kernel<<<1, kScanBlock, 0, st>>>(data, n, nullptr);
-        return cudaGetLastError();
-    }
-    uint32_t* sums = nullptr;
-    cudaError_t e = cudaMallocAsync(&sums, sizeof(uint32_t) * blocks, st);
-    if (e != cudaSuccess) return e;
-    scan_block_kernel<<<blocks, kScanBlock, 0, st>>>(data, n, sums);
-    e = cudaGetLastError();
-    if (e == cudaSuccess) e = scan_exclusive(sums, blocks, st);
-    if (e == cudaSuccess) {
-        scan_add_kernel<<<blocks, kScanBlock, 0, st>>>(data, n, sums);
-        e = cudaGetLastError();
-    }
-    cudaFreeAsync(sums, st);
-    return e;
+    const uint32_t blocks = scan_blocks(n);
+    scan_block_kernel<kFan><<<blocks, kScanBlock, 0, st>>>(src, dst, n, sums);
+    if (blocks > 1 || host) scan_add_kernel<<<blocks, kScanBlock, 0, st>>>(dst, n, sums, last, first_bad, host);
+    return cudaGetLastError();
 }
 
 // first corners -> vertex arrays (position, uv, normal); every corner -> its vertex number
@@ -186,7 +208,7 @@ __global__ void emit_vertices_kernel(const Key* keys, const uint32_t* first, con
     nrm[v] = make_float4(k.b.y, k.b.z, k.b.w, 0.0f);
 }
 
-// polygon p (corner offset, face offset from the host) -> its fan (c0, ci, ci+1)
+// polygon p (corner offset, face offset) -> its fan (c0, ci, ci+1)
 __global__ void fan_faces_kernel(const uint32_t* vid, const uint32_t* poly_corner, const uint32_t* poly_face,
                                  const uint32_t* poly_size, uint32_t np, uint32_t* idx) {
     const uint32_t p = blockIdx.x * kBlock + threadIdx.x;
@@ -291,117 +313,163 @@ extern "C" axr_status axr_mesh_create_from_obj(axr_context* ctx, const axr_obj_d
         (d->num_corners && !d->corners) || (d->num_polygons && !d->polygon_sizes) ||
         (d->num_groups && !d->groups) || (d->num_materials && !d->materials))
         return fail(ctx, AXR_E_INVALID, "OBJ descriptor arrays missing");
-    // host side: polygon offsets (corners and faces), checks
     const uint32_t nc = d->num_corners, np = d->num_polygons;
-    std::vector<uint32_t> poly_corner(np), poly_face(np);
     uint64_t corners = 0, faces = 0;
     for (uint32_t p = 0; p < np; ++p) {
-        poly_corner[p] = (uint32_t)corners;
-        poly_face[p] = (uint32_t)faces;
-        corners += d->polygon_sizes[p];
-        if (d->polygon_sizes[p] >= 3) faces += d->polygon_sizes[p] - 2;
+        const uint32_t k = d->polygon_sizes[p];
+        corners += k;
+        faces += k >= 3u ? k - 2u : 0u;
     }
     if (corners != nc) return fail(ctx, AXR_E_INVALID, "polygon sizes add up to %llu corners, not %u",
                                    (unsigned long long)corners, nc);
     if (faces > kMaxOrdinal + 1ull) return fail(ctx, AXR_E_CAPACITY, "a draw is limited to %u faces", kMaxOrdinal + 1u);
-    for (uint64_t i = 0; i < nc; ++i)
-        if (d->corners[3 * i] < 0 || (uint32_t)d->corners[3 * i] >= d->num_positions)
-            return fail(ctx, AXR_E_INVALID, "corner %llu names position %d of %u", (unsigned long long)i,
-                        d->corners[3 * i], d->num_positions);
+    // the corners' positions are checked on the device with the keys; here only where another
+    // fault would be reported before theirs
+    auto bad_corner = [&](uint64_t i) {
+        return fail(ctx, AXR_E_INVALID, "corner %llu names position %d of %u", (unsigned long long)i, d->corners[3 * i],
+                    d->num_positions);
+    };
+    auto check_corners = [&]() -> axr_status {
+        for (uint64_t i = 0; i < nc; ++i)
+            if (d->corners[3 * i] < 0 || (uint32_t)d->corners[3 * i] >= d->num_positions) return bad_corner(i);
+        return AXR_OK;
+    };
     const uint32_t nf = (uint32_t)faces;
-    uint64_t drawn = 0;
     for (uint32_t g = 0; g < d->num_groups; ++g) {
-        if ((uint64_t)d->groups[g].start_face + d->groups[g].face_count > nf)
-            return fail(ctx, AXR_E_INVALID, "group %u covers faces beyond the mesh", g);
-        if (d->groups[g].material >= d->num_materials)
-            return fail(ctx, AXR_E_INVALID, "group %u names material %u of %u", g, d->groups[g].material,
-                        d->num_materials);
-        drawn += d->groups[g].face_count;
+        const bool beyond = (uint64_t)d->groups[g].start_face + d->groups[g].face_count > nf;
+        if (!beyond && d->groups[g].material < d->num_materials) continue;
+        axr_status st = check_corners();
+        if (st != AXR_OK) return st;
+        if (beyond) return fail(ctx, AXR_E_INVALID, "group %u covers faces beyond the mesh", g);
+        return fail(ctx, AXR_E_INVALID, "group %u names material %u of %u", g, d->groups[g].material, d->num_materials);
     }
     std::lock_guard<std::mutex> lk(ctx->mu);
     DeviceGuard g(ctx->device);
     cudaStream_t st = ctx->stream;
     uint32_t cap = 16;
     while (cap < 2u * std::max<uint32_t>(nc, 1u)) cap <<= 1;
+    if (!ctx->ingest_host) AXR_CUDA(ctx, cudaMallocHost(&ctx->ingest_host, sizeof(IngestHost)));
+    if (!ctx->ingest_pool) {
+        // the context's own pool: what it keeps between calls (at most kIngestKept bytes; without it
+        // every call maps fresh memory) goes back when the context is destroyed and the last mesh in
+        // it is gone
+        cudaMemPoolProps props{};
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = ctx->device;
+        AXR_CUDA(ctx, cudaMemPoolCreate(&ctx->ingest_pool, &props));
+        uint64_t keep = kIngestKept;
+        AXR_CUDA(ctx, cudaMemPoolSetAttribute(ctx->ingest_pool, cudaMemPoolAttrReleaseThreshold, &keep));
+    }
 
-    // device inputs and scratch
-    float *dpos = nullptr, *duv = nullptr, *dnrm = nullptr;
-    int* dcorners = nullptr;
-    uint32_t *dpc = nullptr, *dpf = nullptr, *dps = nullptr;
-    Key* keys = nullptr;
-    int* table = nullptr;
-    uint32_t *first = nullptr, *prefix = nullptr, *rep = nullptr, *vid = nullptr;
-    cudaError_t e = cudaSuccess;
-    auto alloc = [&](auto** p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(p), std::max<size_t>(bytes, 16), st);
+    // device inputs and scratch in one allocation (vertices: at most one per corner)
+    size_t bytes = 0;
+    auto place = [&](size_t n) {
+        const size_t at = bytes;
+        bytes += (std::max<size_t>(n, 16) + 255) & ~size_t(255);
+        return at;
     };
-    auto put = [&](void* dst, const void* src, size_t bytes) {
-        if (e == cudaSuccess && bytes) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st);
+    const uint32_t sums_n = std::max({scan_blocks(nc), scan_blocks(np), 1u});
+    const size_t o_pos = place(12ull * d->num_positions), o_uv = place(8ull * d->num_uvs), o_nrm = place(12ull * d->num_normals);
+    const size_t o_corners = place(12ull * nc), o_sizes = place(4ull * np), o_pc = place(4ull * np), o_pf = place(4ull * np);
+    const size_t o_keys = place(sizeof(Key) * nc), o_table = place(4ull * cap + 4), o_first = place(4ull * nc);
+    const size_t o_prefix = place(4ull * nc), o_rep = place(4ull * nc), o_vid = place(4ull * nc), o_sums = place(4ull * sums_n);
+    const size_t o_ft = place(16ull * nf), o_fb = place(16ull * nf), o_entries = place(12ull * nf);
+    const size_t o_count = place(4ull * nc), o_cursor = place(4ull * nc), o_offset = place(4ull * nc);  // count, cursor: zeroed together
+    const size_t o_pool4 = place(16ull * d->num_positions), o_partial = place(24ull * kBoundsBlocks);
+    unsigned char* mem = nullptr;
+    cudaError_t e = cudaMallocFromPoolAsync(reinterpret_cast<void**>(&mem), bytes, ctx->ingest_pool, st);
+    auto at = [&](auto* type, size_t offset) { return reinterpret_cast<decltype(type)>(mem + offset); };
+    float *dpos = at((float*)nullptr, o_pos), *duv = at((float*)nullptr, o_uv), *dnrm = at((float*)nullptr, o_nrm);
+    int *dcorners = at((int*)nullptr, o_corners), *table = at((int*)nullptr, o_table);
+    Key* keys = at((Key*)nullptr, o_keys);
+    auto words = [&](size_t offset) { return at((uint32_t*)nullptr, offset); };
+    uint32_t *dps = words(o_sizes), *dpc = words(o_pc), *dpf = words(o_pf), *first = words(o_first), *prefix = words(o_prefix),
+             *rep = words(o_rep), *vid = words(o_vid), *sums = words(o_sums), *count = words(o_count),
+             *cursor = words(o_cursor), *offset = words(o_offset), *entries = words(o_entries);
+    float4 *ft = at((float4*)nullptr, o_ft), *fb = at((float4*)nullptr, o_fb);
+    auto put = [&](void* dst, const void* src, size_t n) {
+        if (e == cudaSuccess && n) e = cudaMemcpyAsync(dst, src, n, cudaMemcpyHostToDevice, st);
     };
-    alloc(&dpos, 12ull * d->num_positions);
-    alloc(&duv, 8ull * d->num_uvs);
-    alloc(&dnrm, 12ull * d->num_normals);
-    alloc(&dcorners, 12ull * nc);
-    alloc(&dpc, 4ull * np);
-    alloc(&dpf, 4ull * np);
-    alloc(&dps, 4ull * np);
-    alloc(&keys, sizeof(Key) * nc);
-    alloc(&table, 4ull * cap);
-    alloc(&first, 4ull * nc);
-    alloc(&prefix, 4ull * nc);
-    alloc(&rep, 4ull * nc);
-    alloc(&vid, 4ull * nc);
+    IngestHost* host = ctx->ingest_host;  // written by the kernels
+    host->first_bad = 0xFFFFFFFFu;
+    host->vertices = 0;
+    uint32_t* first_bad = words(o_table) + cap;  // all-ones with the table
     put(dpos, d->positions, 12ull * d->num_positions);
+    // bounding sphere for batch planning: over the position pool (a superset of the vertices)
+    host->bounds.blocks = 0;
+    if (e == cudaSuccess && d->num_positions) {
+        MeshPack pack{};
+        pack.src[0] = dpos;
+        pack.dst[0] = at((float4*)nullptr, o_pool4);
+        pack.n = d->num_positions;
+        pack.arrays = 1;
+        e = launch_mesh_pack(pack, at((float*)nullptr, o_partial), &host->bounds, st, &ctx->launches);
+    }
     put(duv, d->uvs, 8ull * d->num_uvs);
     put(dnrm, d->normals, 12ull * d->num_normals);
     put(dcorners, d->corners, 12ull * nc);
-    put(dpc, poly_corner.data(), 4ull * np);
-    put(dpf, poly_face.data(), 4ull * np);
     put(dps, d->polygon_sizes, 4ull * np);
-    if (e == cudaSuccess) e = cudaMemsetAsync(table, 0xFF, 4ull * cap, st);
+    if (e == cudaSuccess) e = cudaMemsetAsync(table, 0xFF, 4ull * cap + 4, st);
     if (e == cudaSuccess && nc) {
-        corner_keys_kernel<<<grid(nc), kBlock, 0, st>>>(dpos, duv, d->num_uvs, dnrm, d->num_normals, dcorners, nc, keys);
+        corner_keys_kernel<<<grid(nc), kBlock, 0, st>>>(dpos, d->num_positions, duv, d->num_uvs, dnrm, d->num_normals, dcorners,
+                                                        nc, keys, first_bad);
         insert_kernel<<<grid(nc), kBlock, 0, st>>>(keys, table, cap - 1, nc);
         first_flags_kernel<<<grid(nc), kBlock, 0, st>>>(keys, table, cap - 1, nc, first, rep);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(prefix, first, 4ull * nc, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = scan_exclusive(prefix, nc, st);
+        if (e == cudaSuccess) e = scan_exclusive(first, prefix, nc, sums, st, first + nc - 1, first_bad, host);
         ctx->launches += 3;
     }
-    // vertex count = prefix[nc-1] + first[nc-1]
-    uint32_t nv = 0;
-    if (e == cudaSuccess && nc) {
-        uint32_t last[2] = {0, 0};
-        e = cudaMemcpyAsync(&last[0], prefix + nc - 1, 4, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&last[1], first + nc - 1, 4, cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        nv = last[0] + last[1];
+    cudaEvent_t counted = nullptr;  // the vertex count is on the host
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&counted, cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaEventRecord(counted, st);
+    // what does not need the count runs while the host waits for it
+    if (e == cudaSuccess && np) {
+        e = scan_exclusive(dps, dpc, np, sums, st);
+        if (e == cudaSuccess) e = scan_exclusive<true>(dps, dpf, np, sums, st);
     }
+    if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, o_offset - o_count, st);
+    if (counted) {
+        const cudaError_t w = cudaEventSynchronize(counted);
+        if (e == cudaSuccess) e = w;
+        cudaEventDestroy(counted);
+    }
+    const uint32_t nv = e == cudaSuccess ? host->vertices : 0u;
+    if (e == cudaSuccess && host->first_bad != 0xFFFFFFFFu) {
+        cudaFreeAsync(mem, st);
+        cudaStreamSynchronize(st);
+        return bad_corner(host->first_bad);
+    }
+    // the mesh's arrays in one allocation from the pool; its groups and materials in a plain one
+    // (cudaFree of which waits for what still draws the mesh, as for any other mesh)
     auto* m = new axr_mesh();
     m->device = ctx->device;
     m->num_vertices = nv;
     m->num_faces = nf;
     m->num_groups = d->num_groups;
     m->num_materials = d->num_materials;
-    if (e == cudaSuccess) e = dmalloc(&m->pos, nv);
-    if (e == cudaSuccess) e = dmalloc(&m->nrm, nv);
-    if (e == cudaSuccess) e = dmalloc(&m->tan, nv);
-    if (e == cudaSuccess) e = dmalloc(&m->bit, nv);
-    if (e == cudaSuccess) e = dmalloc(&m->uv, nv);
-    if (e == cudaSuccess) e = dmalloc(&m->idx, 3ull * nf);
-    if (e == cudaSuccess) e = dmalloc(&m->staging, m->staging_floats());
-    if (e == cudaSuccess) e = dmalloc(&m->groups, std::max<uint32_t>(1, d->num_groups));
-    if (e == cudaSuccess) e = dmalloc(&m->materials, std::max<uint32_t>(1, d->num_materials));
-    float4 *ft = nullptr, *fb = nullptr;
-    uint32_t *count = nullptr, *offset = nullptr, *cursor = nullptr, *entries = nullptr;
-    alloc(&ft, 16ull * nf);
-    alloc(&fb, 16ull * nf);
-    alloc(&count, 4ull * nv);
-    alloc(&offset, 4ull * nv);
-    alloc(&cursor, 4ull * nv);
-    alloc(&entries, 12ull * nf);
-    if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, 4ull * nv, st);
-    if (e == cudaSuccess) e = cudaMemsetAsync(cursor, 0, 4ull * nv, st);
+    const size_t ng = std::max<uint32_t>(1, d->num_groups), nm = std::max<uint32_t>(1, d->num_materials);
+    bytes = 0;
+    const size_t m_pos = place(16ull * nv), m_nrm = place(16ull * nv), m_tan = place(16ull * nv), m_bit = place(16ull * nv);
+    const size_t m_uv = place(8ull * nv), m_idx = place(12ull * nf), m_staging = place(4 * m->staging_floats());
+    const size_t mem_bytes = bytes;
+    bytes = 0;
+    const size_t m_groups = place(sizeof(DevGroup) * ng), m_mats = place(sizeof(DevMaterial) * nm);
+    unsigned char* tables = nullptr;
+    if (e == cudaSuccess) e = dmalloc(&tables, bytes);
+    if (e == cudaSuccess) e = cudaMallocFromPoolAsync(&m->mem, mem_bytes, ctx->ingest_pool, st);
+    if (e == cudaSuccess) {
+        unsigned char* b = static_cast<unsigned char*>(m->mem);
+        m->pos = reinterpret_cast<float4*>(b + m_pos);
+        m->nrm = reinterpret_cast<float4*>(b + m_nrm);
+        m->tan = reinterpret_cast<float4*>(b + m_tan);
+        m->bit = reinterpret_cast<float4*>(b + m_bit);
+        m->uv = reinterpret_cast<float2*>(b + m_uv);
+        m->idx = reinterpret_cast<uint32_t*>(b + m_idx);
+        m->staging = reinterpret_cast<float*>(b + m_staging);
+        m->groups = reinterpret_cast<DevGroup*>(tables + m_groups);
+        m->materials = reinterpret_cast<DevMaterial*>(tables + m_mats);
+    }
     if (e == cudaSuccess && nc) {
         emit_vertices_kernel<<<grid(nc), kBlock, 0, st>>>(keys, first, prefix, rep, nc, m->pos, m->uv, m->nrm, vid);
         fan_faces_kernel<<<grid(np), kBlock, 0, st>>>(vid, dpc, dpf, dps, np, m->idx);
@@ -411,8 +479,7 @@ extern "C" axr_status axr_mesh_create_from_obj(axr_context* ctx, const axr_obj_d
     if (e == cudaSuccess && nf) {
         face_frames_kernel<<<grid(nf), kBlock, 0, st>>>(m->idx, nf, m->pos, m->uv, m->nrm, ft, fb, count);
         e = cudaGetLastError();
-        if (e == cudaSuccess) e = cudaMemcpyAsync(offset, count, 4ull * nv, cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = scan_exclusive(offset, nv, st);
+        if (e == cudaSuccess) e = scan_exclusive(count, offset, nv, sums, st);
         if (e == cudaSuccess) {
             incidence_kernel<<<grid(nf), kBlock, 0, st>>>(m->idx, nf, offset, cursor, entries);
             e = cudaGetLastError();
@@ -425,14 +492,14 @@ extern "C" axr_status axr_mesh_create_from_obj(axr_context* ctx, const axr_obj_d
         ctx->launches += 1;
     }
     // groups and materials as axr_mesh_create builds them
-    std::vector<DevGroup> groups(std::max<uint32_t>(1, d->num_groups));
+    std::vector<DevGroup> groups(ng);
     uint32_t base = 0;
     for (uint32_t k = 0; k < d->num_groups; ++k) {
         groups[k] = DevGroup{d->groups[k].start_face, d->groups[k].face_count, base, d->groups[k].material};
         base += d->groups[k].face_count;
     }
     m->num_drawn = base;
-    std::vector<DevMaterial> mats(std::max<uint32_t>(1, d->num_materials));
+    std::vector<DevMaterial> mats(nm);
     for (uint32_t k = 0; k < d->num_materials; ++k) {
         const axr_material_desc& md = d->materials[k];
         DevMaterial& dm = mats[k];
@@ -455,20 +522,16 @@ extern "C" axr_status axr_mesh_create_from_obj(axr_context* ctx, const axr_obj_d
     }
     put(m->groups, groups.data(), sizeof(DevGroup) * groups.size());
     put(m->materials, mats.data(), sizeof(DevMaterial) * mats.size());
-    // bounding sphere for batch planning: over the position pool (a superset of the vertices)
-    mesh_bounds(d->positions, d->num_positions, m->bound_center, &m->bound_radius);
-    void* temps[] = {dpos, duv, dnrm, dcorners, dpc, dpf, dps, keys, table, first, prefix, rep, vid,
-                     ft, fb, count, offset, cursor, entries};
-    for (void* p : temps)
-        if (p) cudaFreeAsync(p, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+    if (mem) cudaFreeAsync(mem, st);
+    const cudaError_t done = cudaStreamSynchronize(st);  // also after a failure: kernels write to `host`
+    if (e == cudaSuccess) e = done;
     if (e != cudaSuccess) {
-        dfree(m->pos); dfree(m->nrm); dfree(m->tan); dfree(m->bit); dfree(m->uv); dfree(m->idx);
-        dfree(m->staging); dfree(m->groups); dfree(m->materials);
+        dfree(tables);
+        if (m->mem) cudaFree(m->mem);
         delete m;
         return cuda_fail(ctx, e, "mesh ingest");
     }
-    (void)drawn;
+    take_bounds(m, host->bounds);
     *out = m;
     return AXR_OK;
 }
