@@ -427,15 +427,16 @@ __global__ void __launch_bounds__(kBatchBlock, kBatchMinBlocks) batch_kernel(con
 
 // ---- phased form: one launch per phase, one CTA per work unit (large: persistent warps)
 // (the vertices, faces and large triangles of every shader kind of a launch set together).
-// Each kernel but the first starts while the one before it drains: its CTAs stage their unit, which no
-// kernel of the set writes, and wait there.
+// Each kernel starts while the one before it drains: its CTAs stage their unit, which no kernel
+// writes, and wait there.
 __global__ void __launch_bounds__(kBatchBlock) batch_vertex_kernel(const __grid_constant__ BatchParams bp) {
     __shared__ __align__(16) DrawParams s_p;
     __shared__ UnitInfo s_u;
+    stage_unit(bp, blockIdx.x, &s_p, &s_u);
+    pdl_wait();
     pdl_release();
     if (blockIdx.x == 0 && threadIdx.x < kBatchCountersReset / 4)  // first read by the face kernel
         reinterpret_cast<uint32_t*>(bp.counters)[threadIdx.x] = 0u;
-    stage_unit(bp, blockIdx.x, &s_p, &s_u);
     __syncthreads();
     switch (s_p.u.shader) {
         case kFlat: vertex_unit<kFlat>(s_p, s_u); break;
@@ -515,6 +516,7 @@ __global__ void __launch_bounds__(kBatchBlock, AXR_TILE_MIN_BLOCKS)
     stage_unit(bp, bp.vert_units + bp.face_units + blockIdx.x, &sm.p, &sm.u);
     if (threadIdx.x == 0) sm.fill[0] = 0u;
     pdl_wait();
+    pdl_release();
     __syncthreads();
     const DrawParams& p = sm.p;
     const UnitInfo& ui = sm.u;
@@ -619,6 +621,8 @@ __global__ void __launch_bounds__(kBatchBlock, AXR_TILE_MIN_BLOCKS)
 // multiples of 4 pixels). One CTA per SM walks the spans: 16-byte stores from 256 threads
 // per SM reach the HBM write rate.
 __global__ void __launch_bounds__(kBatchBlock) batch_clear_kernel(const __grid_constant__ BatchParams bp) {
+    pdl_wait();
+    pdl_release();
     const uint2* units = reinterpret_cast<const uint2*>(bp.units) + bp.vert_units + bp.face_units + bp.tile_units;
     for (uint32_t u = blockIdx.x; u < bp.clear_units; u += gridDim.x) {
         const uint2 r = __ldg(units + u);
@@ -663,28 +667,20 @@ __global__ void barrier_probe_kernel(DevCounters* c, unsigned long long timeout_
     grid_barrier(c, nullptr, 0, timeout_ns);
 }
 
-template <class K>
-cudaError_t launch_phase(bool first, K kernel, unsigned grid, unsigned block, const BatchParams& bp, cudaStream_t stream) {
-    if (!first) return launch_dependent(kernel, grid, block, stream, bp);
-    kernel<<<grid, block, 0, stream>>>(bp);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_tiles(int shader, const BatchParams& bp, bool first, cudaStream_t stream) {
+cudaError_t launch_tiles(int shader, const BatchParams& bp, cudaStream_t stream) {
     switch (shader) {
-        case kAnyShader: return launch_phase(first, batch_tile_kernel<kAnyShader>, bp.tile_units, kBatchBlock, bp, stream);
-        case kFlat: return launch_phase(first, batch_tile_kernel<kFlat>, bp.tile_units, kBatchBlock, bp, stream);
-        case kPhong: return launch_phase(first, batch_tile_kernel<kPhong>, bp.tile_units, kBatchBlock, bp, stream);
-        case kPBR: return launch_phase(first, batch_tile_kernel<kPBR>, bp.tile_units, kBatchBlock, bp, stream);
-        case kBlinnPhong: return launch_phase(first, batch_tile_kernel<kBlinnPhong>, bp.tile_units, kBatchBlock, bp, stream);
-        case kGouraud: return launch_phase(first, batch_tile_kernel<kGouraud>, bp.tile_units, kBatchBlock, bp, stream);
+        case kAnyShader: return launch_dependent(batch_tile_kernel<kAnyShader>, bp.tile_units, (unsigned)kBatchBlock, stream, bp);
+        case kFlat: return launch_dependent(batch_tile_kernel<kFlat>, bp.tile_units, (unsigned)kBatchBlock, stream, bp);
+        case kPhong: return launch_dependent(batch_tile_kernel<kPhong>, bp.tile_units, (unsigned)kBatchBlock, stream, bp);
+        case kPBR: return launch_dependent(batch_tile_kernel<kPBR>, bp.tile_units, (unsigned)kBatchBlock, stream, bp);
+        case kBlinnPhong: return launch_dependent(batch_tile_kernel<kBlinnPhong>, bp.tile_units, (unsigned)kBatchBlock, stream, bp);
+        case kGouraud: return launch_dependent(batch_tile_kernel<kGouraud>, bp.tile_units, (unsigned)kBatchBlock, stream, bp);
         default: return cudaErrorInvalidValue;
     }
 }
 
-// One launch set of the phased form, all its shader kinds together. The first raster kernel, and
-// the clear, run in full stream order; the others depend on the one before
-// (30 mixed draws 157.4 to 149.4 us, 4 draws one-shot 62 to 59.6; batches of hundreds of draws are unchanged).
+// One launch set of the phased form, all its shader kinds together, each kernel a dependent launch
+// (30 mixed draws 157.4 to 145.8 us, 20 small draws in one call 62 to 51; batches of hundreds of draws are unchanged).
 cudaError_t launch_phased(int shader, const BatchParams& bp, int num_sms, cudaStream_t stream, cudaEvent_t* ev,
                           uint64_t* launches, bool clear_late) {
     cudaError_t e = cudaSuccess;
@@ -698,34 +694,28 @@ cudaError_t launch_phased(int shader, const BatchParams& bp, int num_sms, cudaSt
     auto clear = [&]() -> cudaError_t {
         if (!bp.clear_units) return cudaSuccess;
         const unsigned g = min(bp.clear_units, (unsigned)num_sms);
-        batch_clear_kernel<<<g, kBatchBlock, 0, stream>>>(bp);
         *launches += 1;
-        return cudaGetLastError();
+        return launch_dependent(batch_clear_kernel, g, (unsigned)kBatchBlock, stream, bp);
     };
-    bool first = true;
     if ((e = mark(0)) != cudaSuccess) return e;
     if (!clear_late && (e = clear()) != cudaSuccess) return e;
     if ((e = mark(1)) != cudaSuccess) return e;
-    if (bp.vert_units) {
-        if ((e = launch_phase(first, batch_vertex_kernel, bp.vert_units, kBatchBlock, bp, stream)) != cudaSuccess) return e;
-        first = false;
-    }
+    if (bp.vert_units && (e = launch_dependent(batch_vertex_kernel, bp.vert_units, (unsigned)kBatchBlock, stream, bp)) != cudaSuccess)
+        return e;
     if ((e = mark(2)) != cudaSuccess) return e;
-    if (bp.face_units) {
-        if ((e = launch_phase(first, batch_face_kernel, bp.face_units, kPhasedFaceUnit, bp, stream)) != cudaSuccess) return e;
-        first = false;
-    }
+    if (bp.face_units && (e = launch_dependent(batch_face_kernel, bp.face_units, kPhasedFaceUnit, stream, bp)) != cudaSuccess)
+        return e;
     if ((e = mark(3)) != cudaSuccess) return e;
     // up to 16 CTAs per SM, about three waves of the 5 resident: the items are strided over
     // all warps of the grid, and the later waves even out the first waves' tails (5 per SM
     // measured 3.041 ms per 512-draw step, 8: 3.027, 10: 3.022, 16: 3.018, 32: 3.020); no more
     // CTAs than a small batch has groups of 4 tiles, since CTAs without an item only cost
     const unsigned large_ctas = max((unsigned)num_sms, min((unsigned)num_sms * 16u, bp.tile_units * bp.tile_unit / 4u));
-    if (bp.face_units && (e = launch_phase(first, batch_large_kernel, large_ctas, kBatchBlock, bp, stream)) != cudaSuccess)
+    if (bp.face_units && (e = launch_dependent(batch_large_kernel, large_ctas, (unsigned)kBatchBlock, stream, bp)) != cudaSuccess)
         return e;
     if (clear_late && (e = clear()) != cudaSuccess) return e;
     if ((e = mark(4)) != cudaSuccess) return e;
-    if (bp.tile_units && (e = launch_tiles(shader, bp, first, stream)) != cudaSuccess) return e;
+    if (bp.tile_units && (e = launch_tiles(shader, bp, stream)) != cudaSuccess) return e;
     if ((e = mark(5)) != cudaSuccess) return e;
     *launches += (bp.vert_units ? 1 : 0) + (bp.face_units ? 2 : 0) + (bp.tile_units ? 1 : 0);
     return cudaSuccess;

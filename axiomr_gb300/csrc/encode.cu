@@ -39,6 +39,7 @@
 
 #include "api_internal.h"
 #include "api_types.h"
+#include "pdl.cuh"
 
 using namespace axr_internal;
 
@@ -241,6 +242,7 @@ __device__ __forceinline__ uint32_t match_code(uint32_t len, uint32_t dc, uint32
 template <int C>
 __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __grid_constant__ PngParams p) {
     __shared__ uint32_t s_buf[kPngWarps][kBufWords];
+    pdl_release();
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t row = blockIdx.x * kPngWarps + (uint32_t)warp;
     if (row >= p.rows) return;
@@ -447,6 +449,8 @@ __global__ void __launch_bounds__(kLayoutThreads) png_layout_kernel(const __grid
     __shared__ unsigned long long s_warp[kLayoutThreads / 32];
     __shared__ unsigned long long s_a[kLayoutThreads / 32], s_b[kLayoutThreads / 32];
     __shared__ unsigned long long s_carry;
+    pdl_wait();
+    pdl_release();
     const PngJob& j = p.jobs[blockIdx.x];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     if (tid == 0) s_carry = kHeaderBits;
@@ -553,6 +557,8 @@ __device__ __forceinline__ uint32_t staged_bits(const uint32_t* __restrict__ slo
 // chunks cost more than the gather. 200 MB of files: 0.38 to 0.21 ms.
 __global__ void __launch_bounds__(256, 6) png_pack_kernel(const __grid_constant__ PngParams p) {
     __shared__ uint32_t s_off[kMaxGroupRows + 1];  // each scanline's first bit; the group's end
+    pdl_wait();
+    pdl_release();
     const uint2 g = p.groups[blockIdx.x];
     const PngLayout& L = p.layout[g.x];
     if (L.error) return;
@@ -639,6 +645,8 @@ __global__ void __launch_bounds__(kCrcThreads) png_crc_kernel(const __grid_const
         for (int i = 0; i < 8; ++i) v ^= (tid >> i & 1) ? p.stride[8 * t + i] : 0u;
         s_t[t][tid] = v;
     }
+    pdl_wait();
+    pdl_release();
     // chunks before each image (exclusive prefix) for images [tile, tile + kCrcJobs), and
     // the end of the tile; every block walks the same tiles in order
     __shared__ unsigned long long s_before[kCrcJobs + 1];
@@ -1029,13 +1037,11 @@ axr_status encode_locked(axr_context* ctx, int32_t count, const axr_framebuffer*
     if (channels == 4) png_rows_kernel<4><<<row_blocks, 32 * kPngWarps, 0, ctx->stream>>>(p);
     else png_rows_kernel<3><<<row_blocks, 32 * kPngWarps, 0, ctx->stream>>>(p);
     AXR_CUDA(ctx, cudaGetLastError());
-    png_layout_kernel<<<(unsigned)count, kLayoutThreads, 0, ctx->stream>>>(p);
-    AXR_CUDA(ctx, cudaGetLastError());
-    png_pack_kernel<<<ng, 256, 0, ctx->stream>>>(p);
-    AXR_CUDA(ctx, cudaGetLastError());
+    AXR_CUDA(ctx, launch_dependent(png_layout_kernel, (unsigned)count, (unsigned)kLayoutThreads, ctx->stream, p));
+    AXR_CUDA(ctx, launch_dependent(png_pack_kernel, (unsigned)ng, 256u, ctx->stream, p));
     // a block per chunk, up to 8 per SM (each builds its tables first)
-    png_crc_kernel<<<(unsigned)std::min<uint64_t>(chunks, (uint64_t)ctx->cfg.num_sms * 8u), kCrcThreads, 0, ctx->stream>>>(p);
-    AXR_CUDA(ctx, cudaGetLastError());
+    AXR_CUDA(ctx, launch_dependent(png_crc_kernel, (unsigned)std::min<uint64_t>(chunks, (uint64_t)ctx->cfg.num_sms * 8u),
+                                   (unsigned)kCrcThreads, ctx->stream, p));
     ctx->launches += 4;
     return AXR_OK;
 }

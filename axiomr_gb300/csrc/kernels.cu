@@ -58,6 +58,7 @@ constexpr int kScanTiles = 2;  // tiles per warp and round of the scan kernel
 
 template <int S>
 __global__ void __launch_bounds__(kBlock) vertex_kernel(const __grid_constant__ DrawParams p) {
+    pdl_wait();
     pdl_release();
     const uint32_t i = blockIdx.x * kBlock + threadIdx.x;
     if (i == 0) {
@@ -272,6 +273,8 @@ __global__ void __launch_bounds__(kBlock, tile_blocks(S)) shade_kernel(const __g
 // Colour and/or depth fill, 16-byte stores (the planes are 256-byte aligned allocations).
 __global__ void clear_kernel(uint32_t* color, float* depth, size_t n, uint32_t bgra, float dv, int do_color,
                              int do_depth) {
+    pdl_wait();
+    pdl_release();
     const size_t stride = (size_t)gridDim.x * blockDim.x;
     const size_t n4 = n / 4;
     const uint4 cv = make_uint4(bgra, bgra, bgra, bgra);
@@ -357,8 +360,8 @@ cudaError_t launch_shaded(const DrawParams& p, const LaunchConfig& cfg, cudaStre
             if ((e = mark(k)) != cudaSuccess) return e;
         return cudaSuccess;
     }
-    vertex_kernel<S><<<grid_for(p.mesh.num_vertices, kBlock, 0x7FFFFFFFu), kBlock, 0, stream>>>(p);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    e = launch_dependent(vertex_kernel<S>, grid_for(p.mesh.num_vertices, kBlock, 0x7FFFFFFFu), (unsigned)kBlock, stream, p);
+    if (e != cudaSuccess) return e;
     if ((e = mark(1)) != cudaSuccess) return e;
     const uint32_t share = face_share(p.mesh.num_drawn, cfg.num_sms);
     e = launch_dependent(geometry_kernel, grid_for(p.mesh.num_drawn, (int)share, 0x7FFFFFFFu), kPhasedFaceUnit, stream, p,
@@ -414,9 +417,8 @@ cudaError_t launch_draw(const DrawParams& p, const LaunchConfig& cfg, cudaStream
 
 cudaError_t launch_clear(uint32_t* color, float* depth, size_t pixels, uint32_t bgra, float depth_value,
                          bool do_color, bool do_depth, cudaStream_t stream) {
-    clear_kernel<<<grid_for(pixels, 256, 4096), 256, 0, stream>>>(color, depth, pixels, bgra, depth_value,
-                                                                  do_color ? 1 : 0, do_depth ? 1 : 0);
-    return cudaGetLastError();
+    return launch_dependent(clear_kernel, grid_for(pixels, 256, 4096), 256u, stream, color, depth, pixels, bgra, depth_value,
+                            do_color ? 1 : 0, do_depth ? 1 : 0);
 }
 
 cudaError_t launch_fill_u64(unsigned long long* dst, size_t n, unsigned long long v, cudaStream_t stream) {
@@ -432,7 +434,7 @@ cudaError_t launch_fill_u64(unsigned long long* dst, size_t n, unsigned long lon
 constexpr int kPackBlock = 256;
 
 __global__ void __launch_bounds__(kPackBlock) mesh_pack_kernel(const __grid_constant__ MeshPack p, float* partial) {
-    pdl_release();
+    if (partial) pdl_release();  // without the radius kernel, what follows may read the arrays
     float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
     for (uint32_t i = blockIdx.x * kPackBlock + threadIdx.x; i < p.n; i += gridDim.x * kPackBlock) {
 #pragma unroll
@@ -478,6 +480,7 @@ __global__ void __launch_bounds__(kPackBlock) mesh_radius_kernel(const float4* p
     __shared__ float s_box[6];
     __shared__ double s_r2[kPackBlock / 32];
     pdl_wait();
+    pdl_release();
     if (threadIdx.x < 192) {  // a warp per bound
         const uint32_t d = threadIdx.x >> 5, lane = threadIdx.x & 31;
         float v = d < 3 ? INFINITY : -INFINITY;

@@ -1,9 +1,11 @@
 // Programmatic dependent launch (PTX griddepcontrol): a kernel launched with launch_dependent may
 // be set up, and its CTAs started, while the kernel before it on the stream still drains; it
-// waits at pdl_wait for that kernel's completion (and its writes) before it reads any of them.
-// What it reads from kernels of the same chain it loads with plain loads after pdl_wait: a
-// read-only (ld.global.nc) load could be moved above the wait. The first kernel of a chain is
-// launched in full stream order, so whatever was there before the chain is complete.
+// waits at pdl_wait for that kernel's completion (and its writes) before it touches any of them, and
+// only then lets the next one start (pdl_release). So when a kernel starts, all but the kernel
+// directly before it are complete: data of those may be read at any point, also by read-only loads
+// (ld.global.nc), which could be moved above the wait; data of the kernel directly before it only
+// by plain loads after the wait. Behind anything else than such a kernel (a copy, a kernel that never
+// releases) the launch is an ordinary one, under capture too.
 #pragma once
 #include <cuda_runtime.h>
 
