@@ -50,10 +50,15 @@ constexpr int kScanTiles = 2;  // tiles per warp and round of the scan kernel
 
 
 // Resident 128-thread CTAs per SM the geometry kernel is compiled for (register budget
-// 65536 / (128 * n)): 64 registers.
+// 65536 / (128 * n)): 56 registers, the fewest without spills. Its gathers' latency is the bound (2M-triangle
+// terrain, us a frame: 7 CTAs 92.1, 8 88.4, 9 86.2, 10 98).
 #ifndef AXR_GEOMETRY_MIN_BLOCKS
-#define AXR_GEOMETRY_MIN_BLOCKS 8
+#define AXR_GEOMETRY_MIN_BLOCKS 9
 #endif
+// A CTA brings the face indices of the CTA this many further on into L2, so that of the two dependent
+// loads before a face's setup the first no longer comes from HBM (the terrain 89.8 to 88.4 us; 1216 and
+// 4864 CTAs ahead 88.5 and 89.1).
+constexpr uint32_t kIndexAhead = 304;
 
 
 template <int S>
@@ -74,6 +79,10 @@ __global__ void __launch_bounds__(kBlock) vertex_kernel(const __grid_constant__ 
 __global__ void __launch_bounds__(kPhasedFaceUnit, AXR_GEOMETRY_MIN_BLOCKS)
     geometry_kernel(const __grid_constant__ DrawParams p, uint32_t faces_per_cta) {
     __shared__ __align__(16) FaceSmem<(int)kPhasedFaceUnit> sm;
+    // 32 words, a line, per thread; with several material groups another CTA's faces may be meant
+    const size_t ahead = 3ull * ((size_t)(blockIdx.x + kIndexAhead) * faces_per_cta) + 32u * threadIdx.x;
+    if (32u * threadIdx.x < 3u * faces_per_cta && ahead < 3ull * p.mesh.num_faces)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(p.mesh.idx + ahead));
     pdl_wait();
     pdl_release();
     face_cta<true, true>(p, blockIdx.x * faces_per_cta, faces_per_cta, p.scratch.counters, p.scratch.collect_stats != 0,
