@@ -107,33 +107,57 @@ constexpr uint32_t kCrcJobs = 1024;  // images whose chunk offsets a crc block k
 
 // ------------------------------------------------------------------ device helpers
 
-__device__ __forceinline__ uint32_t find_job(const PngJob* jobs, uint32_t n, uint32_t row) {
-    uint32_t lo = 0, hi = n;  // the last job with row_base <= row
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (__ldg(&jobs[mid].row_base) <= row) lo = mid; else hi = mid;
+// The last job with row_base <= row (the warp's row), 32 jobs compared at a time.
+__device__ __forceinline__ uint32_t find_job(const PngJob* jobs, uint32_t n, uint32_t row, uint32_t lane) {
+    uint32_t lo = 0, span = n;
+    while (span > 1) {
+        const uint32_t step = (span + 31) / 32, i = lane * step;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, i < span && __ldg(&jobs[lo + i].row_base) <= row);
+        const uint32_t k = (31u - (uint32_t)__clz((int)m)) * step;
+        lo += k;
+        span = min(step, span - k);
     }
     return lo;
 }
 
 __device__ __forceinline__ uint32_t reverse_bits(uint32_t code, uint32_t len) { return __brev(code) >> (32 - len); }
 
-// deflate length symbol (257..285), its extra bits and their value, for 3 <= len <= 258
-__device__ __forceinline__ void length_symbol(uint32_t len, uint32_t& sym, uint32_t& ebits, uint32_t& extra) {
-    if (len == 258) {
-        sym = 285; ebits = 0; extra = 0;
-        return;
-    }
-    const uint32_t v = len - 3;
-    if (v < 8) {
-        sym = 257 + v; ebits = 0; extra = 0;
-        return;
-    }
-    const uint32_t e = (31 - __clz(v)) - 2, m = (v >> e) & 3u;
-    sym = 257 + 4 * (e + 1) + m;
-    ebits = e;
-    extra = v - ((4 + m) << e);
+// Fixed Huffman codes, bits reversed for the LSB-first stream, of matches of 1 to 86 (64) pixels of 3 (4)
+// bytes at a distance of one pixel: length symbol (257..285), its extra bits, 5-bit distance code
+// (2 or 3, without extra bits).
+constexpr uint32_t reversed(uint32_t v, uint32_t n) {
+    uint32_t r = 0;
+    for (uint32_t i = 0; i < n; ++i) r |= (v >> i & 1u) << (n - 1 - i);
+    return r;
 }
+constexpr uint2 left_match(uint32_t channels, uint32_t pixels) {
+    const uint32_t len = pixels * channels, v = len - 3;
+    uint32_t sym = 257 + v, extra_bits = 0, extra = 0;
+    if (len == 258) {
+        sym = 285;
+    } else if (v >= 8) {
+        while (v >> (extra_bits + 3)) ++extra_bits;  // the top three bits of v are 1xx
+        sym = 257 + 4 * (extra_bits + 1) + (v >> extra_bits & 3u);
+        extra = v & ((1u << extra_bits) - 1u);
+    }
+    const uint32_t n = sym < 280 ? 7 : 8;
+    const uint32_t code = sym < 280 ? reversed(sym - 256, 7) : reversed(0xC0 + (sym - 280), 8);
+    return uint2{code | extra << n | reversed(channels - 1, 5) << (n + extra_bits), n + extra_bits + 5};
+}
+struct LeftMatches {
+    uint2 of[2][86];  // channels - 3, pixels - 1
+};
+constexpr LeftMatches left_matches() {
+    LeftMatches t{};
+    for (uint32_t c = 0; c < 2; ++c)
+        for (uint32_t k = 0; k < 258 / (c + 3); ++k) t.of[c][k] = left_match(c + 3, k + 1);
+    return t;
+}
+__device__ const LeftMatches g_left = left_matches();
+template <int C>
+constexpr uint32_t kLongestCode = left_match(C, 258u / C).x;
+template <int C>
+constexpr uint32_t kLongestBits = left_match(C, 258u / C).y;
 
 // deflate distance code (0..29), its extra bits and their value, for 1 <= dist <= 32768
 __device__ __forceinline__ void distance_code(uint32_t dist, uint32_t& code, uint32_t& ebits, uint32_t& extra) {
@@ -147,16 +171,6 @@ __device__ __forceinline__ void distance_code(uint32_t dist, uint32_t& code, uin
     ebits = e;
     extra = v - ((2 + m) << e);
 }
-
-// fixed Huffman code of a literal/length symbol: (code bits already reversed, length)
-__device__ __forceinline__ void litlen_code(uint32_t sym, uint32_t& bits, uint32_t& len) {
-    if (sym < 144) { bits = reverse_bits(0x30 + sym, 8); len = 8; }
-    else if (sym < 256) { bits = reverse_bits(0x190 + (sym - 144), 9); len = 9; }
-    else if (sym < 280) { bits = reverse_bits(sym - 256, 7); len = 7; }
-    else { bits = reverse_bits(0xC0 + (sym - 280), 8); len = 8; }
-}
-
-__device__ __forceinline__ uint32_t literal_bits(uint32_t byte) { return byte < 144 ? 8u : 9u; }
 
 // fixed Huffman code of literal byte b, reversed for the LSB-first stream; returns its length
 __device__ __forceinline__ uint32_t literal_code(uint32_t b, uint32_t& code) {
@@ -208,21 +222,6 @@ __device__ __forceinline__ void put_code(uint32_t* buf, uint32_t pos, uint32_t l
     }
 }
 
-// the code of one match of `len` bytes at distance code (dc, deb, dex)
-__device__ __forceinline__ uint32_t match_code(uint32_t len, uint32_t dc, uint32_t deb, uint32_t dex,
-                                               unsigned long long& code) {
-    uint32_t sym, eb, ex, bits, n;
-    length_symbol(len, sym, eb, ex);
-    litlen_code(sym, bits, n);
-    code = bits;
-    code |= (unsigned long long)ex << n;
-    n += eb;
-    code |= (unsigned long long)reverse_bits(dc, 5) << n;
-    n += 5;
-    code |= (unsigned long long)dex << n;
-    return n + deb;
-}
-
 // One warp per scanline, parsed in steps of 32 pixels: lane i takes pixel x = step + i. It is in
 // a left run when it equals pixel x-1, else in an up run when it equals the pixel above; a run
 // starts where its kind starts in the step and ends where it ends or at the step's end. A run
@@ -234,11 +233,12 @@ __device__ __forceinline__ uint32_t match_code(uint32_t len, uint32_t dc, uint32
 // Issue bound on a batch, latency bound on one image (a warp per scanline leaves most of the GPU
 // idle), so four steps are taken together: their loads, ballots and bit-position scans do not
 // wait for one another, the codes go to the staging slot once per block, and the next block's
-// pixels are loaded ahead. A block that goes on with the pixel before it (flat background, 82%
-// of the 512-frame batch's pixels) costs its loads and one vote: its matches are counted and
-// written together when the run ends, its checksum terms come in closed form. Rows pass of the 512
-// frames of a mixed batch (415 Mpixel, RGB) 1.91 to 1.16 ms, of one 1920x1080 RGBA frame 67 to 22
-// us; at 5 or 3 resident CTAs instead of 4 (64 registers) 1.21 and 1.45 ms.
+// pixels are loaded ahead. A block of one colour that goes on with the pixel before it, or starts the
+// scanline (flat background, 78% of the 512-frame batch's blocks), costs its loads and one vote: its
+// run and its checksum terms are taken in closed form when the run of such blocks ends. Match codes
+// are looked up. Rows pass of the 512 frames of a mixed batch (415 Mpixel, RGB) 1.91 ms a step at a
+// time, 1.16 with four steps and the vote, 0.98 with closed forms and tables; one 1920x1080 RGBA frame
+// 67 to 22 us; at 5 or 3 resident CTAs instead of 4 (64 registers) 1.21 and 1.45 ms (of 1.16).
 template <int C>
 __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __grid_constant__ PngParams p) {
     __shared__ uint32_t s_buf[kPngWarps][kBufWords];
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __gri
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t row = blockIdx.x * kPngWarps + (uint32_t)warp;
     if (row >= p.rows) return;
-    const PngJob& j = p.jobs[find_job(p.jobs, p.jobs_n, row)];
+    const PngJob& j = p.jobs[find_job(p.jobs, p.jobs_n, row, (uint32_t)lane)];
     const uint32_t W = j.width, H = j.height, L = j.row_bytes, row_words = j.row_words;
     const uint32_t r = row - j.row_base;
     const uint32_t mask = C == 4 ? 0xFFFFFFFFu : 0x00FFFFFFu;
@@ -256,15 +256,14 @@ __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __gri
     uint32_t* stage = p.stage + j.stage_base + (size_t)r * row_words;
     uint32_t up_code, up_eb, up_ex;
     distance_code(has_up ? L : 1u, up_code, up_eb, up_ex);
-    uint32_t left_code, left_eb, left_ex;
-    distance_code(C, left_code, left_eb, left_ex);
     constexpr uint32_t kMaxRun = 258u / C;  // pixels in the longest match
-    unsigned long long full_code;
-    const uint32_t full_bits = match_code(kMaxRun * C, left_code, left_eb, left_ex, full_code);
+    constexpr uint32_t full_code = kLongestCode<C>, full_bits = kLongestBits<C>;
+    const uint2* matches = g_left.of[C - 3];
     // lane i's codes of matches of i + 1 pixels (at most 31 bits): a step's runs look theirs up
-    unsigned long long tab;
-    const uint32_t left_bits = match_code((uint32_t)(lane + 1) * C, left_code, left_eb, left_ex, tab), left_tab = (uint32_t)tab;
-    const uint32_t up_bits = match_code((uint32_t)(lane + 1) * C, up_code, up_eb, up_ex, tab), up_tab = (uint32_t)tab;
+    const uint2 mine = __ldg(matches + lane);
+    const uint32_t left_tab = mine.x, left_bits = mine.y, len_bits = left_bits - 5u;
+    const uint32_t up_bits = left_bits + up_eb;
+    const uint32_t up_tab = (left_tab & ((1u << len_bits) - 1u)) | reverse_bits(up_code, 5) << len_bits | up_ex << (len_bits + 5u);
 
     uint32_t* buf = s_buf[warp];
     for (int k = lane; k < kBufWords; k += 32) buf[k] = 0u;
@@ -275,6 +274,8 @@ __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __gri
     uint32_t prev = 0;     // the pixel before this block
     uint32_t pending = 0;  // pixels of a left run carried over whole steps, not yet emitted
     uint32_t whole = 0;    // longest matches of that run, not yet written
+    uint32_t flat = 0;     // pixels of the blocks of one colour just parsed, not yet in the sums
+    uint32_t left_run = 0; // and of their left run, not yet in `pending`
     // Adler-32 partial sums: byte i of the scanline (i = 0 is the filter byte, 0) adds
     // (L - i) * byte: (L - i) * (b0 + b1 + b2 [+ b3]) - (b1 + 2 b2 [+ 3 b3]) per pixel
     uint32_t a0 = 0, u0 = 0;            // this lane's bytes; flat blocks (lane-uniform)
@@ -289,10 +290,25 @@ __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __gri
         for (; whole; whole -= min(whole, 32u)) {
             const uint32_t n = min(whole, 32u);
             if ((uint32_t)lane < n) 
-                put_code<false>(buf, nbits - wbase * 32 + (uint32_t)lane * full_bits, (uint32_t)full_code, 0u, full_bits);
+                put_code<false>(buf, nbits - wbase * 32 + (uint32_t)lane * full_bits, full_code, 0u, full_bits);
             __syncwarp();
             flush_words(buf, stage, row_words, wbase, nbits, nbits + n * full_bits, lane);
         }
+    };
+    const uint32_t up0 = has_up ? __ldg(up) & mask : 0u;
+    // the one-colour blocks that end at pixel x; what is left of `left_run` is the scanline's last part of a step
+    auto fold = [&](uint32_t x) {
+        if (!flat) return;
+        uint32_t sum, lag;
+        byte_sums(prev, sum, lag);  // the sum over their pixels of (L - 1 - x C) sum - lag
+        const unsigned long long n = flat, x0 = x - flat;
+        u0 += flat * sum;
+        u1 += n * ((unsigned long long)(L - 1) * sum - lag) - (unsigned long long)(C * sum) * (n * x0 + n * (n - 1) / 2);
+        flat = 0;
+        pending += left_run & ~(kStep - 1);
+        whole += pending / kMaxRun;
+        pending %= kMaxRun;
+        left_run &= kStep - 1;
     };
     uint32_t raw[kSteps];
 #pragma unroll
@@ -305,22 +321,48 @@ __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __gri
             const uint32_t x = c0 + kBlockPixels + kStep * k + (uint32_t)lane;
             next[k] = x < W ? __ldg(src + x) : 0u;
         }
-        bool same = c0 > 0 && c0 + kBlockPixels <= W;
+        const uint32_t ref = c0 > 0 ? prev : __shfl_sync(0xFFFFFFFFu, raw[0], 0) & mask;
+        bool same = true;
 #pragma unroll
-        for (uint32_t k = 0; k < kSteps; ++k) same = same && (raw[k] & mask) == prev;
-        if (__all_sync(0xFFFFFFFFu, same)) {  // the whole block continues a left run
-            pending += kBlockPixels;
-            whole += pending / kMaxRun;
-            pending %= kMaxRun;
-            uint32_t sum, lag;
-            byte_sums(prev, sum, lag);  // sum over x = c0 .. c0 + 127 of (L - 1 - x C) sum - lag
-            u0 += kBlockPixels * sum;
-            u1 += (unsigned long long)kBlockPixels * ((unsigned long long)(L - 1) * sum - lag) -
-                  (unsigned long long)(C * sum) * (kBlockPixels * c0 + kBlockPixels * (kBlockPixels - 1) / 2);
+        for (uint32_t k = 0; k < kSteps; ++k)
+            same = same && ((raw[k] & mask) == ref || c0 + kStep * k + (uint32_t)lane >= W);
+        if (__all_sync(0xFFFFFFFFu, same)) {  // one colour, a left run but for the scanline's first pixel
+            const uint32_t n = min(W - c0, kBlockPixels);
+            flat += n;
+            left_run += n;
+            if (c0 == 0) {  // the first step: lane 0 the first pixel's code, lane 1 the run after it
+                const uint32_t first = min(W, kStep);
+                const uint32_t lit[4] = {(ref >> 16) & 255u, (ref >> 8) & 255u, ref & 255u, ref >> 24};
+                unsigned long long code = 0;
+                uint32_t bits = 0;
+#pragma unroll
+                for (int q = 0; q < C; ++q) {
+                    uint32_t c;
+                    const uint32_t l = literal_code(lit[q], c);
+                    code |= (unsigned long long)c << bits;
+                    bits += l;
+                }
+                if (has_up && up0 == ref && 12u + up_eb < bits) {
+                    code = __shfl_sync(0xFFFFFFFFu, up_tab, 0);
+                    bits = __shfl_sync(0xFFFFFFFFu, up_bits, 0);
+                }
+                const int at = first > 1 ? (int)first - 2 : 0;
+                const uint32_t cl = __shfl_sync(0xFFFFFFFFu, left_tab, at);
+                const uint32_t nl = first > 1 ? __shfl_sync(0xFFFFFFFFu, left_bits, at) : 0u;
+                const uint32_t pos = nbits - wbase * 32;
+                if (lane < 2)
+                    put_code<C == 4>(buf, lane == 0 ? pos : pos + bits, lane == 0 ? (uint32_t)code : cl,
+                                     lane == 0 ? (uint32_t)(code >> 32) : 0u, lane == 0 ? bits : nl);
+                __syncwarp();
+                flush_words(buf, stage, row_words, wbase, nbits, nbits + bits + nl, lane);
+                left_run -= first;
+            }
+            prev = ref;
 #pragma unroll
             for (uint32_t k = 0; k < kSteps; ++k) raw[k] = next[k];
             continue;
         }
+        fold(c0);
         write_whole();
         uint32_t u[kSteps], v[kSteps], m_l[kSteps];
 #pragma unroll
@@ -328,24 +370,24 @@ __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __gri
             const uint32_t x = c0 + kStep * k + (uint32_t)lane;
             u[k] = (has_up && x < W) ? (__ldg(up + x) & mask) : 0u;
         }
+        uint32_t terms = 0;  // of a1: four at most, each below 131072 * 4 * 1020
 #pragma unroll
         for (uint32_t k = 0; k < kSteps; ++k) {
             const uint32_t x = c0 + kStep * k + (uint32_t)lane;
             v[k] = raw[k] & mask;
-            if (x < W) {
-                uint32_t sum, lag;
-                byte_sums(raw[k], sum, lag);
-                a0 += sum;
-                a1 += (unsigned long long)(L - 1 - x * C) * sum - lag;
-            }
+            uint32_t sum, lag;  // (0 past the scanline's end)
+            byte_sums(raw[k], sum, lag);
+            a0 += sum;
+            terms += (L - 1 - x * C) * sum - lag;
             uint32_t left = __shfl_up_sync(0xFFFFFFFFu, v[k], 1);
             if (lane == 0) left = prev;
             prev = __shfl_sync(0xFFFFFFFFu, v[k], 31);
             m_l[k] = __ballot_sync(0xFFFFFFFFu, x < W && x > 0 && v[k] == left);
         }
+        a1 += terms;
         // each step's match before its own codes (the run carried to it, in pixels; lane k keeps
         // step k's) and each lane's code per step
-        uint32_t ahead = 0, n[kSteps], incl[kSteps], lo[kSteps], hi[kSteps];  // hi: RGBA literals' bits past 32
+        uint32_t ahead = 0, n[kSteps], lo[kSteps], hi[kSteps];  // hi: RGBA literals' bits past 32
 #pragma unroll
         for (uint32_t k = 0; k < kSteps; ++k) {
             const uint32_t x = c0 + kStep * k + (uint32_t)lane;
@@ -392,48 +434,56 @@ __global__ void __launch_bounds__(32 * kPngWarps, 4) png_rows_kernel(const __gri
                 }
             }
             if ((uint32_t)lane == k) ahead = before;
-            incl[k] = n[k];
         }
-        unsigned long long ahead_code = 0;
-        uint32_t ahead_bits = 0;
-        if (ahead) ahead_bits = match_code(ahead * C, left_code, left_eb, left_ex, ahead_code);
-        // bit positions of the lanes' codes in each step
+        const uint2 ahead_code = ahead ? __ldg(matches + ahead - 1) : make_uint2(0u, 0u);
+        // bit positions of the lanes' codes, two steps' sums (below 2^11) in a word
+        static_assert(kSteps == 4, "two words");
+        uint32_t in01 = n[0] | n[1] << 16, in23 = n[2] | n[3] << 16;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-#pragma unroll
-            for (uint32_t k = 0; k < kSteps; ++k) {
-                const uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl[k], o);
-                if (lane >= o) incl[k] += t;
+            const uint32_t t01 = __shfl_up_sync(0xFFFFFFFFu, in01, o), t23 = __shfl_up_sync(0xFFFFFFFFu, in23, o);
+            if (lane >= o) {
+                in01 += t01;
+                in23 += t23;
             }
         }
+        const uint32_t all01 = __shfl_sync(0xFFFFFFFFu, in01, 31), all23 = __shfl_sync(0xFFFFFFFFu, in23, 31);
+        const uint32_t incl[kSteps] = {in01 & 0xFFFFu, in01 >> 16, in23 & 0xFFFFu, in23 >> 16};
+        const uint32_t all[kSteps] = {all01 & 0xFFFFu, all01 >> 16, all23 & 0xFFFFu, all23 >> 16};
         uint32_t pos = nbits - wbase * 32, ahead_pos = 0;
 #pragma unroll
         for (uint32_t k = 0; k < kSteps; ++k) {
             if ((uint32_t)lane == k) ahead_pos = pos;
-            pos += __shfl_sync(0xFFFFFFFFu, ahead_bits, (int)k);
+            pos += __shfl_sync(0xFFFFFFFFu, ahead_code.y, (int)k);
             put_code<C == 4>(buf, pos + incl[k] - n[k], lo[k], hi[k], n[k]);
-            pos += __shfl_sync(0xFFFFFFFFu, incl[k], 31);
+            pos += all[k];
         }
-        put_code<false>(buf, ahead_pos, (uint32_t)ahead_code, 0u, ahead_bits);
+        put_code<false>(buf, ahead_pos, ahead_code.x, 0u, ahead_code.y);
         __syncwarp();
         flush_words(buf, stage, row_words, wbase, nbits, wbase * 32 + pos, lane);
 #pragma unroll
         for (uint32_t k = 0; k < kSteps; ++k) raw[k] = next[k];
     }
+    fold(W);
     write_whole();
-    if (pending) {
-        unsigned long long c;
-        const uint32_t n = match_code(pending * C, left_code, left_eb, left_ex, c);
-        if (lane == 0) put_code<false>(buf, nbits - wbase * 32, (uint32_t)c, 0u, n);
+    if (pending | left_run) {  // lane 0: what the run carried over; lane 1: its part of the last step
+        const uint32_t px = lane == 0 ? pending : lane == 1 ? left_run : 0u;
+        const uint2 c = px ? __ldg(matches + px - 1) : make_uint2(0u, 0u);
+        const uint32_t nb = __shfl_sync(0xFFFFFFFFu, c.y, 0), nl = __shfl_sync(0xFFFFFFFFu, c.y, 1);
+        put_code<false>(buf, nbits - wbase * 32 + (lane == 0 ? 0u : nb), c.x, 0u, c.y);
         __syncwarp();
-        flush_words(buf, stage, row_words, wbase, nbits, nbits + n, lane);
+        flush_words(buf, stage, row_words, wbase, nbits, nbits + nb + nl, lane);
     }
     if (lane == 0 && (nbits & 31u) && wbase < row_words) stage[wbase] = buf[0];
-    const unsigned long long s0 = warp_sum64(a0) + u0;
-    a1 = warp_sum64(a1) + u1;
+    uint32_t s0 = u0;
+    if (__any_sync(0xFFFFFFFFu, a0 != 0u)) {  // (a lane without bytes has no a1 either)
+        s0 += __reduce_add_sync(0xFFFFFFFFu, a0);
+        a1 = warp_sum64(a1);
+    }
+    a1 += u1;
     if (lane == 0) {
         p.row_bits[row] = nbits;
-        p.s0[row] = (uint32_t)s0;
+        p.s0[row] = s0;
         p.s1[row] = a1;
     }
 }
