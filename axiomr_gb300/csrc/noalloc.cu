@@ -13,7 +13,7 @@
 //
 // Limits: at most kNoAllocMaxVertices vertices, kNoAllocMaxFaces drawn faces and
 // kNoAllocMaxPixels framebuffer pixels per call; larger draws are rejected with
-// AXR_E_CAPACITY. The array (about 32 MiB) is reserved on every GPU that loads the library
+// AXR_E_CAPACITY. The array (about 28 MiB) is reserved on every GPU that loads the library
 // and stays reserved until the process exits.
 //
 // Set-up: the first call on each device looks up the array's device address with

@@ -337,7 +337,7 @@ axr_status axr_get_bin_params(const axr_context* ctx, axr_bin_params* out);
 /* No counterpart in the reference. The same draw as axr_draw_mesh for callers that cannot
  * allocate device memory: a renderer recording its frame into a CUDA graph, a real-time
  * loop that forbids allocator calls after start-up, or a host that owns the device-memory
- * budget. Its scratch lives in one fixed device array inside the library (about 32 MiB,
+ * budget. Its scratch lives in one fixed device array inside the library (about 28 MiB,
  * reserved on every GPU that loads the library until exit), so the call allocates nothing.
  * Limits: 65536 vertices, 65536 drawn faces, 1024*1024 framebuffer pixels; larger draws
  * return AXR_E_CAPACITY. The first call on a device looks up the array's address, so make
