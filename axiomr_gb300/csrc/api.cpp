@@ -215,14 +215,50 @@ axr_status check_mesh_desc(axr_context* ctx, const axr_mesh_desc* d) {
     return AXR_OK;
 }
 
-// The arrays of a mesh on their way to the device: the float3 ones into the staging area and, as
-// many at a time as it holds, widened to float4 by one kernel, which with `bounds` also starts the
-// positions' bounds.
+// The device's address of 16-byte aligned pinned host memory; NULL for anything else.
+template <class T>
+const T* pinned(const T* p) {
+    cudaPointerAttributes a{};
+    if ((reinterpret_cast<uintptr_t>(p) & 15u) || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    return a.type == cudaMemoryTypeHost ? static_cast<const T*>(a.devicePointer) : nullptr;
+}
+
+// The arrays of a mesh on their way to the device. When all of them are pinned and
+// aligned, one kernel reads them from there (faster at every size, see mesh_import_kernel); otherwise
+// the float3 ones are copied into the staging area and, as many at a time as it holds, widened to
+// float4 by one kernel. With `bounds` either kernel also starts the positions' bounds.
 axr_status upload_mesh_arrays(axr_context* ctx, axr_mesh* m, const axr_mesh_desc* d, axr::MeshBounds* bounds) {
     const size_t V = m->num_vertices;
+    const float* src[4] = {d->positions, d->normals, d->tangents, d->bitangents};
+    float4* dst[4] = {m->pos, m->nrm, m->tan, m->bit};
+    if (V && m->num_faces) {
+        MeshImport in{};
+        in.pack.n = m->num_vertices;
+        bool all = true;
+        for (int k = 0; k < 4 && all; ++k) {
+            if (!src[k] || !dst[k]) continue;
+            in.pack.src[in.pack.arrays] = pinned(src[k]);
+            all = in.pack.src[in.pack.arrays] != nullptr;
+            in.pack.dst[in.pack.arrays++] = dst[k];
+        }
+        if (all) {
+            in.copy_src[0] = reinterpret_cast<const uint4*>(pinned(d->uvs));
+            in.copy_src[1] = reinterpret_cast<const uint4*>(pinned(d->indices));
+            in.copy_dst[0] = reinterpret_cast<uint4*>(m->uv);
+            in.copy_dst[1] = reinterpret_cast<uint4*>(m->idx);
+            in.copy_bytes[0] = 8ull * V;
+            in.copy_bytes[1] = 12ull * m->num_faces;
+            if (in.copy_src[0] && in.copy_src[1]) {
+                AXR_CUDA(ctx, launch_mesh_import(in, bounds ? m->staging + 3 * V * m->staging_slots : nullptr, bounds,
+                                                 ctx->stream, &ctx->launches));
+                return AXR_OK;
+            }
+        }
+    }
     if (V) {
-        const float* src[4] = {d->positions, d->normals, d->tangents, d->bitangents};
-        float4* dst[4] = {m->pos, m->nrm, m->tan, m->bit};
         MeshPack pack{};
         pack.n = m->num_vertices;
         for (int k = 0; k < 4; ++k) {

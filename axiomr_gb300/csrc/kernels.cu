@@ -442,26 +442,8 @@ cudaError_t launch_fill_u64(unsigned long long* dst, size_t n, unsigned long lon
 // mesh updated and drawn: 160 to 112 us).
 constexpr int kPackBlock = 256;
 
-__global__ void __launch_bounds__(kPackBlock) mesh_pack_kernel(const __grid_constant__ MeshPack p, float* partial) {
-    if (partial) pdl_release();  // without the radius kernel, what follows may read the arrays
-    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
-    for (uint32_t i = blockIdx.x * kPackBlock + threadIdx.x; i < p.n; i += gridDim.x * kPackBlock) {
-#pragma unroll
-        for (uint32_t k = 0; k < 4; ++k) {
-            if (k >= p.arrays) break;
-            const float* s = p.src[k] + 3ull * i;
-            const float v[3] = {s[0], s[1], s[2]};
-            p.dst[k][i] = make_float4(v[0], v[1], v[2], 0.0f);
-            if (k == 0) {
-#pragma unroll
-                for (int d = 0; d < 3; ++d) {
-                    lo[d] = fminf(lo[d], v[d]);
-                    hi[d] = fmaxf(hi[d], v[d]);
-                }
-            }
-        }
-    }
-    if (!partial) return;
+// The block's box of its threads' boxes.
+__device__ __forceinline__ void block_box(float lo[3], float hi[3], float* partial) {
     __shared__ float s_box[kPackBlock / 32][6];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -481,6 +463,90 @@ __global__ void __launch_bounds__(kPackBlock) mesh_pack_kernel(const __grid_cons
             v = threadIdx.x < 3 ? fminf(v, s_box[w][threadIdx.x]) : fmaxf(v, s_box[w][threadIdx.x]);
         partial[6 * blockIdx.x + threadIdx.x] = v;
     }
+}
+
+__global__ void __launch_bounds__(kPackBlock) mesh_pack_kernel(const __grid_constant__ MeshPack p, float* partial) {
+    if (partial) pdl_release();  // without the radius kernel, what follows may read the arrays
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (uint32_t i = blockIdx.x * kPackBlock + threadIdx.x; i < p.n; i += gridDim.x * kPackBlock) {
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (k >= p.arrays) break;
+            const float* s = p.src[k] + 3ull * i;
+            const float v[3] = {s[0], s[1], s[2]};
+            p.dst[k][i] = make_float4(v[0], v[1], v[2], 0.0f);
+            if (k == 0) {
+#pragma unroll
+                for (int d = 0; d < 3; ++d) {
+                    lo[d] = fminf(lo[d], v[d]);
+                    hi[d] = fmaxf(hi[d], v[d]);
+                }
+            }
+        }
+    }
+    if (partial) block_box(lo, hi, partial);
+}
+
+// The same from pinned host memory, with the other arrays: the first vertex_blocks CTAs take 256 vertices
+// at a time through shared memory (16-byte loads, all arrays' in flight together), the others copy
+// the flat arrays. Bound by the link. Copies into a staging area, one after another and each with its
+// start, and a kernel behind them took longer at every size (update and frame, us, copies / this kernel:
+// 256 vertices 59 / 40, 4k 68 / 58, 65k 108 / 83, 262k 200 / 181, 1M 590 / 572).
+__global__ void __launch_bounds__(kPackBlock) mesh_import_kernel(const __grid_constant__ MeshImport p, uint32_t vertex_blocks,
+                                                                 float* partial) {
+    if (partial) pdl_release();
+    const int tid = threadIdx.x;
+    if (blockIdx.x >= vertex_blocks) {
+        const size_t first = (size_t)(blockIdx.x - vertex_blocks) * kPackBlock + tid;
+        const size_t stride = (size_t)(gridDim.x - vertex_blocks) * kPackBlock;
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+            const size_t n = p.copy_bytes[a] / 16;
+#pragma unroll 4
+            for (size_t i = first; i < n; i += stride) p.copy_dst[a][i] = p.copy_src[a][i];
+            const uint32_t* s = reinterpret_cast<const uint32_t*>(p.copy_src[a]);
+            uint32_t* d = reinterpret_cast<uint32_t*>(p.copy_dst[a]);
+            const size_t w = n * 4 + first;
+            if (w < p.copy_bytes[a] / 4) d[w] = s[w];  // at most three words
+        }
+        return;
+    }
+    __shared__ __align__(16) float s_in[4][3 * kPackBlock];
+    float lo[3] = {INFINITY, INFINITY, INFINITY}, hi[3] = {-INFINITY, -INFINITY, -INFINITY};
+    for (uint32_t v0 = blockIdx.x * kPackBlock; v0 < p.pack.n; v0 += vertex_blocks * kPackBlock) {
+        const uint32_t floats = 3u * min((uint32_t)kPackBlock, p.pack.n - v0);
+        const uint32_t whole = floats / 4;
+        float4 r[4];
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k)
+            if (k < p.pack.arrays && (uint32_t)tid < whole)
+                r[k] = reinterpret_cast<const float4*>(p.pack.src[k] + 3ull * v0)[tid];
+        __syncthreads();  // the previous vertices have been read
+#pragma unroll
+        for (uint32_t k = 0; k < 4; ++k) {
+            if (k >= p.pack.arrays) break;
+            if ((uint32_t)tid < whole) reinterpret_cast<float4*>(s_in[k])[tid] = r[k];
+            const uint32_t w = 4 * whole + (uint32_t)tid;
+            if (w < floats) s_in[k][w] = p.pack.src[k][3ull * v0 + w];
+        }
+        __syncthreads();
+        if (3u * (uint32_t)tid < floats) {
+#pragma unroll
+            for (uint32_t k = 0; k < 4; ++k) {
+                if (k >= p.pack.arrays) break;
+                const float v[3] = {s_in[k][3 * tid], s_in[k][3 * tid + 1], s_in[k][3 * tid + 2]};
+                p.pack.dst[k][v0 + tid] = make_float4(v[0], v[1], v[2], 0.0f);
+                if (k == 0) {
+#pragma unroll
+                    for (int d = 0; d < 3; ++d) {
+                        lo[d] = fminf(lo[d], v[d]);
+                        hi[d] = fmaxf(hi[d], v[d]);
+                    }
+                }
+            }
+        }
+    }
+    if (partial) block_box(lo, hi, partial);
 }
 
 // The box of all blocks, then each block's largest squared distance from its centre.
@@ -542,6 +608,21 @@ cudaError_t launch_mesh_pack(const MeshPack& p, float* partial, MeshBounds* boun
     if (!partial) return cudaSuccess;
     *launches += 1;
     return launch_dependent(mesh_radius_kernel, g, (unsigned)kPackBlock, stream, (const float4*)p.dst[0], p.n,
+                            (const float*)partial, bounds);
+}
+
+cudaError_t launch_mesh_import(const MeshImport& p, float* partial, MeshBounds* bounds, cudaStream_t stream, uint64_t* launches) {
+    const unsigned vb = p.pack.n ? grid_for(p.pack.n, kPackBlock, kBoundsBlocks) : 0u;
+    const size_t bytes = p.copy_bytes[0] + p.copy_bytes[1];
+    const unsigned cb = bytes ? grid_for(bytes / 16, kPackBlock * 4, kBoundsBlocks) : 0u;
+    if (vb + cb == 0) return cudaSuccess;
+    mesh_import_kernel<<<vb + cb, kPackBlock, 0, stream>>>(p, vb, vb ? partial : nullptr);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return e;
+    *launches += 1;
+    if (!partial || !vb) return cudaSuccess;
+    *launches += 1;
+    return launch_dependent(mesh_radius_kernel, vb, (unsigned)kPackBlock, stream, (const float4*)p.pack.dst[0], p.pack.n,
                             (const float*)partial, bounds);
 }
 

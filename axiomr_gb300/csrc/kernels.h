@@ -49,6 +49,16 @@ struct MeshPack {
 };
 cudaError_t launch_mesh_pack(const MeshPack& p, float* partial, MeshBounds* bounds, cudaStream_t stream, uint64_t* launches);
 
+// A mesh's arrays read by the GPU straight from pinned host memory (all 16-byte aligned): float3
+// arrays widened as above, texture coordinates and indices copied.
+struct MeshImport {
+    MeshPack pack;
+    const uint4* copy_src[2];  // uvs, indices
+    uint4* copy_dst[2];
+    size_t copy_bytes[2];      // multiples of 4
+};
+cudaError_t launch_mesh_import(const MeshImport& p, float* partial, MeshBounds* bounds, cudaStream_t stream, uint64_t* launches);
+
 // Stage dump for parity tests: every triangle that survives clip + cull, unordered, as
 // (tag, screen x0 y0 x1 y1 x2 y2, ndcZ0..2, minX, minY, maxX, maxY) = 14 words.
 cudaError_t launch_debug_triangles(const DrawParams& p, float* out, uint32_t* count, uint32_t capacity,
