@@ -261,9 +261,9 @@ axr_status axr_framebuffers_read_png(axr_context* ctx, int32_t count, const axr_
 /* The same read-back in steps, for pipelines: a batch keeps its files on the device and has
  * its own copy streams. axr_png_batch_encode enqueues the encode of `count` framebuffers on
  * the context stream (after the work already there, and after this batch's previous files
- * were read) and returns at once; axr_png_batch_sizes waits for that encode and returns the
- * file sizes; axr_png_batch_read copies the files to host buffers (capacity[i] bytes each)
- * and returns when they are there. Render and encode batch k+1 while reading batch k. */
+ * were read) and returns at once; axr_png_batch_sizes waits until that encode has read the
+ * framebuffers and returns the file sizes; axr_png_batch_read copies the files to host
+ * buffers (capacity[i] bytes each) and returns when they are there. Render and encode batch k+1 while reading batch k. */
 typedef struct axr_png_batch axr_png_batch;
 axr_status axr_png_batch_create(axr_context* ctx, axr_png_batch** out);
 void axr_png_batch_destroy(axr_context* ctx, axr_png_batch* batch);
