@@ -928,7 +928,7 @@ def run_batch(args, dist: Dist):
         "triangles_per_step": int(st["triangles"]), "faces_per_step": int(faces),
         "pixels_per_step": int(info["pixels"]),
         "plain": {"value": round(plain_value, 2), "unit": "frames/s", "ms_per_step": round(sum(plain_ms) / len(plain_ms), 4),
-                  "form": "per draw: clearColor, clearDepth, drawMesh (9 launches), replayed from a CUDA graph",
+                  "form": "per draw: clearColor, clearDepth, drawMesh, replayed from a CUDA graph",
                   "launches_per_draw": int(plain_launches_per_draw)},
         "plain_eager": {"value": round(eager_value, 2), "unit": "frames/s",
                         "form": "the same per-draw calls issued from the Python host loop"},
