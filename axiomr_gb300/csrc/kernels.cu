@@ -46,7 +46,7 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr int kClipBlock = 64;
-constexpr int kScanTiles = 2;  // tiles per warp and round of the scan kernel
+constexpr int kScanTiles = 1;  // tiles per warp and round of the scan kernel
 
 
 // Resident 128-thread CTAs per SM the geometry kernel is compiled for (register budget
@@ -195,8 +195,10 @@ __global__ void __launch_bounds__(kBlock, tile_blocks(S)) tile_kernel(const __gr
 // once; the covered pixels are appended to the shade list, their keys and the tiles' flags
 // reset. List space is taken once per CTA round (a prefix over the warps), so the global counter
 // sees few atomics; the warps' counts are double-buffered, so that a round has two barriers.
-// Bound by the keys' reads.
-__global__ void __launch_bounds__(kBlock, 3) scan_kernel(const __grid_constant__ DrawParams p) {
+// Bound by the keys' reads: many warps with a tile each hide them better than few with two (2M-triangle
+// terrain / 200k small triangles at 3840x2160, us a frame: one tile, 6 CTAs per SM 85.4 / 95.9; two, 3 CTAs
+// 86.2 / 97.5; two, 4 CTAs 86.5 / 95.0; one, 7 CTAs (spills) 89.4 / 103; four, 2 CTAs 87.5 / 102).
+__global__ void __launch_bounds__(kBlock, 6) scan_kernel(const __grid_constant__ DrawParams p) {
     constexpr int kWarps = kBlock / 32;
     __shared__ uint32_t s_count[2][kWarps], s_base[2];
     DevCounters* c = p.scratch.counters;
