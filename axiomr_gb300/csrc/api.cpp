@@ -4,6 +4,7 @@
 #include "axr.h"
 
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 
 #include <algorithm>
 #include <cmath>
@@ -17,6 +18,7 @@
 #include "device_types.h"
 #include "hostmath.h"
 #include "kernels.h"
+#include "pinned.h"
 
 using namespace axr;
 
@@ -215,18 +217,39 @@ axr_status check_mesh_desc(axr_context* ctx, const axr_mesh_desc* d) {
     return AXR_OK;
 }
 
-// The device's address of 16-byte aligned pinned host memory; NULL for anything else.
+// The device's address of an array that the GPU may read in place (readable_in_place); NULL for anything
+// else. The range comes from the driver, which knows each allocation's and registration's extent.
 template <class T>
-const T* pinned(const T* p) {
+const T* pinned(const T* p, size_t bytes) {
+    static std::once_flag once;
+    static PFN_cuPointerGetAttribute_v4000 get = nullptr;
+    std::call_once(once, [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q{};
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttribute", &f, 4000, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            get = reinterpret_cast<PFN_cuPointerGetAttribute_v4000>(f);
+        else
+            cudaGetLastError();
+    });
     cudaPointerAttributes a{};
-    if ((reinterpret_cast<uintptr_t>(p) & 15u) || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    if (!get || cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         cudaGetLastError();
         return nullptr;
     }
-    return a.type == cudaMemoryTypeHost ? static_cast<const T*>(a.devicePointer) : nullptr;
+    if (a.type != cudaMemoryTypeHost || !a.devicePointer) return nullptr;
+    PinnedRange r{reinterpret_cast<uint64_t>(a.devicePointer), 0, 0};
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    if (get(&start, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, r.device) == CUDA_SUCCESS &&
+        get(&size, CU_POINTER_ATTRIBUTE_RANGE_SIZE, r.device) == CUDA_SUCCESS) {
+        r.start = start;
+        r.size = size;
+    }
+    return reinterpret_cast<const T*>(readable_in_place(reinterpret_cast<uintptr_t>(p), bytes, r));
 }
 
-// The arrays of a mesh on their way to the device. When all of them are pinned and
+// The arrays of a mesh on their way to the device. When all of them are wholly pinned and
 // aligned, one kernel reads them from there (faster at every size, see mesh_import_kernel); otherwise
 // the float3 ones are copied into the staging area and, as many at a time as it holds, widened to
 // float4 by one kernel. With `bounds` either kernel also starts the positions' bounds.
@@ -240,17 +263,17 @@ axr_status upload_mesh_arrays(axr_context* ctx, axr_mesh* m, const axr_mesh_desc
         bool all = true;
         for (int k = 0; k < 4 && all; ++k) {
             if (!src[k] || !dst[k]) continue;
-            in.pack.src[in.pack.arrays] = pinned(src[k]);
+            in.pack.src[in.pack.arrays] = pinned(src[k], 12 * V);
             all = in.pack.src[in.pack.arrays] != nullptr;
             in.pack.dst[in.pack.arrays++] = dst[k];
         }
         if (all) {
-            in.copy_src[0] = reinterpret_cast<const uint4*>(pinned(d->uvs));
-            in.copy_src[1] = reinterpret_cast<const uint4*>(pinned(d->indices));
-            in.copy_dst[0] = reinterpret_cast<uint4*>(m->uv);
-            in.copy_dst[1] = reinterpret_cast<uint4*>(m->idx);
             in.copy_bytes[0] = 8ull * V;
             in.copy_bytes[1] = 12ull * m->num_faces;
+            in.copy_src[0] = reinterpret_cast<const uint4*>(pinned(d->uvs, in.copy_bytes[0]));
+            in.copy_src[1] = reinterpret_cast<const uint4*>(pinned(d->indices, in.copy_bytes[1]));
+            in.copy_dst[0] = reinterpret_cast<uint4*>(m->uv);
+            in.copy_dst[1] = reinterpret_cast<uint4*>(m->idx);
             if (in.copy_src[0] && in.copy_src[1]) {
                 AXR_CUDA(ctx, launch_mesh_import(in, bounds ? m->staging + 3 * V * m->staging_slots : nullptr, bounds,
                                                  ctx->stream, &ctx->launches));
