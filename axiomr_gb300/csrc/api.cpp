@@ -89,6 +89,16 @@ bool mesh_clip_free(const axr_mesh* m, const float mvp[16]) {
     return true;
 }
 
+bool recording(const axr_context* ctx) {
+    if (ctx->capturing) return true;
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(ctx->stream, &status) != cudaSuccess) {
+        cudaGetLastError();
+        return true;  // a capture that the stream takes part in without leave
+    }
+    return status != cudaStreamCaptureStatusNone;
+}
+
 void take_bounds(const axr_mesh* m, const MeshBounds& b) {
     double r2 = 0.0;
     for (uint32_t k = 0; k < b.blocks; ++k) r2 = std::max(r2, b.r2[k]);
@@ -1063,7 +1073,9 @@ axr_status axr_draw_mesh(axr_context* ctx, const axr_mesh* mesh, const float mod
     }
     if (ctx->draw_form != AXR_DRAW_BINNED) {
         LaunchConfig cfg = ctx->cfg;
-        cfg.clip_free = mesh_clip_free(mesh, u.mvp);
+        // a recorded draw meets whatever vertices the device holds at each replay, not the ones whose
+        // bounds are known now: it always has its clip pass
+        cfg.clip_free = !recording(ctx) && mesh_clip_free(mesh, u.mvp);
         AXR_CUDA(ctx, launch_draw(p, cfg, ctx->stream, ev, &ctx->launches));
         return AXR_OK;
     }

@@ -41,6 +41,9 @@ void encode_framebuffer_maps(axr_framebuffer* fb);
 void mesh_bounds(const float* pos, uint32_t n, float center[3], float* radius);
 // Waits for and takes the device-computed bounds of the last axr_mesh_update, if any.
 void mesh_sync_bounds(const axr_mesh* m);
+// Whether work enqueued on the context's stream goes into a graph (axr_graph_begin, or a capture of a
+// stream that the caller set).
+bool recording(const axr_context* ctx);
 // The bounding sphere of m's positions from the device's bounds.
 void take_bounds(const axr_mesh* m, const axr::MeshBounds& b);
 // Release a batch's device memory (the caller synchronises first).
