@@ -59,9 +59,9 @@ void dfree(void* p) {
 // (x+w, w-x, y+w, w-y, z+w, w-z >= 0 of clip = mvp * (p, 1)) for the column-major mvp: the
 // smallest value of each plane's function over the mesh's bounding sphere, in double, must
 // exceed a margin far above the rounding of the device's float evaluation. Unknown bounds
-// (an update still in flight) or non-finite values answer false.
+// (an update still in flight or recorded into a graph) or non-finite values answer false.
 bool mesh_clip_free(const axr_mesh* m, const float mvp[16]) {
-    if (!m || m->num_vertices == 0) return false;
+    if (!m || m->num_vertices == 0 || m->recorded_update) return false;
     if (m->bounds_pending) {
         if (cudaEventQuery(m->bounds_ready) != cudaSuccess) {
             cudaGetLastError();  // cudaErrorNotReady is no error here
@@ -693,11 +693,17 @@ axr_status axr_mesh_update(axr_context* ctx, axr_mesh* m, const axr_mesh_desc* d
     // for a large one on the device behind the upload (a host pass over a million vertices
     // takes milliseconds), which batch planning waits for if it must
     if (m->num_vertices <= kHostBoundsMaxVertices) {
+        if (recording(ctx)) m->recorded_update = true;
         axr_status st = upload_mesh_arrays(ctx, m, d, nullptr);
         if (st != AXR_OK) return st;
         mesh_bounds(d->positions, d->num_vertices, m->bound_center, &m->bound_radius);
         m->bounds_pending = false;
         return AXR_OK;
+    }
+    if (recording(ctx)) {
+        // no bounds come of it (a replay tells the host nothing): planning keeps those of before
+        m->recorded_update = true;
+        return upload_mesh_arrays(ctx, m, d, nullptr);
     }
     if (!m->bounds_host) AXR_CUDA(ctx, cudaMallocHost(&m->bounds_host, sizeof(MeshBounds)));
     if (!m->bounds_ready) AXR_CUDA(ctx, cudaEventCreateWithFlags(&m->bounds_ready, cudaEventDisableTiming));

@@ -64,6 +64,9 @@ struct axr_mesh {
     mutable float bound_center[3] = {0.f, 0.f, 0.f};
     mutable float bound_radius = 0.f;
     mutable bool bounds_pending = false;
+    // an update was recorded into a graph, which may bring other positions at any time: the bounds
+    // serve planning only (density classes), no draw is taken for free of clipping by them
+    bool recorded_update = false;
     axr::MeshBounds* bounds_host = nullptr;  // pinned
     cudaEvent_t bounds_ready = nullptr;
 };

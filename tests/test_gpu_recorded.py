@@ -1,6 +1,7 @@
-"""Draws recorded into a graph: what a replay draws is decided by the vertices it finds on the device,
-which may cross the view volume although none did when it was recorded; and draws outside a graph, of a mesh whose
-bounds come from the device."""
+"""Draws and mesh updates recorded into a graph: what a replay draws is decided by the vertices it finds
+on the device, which may cross the view volume although none did when it was recorded, and an update that a
+graph may repeat at any time says nothing about the vertices of a later draw. And draws outside a graph, of a
+mesh whose bounds come from the device."""
 import dataclasses
 
 import numpy as np
@@ -8,6 +9,7 @@ import pytest
 
 from axiomr_gb300 import api
 from axiomr_gb300 import workloads as W
+from test_gpu_mesh_import import pin
 
 pytestmark = pytest.mark.gpu
 
@@ -67,6 +69,47 @@ def test_recorded_draw(ctx, lon, size, shader):
         g.launch()
         f.check(ctx, shift, "replayed")
     g.close()
+
+
+@pytest.mark.parametrize("lon", [32, 128])
+@pytest.mark.parametrize("pinned", [True, False])  # one kernel reads the arrays, or copies do
+def test_recorded_update(ctx, lon, pinned):
+    """An update recorded with the draw behind it, then a graph with the update alone and draws outside it."""
+    f = Frame(lon)
+    keep = [pin(a) if a is not None else (None, None) for a in f.pose(SHIFTS[0])]
+    pose = [k[0] for k in keep]
+    if not pinned:  # (a pageable copy cannot be recorded; one array a word off an aligned address can)
+        keep[2] = pin(pose[2], 4)
+        pose[2] = keep[2][0]
+    f.mesh.update(*pose)  # allocates what later updates need
+    f.draw()
+    f.ctx.sync()
+    both, alone = api.Graph(f.ctx), api.Graph(f.ctx)
+    both.begin()
+    f.mesh.update(*pose)
+    f.draw()
+    both.end()
+    alone.begin()
+    f.mesh.update(*pose)
+    alone.end()
+    cls = api.density_class(api.Draw(f.mesh, f.fb, api.Camera.from_workload(f.sc.camera), api.FlatShader()))
+    for shift in SHIFTS:
+        pose[0][...] = f.pose(shift)[0]
+        both.launch()
+        f.check(ctx, shift, "update and draw replayed")
+    for shift in SHIFTS:
+        pose[0][...] = f.pose(shift)[0]
+        alone.launch()
+        f.draw()
+        f.check(ctx, shift, "update replayed, then drawn")
+    # planning goes by the bounds known last, and a batch draws the mesh as it is
+    draw = api.Draw(f.mesh, f.fb, api.Camera.from_workload(f.sc.camera), api.Shader(f.sc.shader.kind, tuple(
+        f.sc.shader.light_direction), tuple(f.sc.shader.light_color)), f.sc.model, (0, 0, 0, 255), float("inf"))
+    assert api.density_class(draw) == cls
+    api.draw_batch(f.ctx, [draw])
+    f.check(ctx, SHIFTS[-1], "batch")
+    both.close()
+    alone.close()
 
 
 @pytest.mark.parametrize("lon", [130, 256])
