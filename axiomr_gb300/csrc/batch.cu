@@ -210,7 +210,7 @@ __device__ __forceinline__ uint32_t tile_scan(const DrawParams& p, const UnitInf
     }
     if (dirty && lane == 0) {
         t.tile_flag[c.tile] = 0u;
-        if (stats) {
+        if (stats && count) {
             atomicAdd(&counters->stat_tiles, 1ull);
             atomicAdd(&counters->stat_shaded, (unsigned long long)((count & 0xFFFFu) + (count >> 16)));
         }

@@ -121,7 +121,7 @@ struct DevCounters {
     unsigned long long stat_triangles;   // triangles that passed clip + cull
     unsigned long long stat_fragments;   // covered (triangle, pixel) pairs
     unsigned long long stat_large;       // triangles sent to the tile rasteriser
-    unsigned long long stat_tiles;       // dirty tiles resolved
+    unsigned long long stat_tiles;       // tiles with a depth key (a flagged tile may have none)
     unsigned long long stat_tested;      // (triangle, pixel) coverage tests evaluated
     unsigned long long stat_shaded;      // winning fragments shaded
 };

@@ -184,7 +184,7 @@ __global__ void __launch_bounds__(kBlock, tile_blocks(S)) tile_kernel(const __gr
     }
     __syncthreads();
     const uint32_t n = s_fill;
-    if (p.scratch.collect_stats && tid == 0) {
+    if (p.scratch.collect_stats && tid == 0 && n) {
         atomicAdd(&p.scratch.counters->stat_tiles, 1ull);
         atomicAdd(&p.scratch.counters->stat_shaded, (unsigned long long)n);
     }
@@ -264,7 +264,7 @@ __global__ void __launch_bounds__(kBlock, 6) scan_kernel(const __grid_constant__
             }
             if (lane == 0) {
                 t.tile_flag[first + (uint32_t)(warp * kScanTiles + k)] = 0u;
-                if (p.scratch.collect_stats) atomicAdd(&c->stat_tiles, 1ull);
+                if (p.scratch.collect_stats && count) atomicAdd(&c->stat_tiles, 1ull);
             }
         }
         if (p.scratch.collect_stats && lane == 0) atomicAdd(&c->stat_shaded, (unsigned long long)count);

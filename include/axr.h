@@ -615,7 +615,8 @@ typedef struct axr_draw_stats {
     uint64_t triangles;  /* triangles that survived clipping and culling */
     uint64_t fragments;  /* covered (triangle, pixel) pairs */
     uint64_t large;      /* triangles rasterised by the tile kernel */
-    uint64_t tiles;      /* 16x16 tiles resolved */
+    uint64_t tiles;      /* 16x16 tiles resolved: those in which a triangle covers a pixel
+                          * (binned forms: bins that a triangle reaches) */
     uint64_t tested;     /* (triangle, pixel) coverage tests evaluated */
     uint64_t shaded;     /* winning fragments shaded (covered pixels after the depth test) */
 } axr_draw_stats;

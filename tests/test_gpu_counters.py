@@ -1,0 +1,52 @@
+"""What the library counts and times: tiles with a covered pixel."""
+import numpy as np
+import pytest
+
+from axiomr_gb300 import api
+from axiomr_gb300 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+def covered_tiles(depth):
+    """16x16 tiles that hold a covered pixel of a frame cleared to infinity."""
+    h, w = depth.shape
+    d = np.zeros(((h + 15) // 16 * 16, (w + 15) // 16 * 16), bool)
+    d[:h, :w] = np.isfinite(depth)
+    return int(d.reshape(d.shape[0] // 16, 16, -1, 16).any(axis=(1, 3)).sum())
+
+
+# triangles of a pixel or two, many of which cover no pixel centre of their box, in frames of either tile
+# pass, from each form
+@pytest.mark.parametrize("size,count", [((640, 480), 400), ((1921, 1083), 3000)])
+@pytest.mark.parametrize("form", ["draw", "noalloc", api.BATCH_PHASED, api.BATCH_PERSISTENT])
+@pytest.mark.parametrize("depth_min", [1.0, 0.09])  # the latter: some cut by the near plane
+def test_tiles_with_a_covered_pixel(size, count, form, depth_min):
+    if form == "noalloc" and size[0] * size[1] > 1 << 20:
+        return  # beyond its limit
+    ctx = api.Context(0)
+    sc = W.soup_scene(count=count, width=size[0], height=size[1], seed=7, edge_min=0.5, edge_max=4.0, depth_min=depth_min,
+                      depth_max=0.5 if depth_min < 0.1 else 50.0)
+    sc.shader = W.Shader(W.SHADER_GOURAUD)
+    ctx.stats(True)
+    ctx.stats()
+    if form == "noalloc":
+        fb, mesh = api.Framebuffer(ctx, *size), api.Mesh.from_workload(ctx, sc.mesh)
+        fb.clearColor(0, 0, 0, 255)
+        fb.clearDepth()
+        api.TiledPipeline(ctx, api.Camera.from_workload(sc.camera), fb).setShader(api.GouraudShader())
+        model = np.ascontiguousarray(sc.model, np.float32)
+        api.check(ctx.lib.axr_draw_mesh_noalloc(ctx.handle, mesh.handle, model.ctypes.data), ctx.handle)
+        depth = fb.read()[1]
+    elif form == "draw":
+        ctx.draw_form = api.DRAW_KEYED
+        depth = api.render_scene(ctx, sc)[1]
+    else:
+        ctx.batch_form = form
+        draws = api.batch_draws(ctx, [sc])
+        api.draw_batch(ctx, draws)
+        depth = draws[0].framebuffer.read()[1]
+    stats = ctx.stats()
+    ctx.close()
+    assert stats["shaded"] == np.isfinite(depth).sum() > 0
+    assert stats["tiles"] == covered_tiles(depth)
