@@ -1231,7 +1231,7 @@ axr_status axr_profile_read(axr_context* ctx, axr_profile* out) {
     AXR_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     axr_profile r{};
     for (size_t k = 0; k + kStageEvents <= ctx->events_used; k += kStageEvents) {
-        double* out[6] = {&r.vertex_ms, &r.geometry_ms, &r.clipped_ms, &r.large_ms, &r.shade_ms, &r.scan_ms};
+        double* out[6] = {&r.vertex_ms, &r.geometry_ms, &r.clipped_ms, &r.large_ms, &r.scan_ms, &r.shade_ms};
         for (int j = 0; j < 6; ++j) {
             float ms = 0.f;
             AXR_CUDA(ctx, cudaEventElapsedTime(&ms, ctx->event_pool[k + j], ctx->event_pool[k + j + 1]));

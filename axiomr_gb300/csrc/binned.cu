@@ -92,12 +92,11 @@ cudaError_t launch_solo_s(const SoloBinned& sb, cudaStream_t stream, cudaEvent_t
     if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(1)) != cudaSuccess) return e;
     solo_face_kernel<<<blocks_for(sb.p.mesh.num_drawn), kBlock, 0, stream>>>(sb);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // stage events 2..4 (large, scan) have no kernel in this form
-    for (int k = 2; k <= 4; ++k)
+    // stages 2..4 (clip, large, scan) have no kernel in this form
+    for (int k = 2; k <= 5; ++k)
         if ((e = mark(k)) != cudaSuccess) return e;
     solo_bin_kernel<S><<<(unsigned)sb.bins.nbins, kBinThreads, 0, stream>>>(sb);
-    if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(5)) != cudaSuccess || (e = mark(6)) != cudaSuccess)
-        return e;
+    if ((e = cudaGetLastError()) != cudaSuccess || (e = mark(6)) != cudaSuccess) return e;
     *launches += 3;
     return cudaSuccess;
 }

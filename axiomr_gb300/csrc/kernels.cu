@@ -388,19 +388,23 @@ cudaError_t launch_shaded(const DrawParams& p, const LaunchConfig& cfg, cudaStre
     e = launch_dependent(large_kernel, (unsigned)(cfg.num_sms * cfg.large_ctas_per_sm), (unsigned)kBlock, stream, p);
     if (e != cudaSuccess || (e = mark(4)) != cudaSuccess) return e;
     const uint32_t tiles = (uint32_t)(p.target.tiles_x * p.target.tiles_y);
-    if (!scan_pass(tiles, cfg.num_sms)) {
-        e = clipped ? launch_dependent(tile_kernel<S, true>, tiles, (unsigned)kBlock, stream, p)
-                    : launch_dependent(tile_kernel<S, false>, tiles, (unsigned)kBlock, stream, p);
-    } else {
+    const bool scan = scan_pass(tiles, cfg.num_sms);
+    if (scan) {
         const unsigned scan_ctas = (tiles + kBlock / 32 * kScanTiles - 1) / (kBlock / 32 * kScanTiles);
         e = launch_dependent(scan_kernel, scan_ctas, (unsigned)kBlock, stream, p);
         if (e != cudaSuccess) return e;
         *launches += 1;
+    }
+    if ((e = mark(5)) != cudaSuccess) return e;
+    if (!scan) {
+        e = clipped ? launch_dependent(tile_kernel<S, true>, tiles, (unsigned)kBlock, stream, p)
+                    : launch_dependent(tile_kernel<S, false>, tiles, (unsigned)kBlock, stream, p);
+    } else {
         const unsigned shade_ctas = (unsigned)(cfg.num_sms * tile_blocks(S));
         e = clipped ? launch_dependent(shade_kernel<S, true>, shade_ctas, (unsigned)kBlock, stream, p)
                     : launch_dependent(shade_kernel<S, false>, shade_ctas, (unsigned)kBlock, stream, p);
     }
-    if (e != cudaSuccess || (e = mark(5)) != cudaSuccess) return e;
+    if (e != cudaSuccess) return e;
     *launches += clipped ? 5 : 4;
     return mark(6);
 }

@@ -22,14 +22,14 @@ struct LaunchConfig {
     bool clip_free = false;
 };
 
-// One draw: vertices, faces (clip classification, cull, setup, raster of the smaller boxes), the
-// clip pass, large-triangle tiles, tile pass (key scan, shading, merge). `stage_events` (optional,
-// kStageEvents events) are recorded before the first kernel and after each of vertex, geometry,
-// clip, large, tile (and once more). Adds the number of kernels launched to *launches.
 // Whether a draw into a frame of so many tiles lists its covered pixels in scratch.shade (a scan
 // and a shade kernel) instead of tile by tile in shared memory.
 bool scan_pass(uint32_t tiles, int num_sms);
 
+// One draw: vertices, faces (clip classification, cull, setup, raster of the smaller boxes), the
+// clip pass, large-triangle tiles, key scan (larger frames), shading and merge (the tile pass).
+// `stage_events` (optional, kStageEvents events) are recorded before the first kernel and after each of
+// these six stages. Adds the number of kernels launched to *launches.
 constexpr int kStageEvents = 7;
 cudaError_t launch_draw(const DrawParams& p, const LaunchConfig& cfg, cudaStream_t stream, cudaEvent_t* stage_events,
                         uint64_t* launches);

@@ -428,6 +428,9 @@ def run_ours(args, dist: Dist):
     P = scene.width * scene.height
     frags = st["fragments"]
     scanned_px = min(P, st["tiles"] * 256)
+    # the key scan is a kernel of its own above 30 tiles of 16x16 per SM
+    sms = torch.cuda.get_device_properties(dev).multi_processor_count
+    scans = -(-scene.width // 16) * -(-scene.height // 16) > 30 * sms
     vattr = {W.SHADER_PHONG: 64, W.SHADER_PBR: 64, W.SHADER_BLINN_PHONG: 32}.get(shader_kind, 16)
     vin = 40 + (24 if need_tbn else 0)  # position, normal, uv (+ tangent, bitangent) read per vertex
     algo_bytes = {
@@ -437,14 +440,18 @@ def run_ours(args, dist: Dist):
         # depth-key write per covered fragment
         "geometry": 12.0 * F + 16.0 * V + 8.0 * frags,
         "large": 8.0 * frags,
-        "scan": 0.0,  # part of the shade stage
-        # keys of the dirty tiles read; per covered pixel: indices, depth read, colour + depth
-        # write; the vertex cache read once
-        "shade": 8.0 * scanned_px + frags * (12.0 + 4.0 + 8.0) + float(V) * (16 + vattr),
+        # larger frames: keys of the dirty tiles read, one 8-byte work entry per covered pixel written;
+        # smaller ones read the keys in the shade stage
+        "scan": 8.0 * scanned_px + 8.0 * frags if scans else 0.0,
+        # per covered pixel: (work entry,) indices, depth read, colour + depth write; the vertex cache
+        # read once
+        "shade": (8.0 * frags if scans else 8.0 * scanned_px) + frags * (12.0 + 4.0 + 8.0) + float(V) * (16 + vattr),
         "clipped": 0.0,
     }
     kernel_names = {k: k + "_kernel" for k in stages}
     kernel_names["clipped"] = "clip_kernel"
+    if not scans:
+        kernel_names["shade"] = "tile_kernel"
     if args.draw_form == "binned":
         # three kernels: vertices, faces (setup and binning; the profile's geometry stage) and
         # bins (raster, shading and tile write-out; its shading stage). Algorithmic bytes: the

@@ -634,8 +634,9 @@ typedef struct axr_profile {
     double vertex_ms;        /* per-vertex transform and vertex shader */
     double geometry_ms;      /* cull, setup, raster of smaller boxes */
     double large_ms;         /* large-triangle tile raster */
-    double scan_ms;          /* 0: the key scan is part of shade_ms */
-    double shade_ms;         /* key scan, per-pixel resolve and shading */
+    double scan_ms;          /* key scan of larger frames (more than 30 tiles of 16x16 per SM); in
+                              * smaller ones it is part of shade_ms, and this the events' distance */
+    double shade_ms;         /* per-pixel resolve and shading */
     double clipped_ms;       /* clipper on faces that straddle the view volume */
     uint64_t kernel_launches;/* all kernels launched on this context since creation */
     uint64_t batch_launches; /* batched launches timed (including graph replays) */
