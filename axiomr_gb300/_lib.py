@@ -67,7 +67,7 @@ AXR_BATCH_PHASED = 1
 
 
 class BatchInfo(C.Structure):
-    _fields_ = [("draws", C.c_uint32), ("launches", C.c_uint32), ("form", C.c_int32), ("pad_", C.c_uint32),
+    _fields_ = [("draws", C.c_uint32), ("launches", C.c_uint32), ("form", C.c_int32), ("launch_sets", C.c_uint32),
                 ("vertices", C.c_uint64), ("faces", C.c_uint64),
                 ("pixels", C.c_uint64), ("tiles", C.c_uint64), ("device_bytes", C.c_uint64)]
 

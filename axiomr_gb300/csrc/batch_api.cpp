@@ -571,6 +571,7 @@ axr_status axr_batch_get_info(const axr_batch* b, axr_batch_info* out) {
     if (!b || !out) return fail(nullptr, AXR_E_INVALID, "NULL argument");
     out->draws = b->count;
     out->launches = b->launches.empty() ? 0u : b->kind_sets;
+    out->launch_sets = (uint32_t)b->launches.size();
     out->form = b->form;
     out->vertices = b->vertices;
     out->faces = b->faces;

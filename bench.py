@@ -914,12 +914,12 @@ def run_batch(args, dist: Dist):
         "form_desc": ("batched, binned: three launches over the work units of all draws (vertices; faces, "
                       "set up and binned into bins of 8 tiles; one CTA per bin rasterising it in shared memory, "
                       "shading the winners and writing colour and depth once with TMA stores, clears fused)"
-                      + (", as two launch sets of alternating draws on two streams" if info["launches"] > 1 else "")
+                      + (", as two launch sets of alternating draws on two streams" if info["launch_sets"] > 1 else "")
                       if info["form"] == 2 else
                       "batched, phased: four phase launches (the tile pass also clearing the key-less tiles "
                       "with TMA stores) over the work units of "
                       "all draws, as two launch sets of alternating draws on two streams"
-                      if info["form"] == 1 and info["launches"] > 1 else
+                      if info["form"] == 1 and info["launch_sets"] > 1 else
                       "batched, phased: four phase launches per step (the tile pass also clearing the "
                       "key-less tiles with TMA stores) over the work "
                       "units of all draws" if info["form"] == 1 else

@@ -403,10 +403,12 @@ int32_t axr_batch_get_form(const axr_context* ctx);
 
 typedef struct axr_batch_info {
     uint32_t draws;
-    uint32_t launches;        /* shader kinds times launch sets: one per shader kind, two for a
-                               * phased or binned batch of 128+ draws */
+    uint32_t launches;        /* (shader kind, half) pairs with draws: one per shader kind, two in a
+                               * phased or binned batch of 128+ draws; the phased form runs those of all
+                               * kinds together, see launch_sets */
     int32_t form;             /* AXR_BATCH_* the batch was planned for */
-    uint32_t pad_;
+    uint32_t launch_sets;     /* sets of kernels that axr_batch_launch enqueues: phased one (two for 128+
+                               * draws), the other forms one for each of `launches` */
     uint64_t vertices;        /* vertices of all draws */
     uint64_t faces;           /* faces in draw order of all draws */
     uint64_t pixels;          /* framebuffer pixels of all draws */

@@ -1,4 +1,5 @@
-"""What the library counts and times: tiles with a covered pixel, and the key scan's own time."""
+"""What the library counts and times: tiles with a covered pixel, the key scan's own time, and the launches of a
+batch."""
 import numpy as np
 import pytest
 
@@ -69,3 +70,28 @@ def test_scan_time():
     assert p["draws"] == 10
     print(p)
     assert p["scan_ms"] / 10 > 0.006 and p["shade_ms"] > 0.0
+
+
+KINDS = (W.SHADER_FLAT, W.SHADER_PHONG, W.SHADER_PBR, W.SHADER_BLINN_PHONG, W.SHADER_GOURAUD)
+
+
+# a phased batch runs all shader kinds in one launch set (two from 128 draws on), the others a set per kind
+@pytest.mark.parametrize("form,count,sets", [(api.BATCH_PHASED, 5, 1), (api.BATCH_PHASED, 130, 2), (api.BATCH_PERSISTENT, 5, 5),
+                                             (api.BATCH_PERSISTENT, 130, 5), (api.BATCH_BINNED, 5, 5), (api.BATCH_BINNED, 130, 10),
+                                             (api.BATCH_PHASED, 0, 0)])
+def test_launch_sets(form, count, sets):
+    ctx = api.Context(0)
+    base = {k: W.sphere_scene(width=64, height=48, lon=16, lat=8, tex_size=16, shader=k) for k in KINDS}
+    draws = api.batch_draws(ctx, [base[KINDS[k % 5]] for k in range(count)])
+    ctx.batch_form = form
+    batch = api.Batch(ctx, draws)
+    assert batch.info()["launch_sets"] == sets
+    before = ctx.profile()["kernel_launches"]
+    batch.launch()
+    ctx.sync()
+    # kernels per set: vertices, faces, large triangles, tiles; one; vertices, faces, bins. Two sets: their counts merged
+    per = {api.BATCH_PHASED: 4, api.BATCH_PERSISTENT: 1, api.BATCH_BINNED: 3}[form]
+    merges = 1 if count >= 128 and form != api.BATCH_PERSISTENT else 0
+    assert ctx.profile()["kernel_launches"] - before == sets * per + merges
+    batch.close()
+    ctx.close()
