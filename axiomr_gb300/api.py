@@ -90,7 +90,8 @@ class Context:
 
     def tuning(self) -> list:
         """The batched form's tuning table: per density class, the largest triangle pixel
-        box rasterised in the face phase."""
+        box rasterised in the face phase (256 where it was neither set nor tuned; smaller
+        batches are planned with less there)."""
         out = (C.c_int32 * AXR_TUNE_CLASSES)()
         check(self.lib.axr_batch_get_tuning(self.handle, out), self.handle)
         return list(out)

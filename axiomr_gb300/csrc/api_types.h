@@ -149,10 +149,11 @@ struct axr_context {
     uint32_t large_cap = 0, item_cap = 0, vcap = 0, px_cap = 0, rec_cap = 0;
     int collect_stats = 0;
     int small_max_pixels = 64;
-    // batched form: per density class, the largest pixel box rasterised in the face phase
-    // (autotuned; face_pixels bounds it in smaller batches), and the reusable plan of
-    // axr_draw_batch
+    // batched form: per density class, the largest pixel box rasterised in the face phase, and whether
+    // it was set or tuned (then it is used as it is; the default is bounded by face_pixels in
+    // smaller batches)
     int32_t tune_small[AXR_TUNE_CLASSES] = {256, 256, 256, 256, 256, 256};
+    bool tune_given[AXR_TUNE_CLASSES] = {};
     // binned batched form: bin parameters per density class (autotuned)
     axr_bin_params tune_bin[AXR_TUNE_CLASSES] = {{256, 4, 64, 2}, {256, 4, 64, 2}, {256, 4, 64, 2},
                                                  {256, 4, 64, 2}, {256, 4, 64, 2}, {256, 4, 64, 2}};
@@ -165,7 +166,7 @@ struct axr_context {
     float4* bin_crec = nullptr;
     uint32_t bin_count_cap = 0, crec_cap = 0;
     size_t bin_entry_cap = 0;
-    axr_batch* oneshot = nullptr;
+    axr_batch* oneshot = nullptr;  // the reusable plan of axr_draw_batch
     axr::BatchProfile* batch_prof = nullptr;  // device-side phase timing of persistent launches
     int batch_form = axr::kFormPhased;        // launch form of batches planned next
     std::vector<cudaEvent_t> batch_events;     // phase events of phased launches (6 per launch)

@@ -296,7 +296,9 @@ axr_status plan_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t coun
                                : DevScratch{d_counters[set], d_large[set], d_items[set], vscreen, vattr, nullptr,
                                             nullptr, nullptr, large_cap, item_cap, m->num_vertices, 0u, 0u, 0, 0,
                                             d_large_draw[set], rec};
-            p.small_max_pixels = std::min(ctx->tune_small[density_class(d)], face_pixels(faces, ctx->cfg.num_sms));
+            const int dc = density_class(d);
+            p.small_max_pixels = ctx->tune_small[dc];
+            if (!ctx->tune_given[dc]) p.small_max_pixels = std::min(p.small_max_pixels, face_pixels(faces, ctx->cfg.num_sms));
             p.draw = (uint32_t)k;
             if (binned) {
                 const BinPlanD& bp = bplan[(size_t)order[first + k]];
@@ -608,6 +610,7 @@ axr_status axr_batch_set_tuning(axr_context* ctx, const int32_t small_max_pixels
             return fail(ctx, AXR_E_INVALID, "class %d: pixel box limit %d (0..65536)", k, small_max_pixels[k]);
     std::lock_guard<std::mutex> lk(ctx->mu);
     std::memcpy(ctx->tune_small, small_max_pixels, sizeof(ctx->tune_small));
+    std::fill(ctx->tune_given, ctx->tune_given + AXR_TUNE_CLASSES, true);
     return AXR_OK;
 }
 
@@ -727,6 +730,7 @@ axr_status axr_batch_autotune(axr_context* ctx, const axr_draw_desc* draws, int3
         if (sub.empty()) continue;
         float best_ms = 0.f;
         int32_t best = ctx->tune_small[k];
+        ctx->tune_given[k] = true;
         for (int32_t cand : kCandidates) {
             ctx->tune_small[k] = cand;
             float ms = 0.f;

@@ -101,8 +101,8 @@ inline uint32_t face_share(uint64_t faces, int num_sms) {
     return n;
 }
 
-// Most pixels of a box that the face phase of a keyed batch of `faces` faces rasterises,
-// whatever the density classes allow: with few CTAs, those with large boxes outlast the others,
+// Most pixels of a box that the face phase of a keyed batch of `faces` faces rasterises where no
+// limit was set or tuned: with few CTAs, those with large boxes outlast the others,
 // while the large-triangle pass spreads such boxes over all SMs (20 small draws, 30k faces: 63
 // us at 64 pixels, 73 at 256; 30 mixed draws, 320k faces: 159 us at 96, 180 at 256; 512 mixed
 // draws, 5.4M faces, with their PNG files: 5.91 ms at 64, 5.50 at 256).

@@ -432,6 +432,10 @@ axr_status axr_draw_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t 
 #define AXR_TUNE_CLASSES 6
 axr_status axr_batch_autotune(axr_context* ctx, const axr_draw_desc* draws, int32_t count, int32_t repeats,
                               int32_t out_small_max_pixels[AXR_TUNE_CLASSES]);
+/* The table: limits of 0 to 65536 pixels. One that was set here or tuned is used as it is in every
+ * batch planned afterwards; a class that was neither reads 256, the default, which the planner bounds
+ * by 64 or 96 in batches of few faces. Boxes past what the face phase's tables hold (on
+ * average 256 pixels a face) are rasterised as larger ones whatever the limit. */
 axr_status axr_batch_get_tuning(const axr_context* ctx, int32_t small_max_pixels[AXR_TUNE_CLASSES]);
 axr_status axr_batch_set_tuning(axr_context* ctx, const int32_t small_max_pixels[AXR_TUNE_CLASSES]);
 /* Bin parameters per density class of the binned form (capacity 16..65536, never 0). */
