@@ -724,23 +724,30 @@ axr_status axr_batch_autotune(axr_context* ctx, const axr_draw_desc* draws, int3
         }
         ctx->batch_form = best;
     }
-    // the keyed forms' per-thread pixel-box limit per density class
-    for (int k = 0; k < AXR_TUNE_CLASSES && st == AXR_OK && ctx->batch_form != kFormBinned; ++k) {
-        const std::vector<axr_draw_desc>& sub = by_class[(size_t)k];
-        if (sub.empty()) continue;
+    // the keyed forms' pixel-box limit per density class, timed in the whole batch: what a limit is worth
+    // depends on how many CTAs the face phase has. A class keeps what it has unless a candidate makes the
+    // batch faster by more than such timings differ.
+    if (st == AXR_OK && ctx->batch_form != kFormBinned) {
         float best_ms = 0.f;
-        int32_t best = ctx->tune_small[k];
-        ctx->tune_given[k] = true;
-        for (int32_t cand : kCandidates) {
-            ctx->tune_small[k] = cand;
-            float ms = 0.f;
-            if ((st = time_plan(sub.data(), (int32_t)sub.size(), &ms)) != AXR_OK) break;
-            if (best_ms == 0.f || ms < best_ms) {
-                best_ms = ms;
-                best = cand;
+        st = time_plan(draws, count, &best_ms);
+        for (int k = 0; k < AXR_TUNE_CLASSES && st == AXR_OK; ++k) {
+            if (by_class[(size_t)k].empty()) continue;
+            int32_t best = ctx->tune_small[k];
+            bool given = ctx->tune_given[k];
+            ctx->tune_given[k] = true;
+            for (int32_t cand : kCandidates) {
+                ctx->tune_small[k] = cand;
+                float ms = 0.f;
+                if ((st = time_plan(draws, count, &ms)) != AXR_OK) break;
+                if (ms < 0.995f * best_ms) {
+                    best_ms = ms;
+                    best = cand;
+                    given = true;
+                }
             }
+            ctx->tune_small[k] = best;
+            ctx->tune_given[k] = given;
         }
-        ctx->tune_small[k] = best;
     }
     cudaStreamSynchronize(ctx->stream);
     free_batch(&trial);

@@ -421,10 +421,11 @@ axr_status axr_batch_get_info(const axr_batch* batch, axr_batch_info* out);
  * and launch it. Not for graph capture (the draw table is uploaded by this call). */
 axr_status axr_draw_batch(axr_context* ctx, const axr_draw_desc* draws, int32_t count);
 
-/* Autotuner. First the launch form, timing the whole batch in both forms. Then, per
- * density class, the largest triangle pixel box rasterised in the face phase (larger boxes go
- * to the warp-per-tile rasteriser), timing the sub-batch of the given draws in that class
- * with each candidate `repeats` times. A draw's density class is the estimated mean screen
+/* Autotuner. First the binned form's parameters per density class, on the sub-batch of the
+ * given draws in that class; then the launch form, timing the whole batch in each. Then, per density
+ * class, the largest triangle pixel box rasterised in the face phase (larger boxes go
+ * to the warp-per-tile rasteriser), timing the whole batch with each candidate `repeats` times;
+ * a class keeps its limit unless one is faster. A draw's density class is the estimated mean screen
  * area of its front-facing triangles, from the mesh's bounding sphere projected through
  * its camera: class k covers [2^(2k-1), 2^(2k+1)) pixels (class 0 below 2, the last class
  * 512 and above). The form and the table are the context's; batches planned afterwards

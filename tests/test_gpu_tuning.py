@@ -1,6 +1,7 @@
 """The batched form's pixel-box limits: a limit that was set is the one used, whatever the batch's size; and
 boxes that the pair tables of the face phase do not hold go to the large-triangle pass. The triangles sent there
-are counted from the clip stage's records by the face phase's rules."""
+are counted from the clip stage's records by the face phase's rules. And the autotuner times its limits in the
+batch that they are for."""
 import numpy as np
 import pytest
 import torch
@@ -93,3 +94,25 @@ def test_limit_is_used(port, form, limit):
 def test_pair_tables_overflow(port, form, limit, count, edge, edge_max):
     s = check(port, soup(count, edge, edge_max), limit, form)
     assert 0 < s["large"] <= s["triangles"]
+
+
+def test_autotune_times_the_whole_batch():
+    """Each launch of the search for the limits draws the whole batch. With one repeat every setting is launched twice:
+    the binned form's 21 a class, all classes together once the batch; three forms; the limits, five per class
+    of the batch and the table as it was."""
+    ctx = api.Context(0)
+    draws = api.batch_draws(ctx, W.batch_scenes(count=24, seed=5, tex_size=32, resolution_scale=0.25))
+    classes = len({api.density_class(d) for d in draws})
+    assert classes >= 3
+    ctx.batch_form = api.BATCH_PHASED
+    batch = api.Batch(ctx, draws)
+    ctx.stats(True)
+    ctx.stats()
+    batch.launch()
+    whole = ctx.stats()["triangles"]
+    api.autotune(ctx, draws, repeats=1)
+    launches = ctx.stats()["triangles"] / whole
+    assert ctx.batch_form != api.BATCH_BINNED  # its own search would end there
+    assert launches == 2 * (21 + 3 + 1 + 5 * classes)
+    batch.close()
+    ctx.close()
