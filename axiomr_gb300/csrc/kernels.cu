@@ -46,8 +46,6 @@ namespace {
 
 constexpr int kBlock = 256;
 constexpr int kClipBlock = 64;
-constexpr int kScanTiles = 1;  // tiles per warp and round of the scan kernel
-
 
 // Resident 128-thread CTAs per SM the geometry kernel is compiled for (register budget
 // 65536 / (128 * n)): 56 registers, the fewest without spills. Its gathers' latency is the bound (2M-triangle
@@ -191,83 +189,70 @@ __global__ void __launch_bounds__(kBlock, tile_blocks(S)) tile_kernel(const __gr
     if ((uint32_t)tid < n) shade_listed<S, kClip>(p, s_list[tid]);
 }
 
-// Key scan of a larger frame: kScanTiles tiles per warp and round, all their keys in flight at
-// once; the covered pixels are appended to the shade list, their keys and the tiles' flags
-// reset. List space is taken once per CTA round (a prefix over the warps), so the global counter
-// sees few atomics; the warps' counts are double-buffered, so that a round has two barriers.
+// Key scan of a larger frame: a tile per warp, all its keys in flight at once; the covered pixels are
+// appended to the shade list, their keys and the tile's flag reset. List space is taken once per CTA (a
+// prefix over the warps), so the global counter sees few atomics.
 // Bound by the keys' reads: many warps with a tile each hide them better than few with two (2M-triangle
 // terrain / 200k small triangles at 3840x2160, us a frame: one tile, 6 CTAs per SM 85.4 / 95.9; two, 3 CTAs
 // 86.2 / 97.5; two, 4 CTAs 86.5 / 95.0; one, 7 CTAs (spills) 89.4 / 103; four, 2 CTAs 87.5 / 102).
 __global__ void __launch_bounds__(kBlock, 6) scan_kernel(const __grid_constant__ DrawParams p) {
     constexpr int kWarps = kBlock / 32;
-    __shared__ uint32_t s_count[2][kWarps], s_base[2];
+    __shared__ uint32_t s_count[kWarps], s_base;
     DevCounters* c = p.scratch.counters;
     const DevTarget& t = p.target;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned below = (1u << lane) - 1u;
-    const uint32_t ntiles = (uint32_t)t.tiles_x * (uint32_t)t.tiles_y, per_round = kWarps * kScanTiles;
+    const uint32_t ntiles = (uint32_t)t.tiles_x * (uint32_t)t.tiles_y, tile = blockIdx.x * kWarps + (uint32_t)warp;
     pdl_wait();
     pdl_release();
-    int buf = 0;
-    for (uint32_t first = blockIdx.x * per_round; first < ntiles; first += gridDim.x * per_round, buf ^= 1) {
-        unsigned long long keys[kScanTiles][8];
-        uint32_t pos[kScanTiles], count = 0;
-        bool dirty[kScanTiles];
+    const bool dirty = tile < ntiles && ld_volatile(&t.tile_flag[tile]) != 0u;
+    const uint32_t pos = (tile % (uint32_t)t.tiles_x * kTile + (uint32_t)(lane & 15)) |
+                         (tile / (uint32_t)t.tiles_x * kTile + (uint32_t)(lane >> 4)) << 16;  // the lane's first pixel
+    unsigned long long keys[8];
+    uint32_t count = 0;
+    {
+        const uint32_t px = pos & 0xFFFFu, py = pos >> 16;
+        const unsigned long long* at = t.key + (size_t)py * (size_t)t.width + px;
 #pragma unroll
-        for (int k = 0; k < kScanTiles; ++k) {
-            const uint32_t tile = first + (uint32_t)(warp * kScanTiles + k);
-            dirty[k] = tile < ntiles && ld_volatile(&t.tile_flag[tile]) != 0u;
-            pos[k] = (tile % (uint32_t)t.tiles_x * kTile + (uint32_t)(lane & 15)) |
-                     (tile / (uint32_t)t.tiles_x * kTile + (uint32_t)(lane >> 4)) << 16;
+        for (int r = 0; r < 8; ++r) {
+            keys[r] = (dirty && px < (uint32_t)t.width && py + 2 * r < (uint32_t)t.height) ? __ldcg(at) : kEmptyKey;
+            at += 2 * (size_t)t.width;
         }
+    }
+    if (dirty) {
 #pragma unroll
-        for (int k = 0; k < kScanTiles; ++k) {
-            const uint32_t px = pos[k] & 0xFFFFu, py = pos[k] >> 16;
-            const unsigned long long* at = t.key + (size_t)py * (size_t)t.width + px;
+        for (int r = 0; r < 8; ++r) count += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, keys[r] != kEmptyKey));
+    }
+    if (lane == 0) s_count[warp] = count;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
 #pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                keys[k][r] = (dirty[k] && px < (uint32_t)t.width && py + 2 * r < (uint32_t)t.height) ? __ldcg(at) : kEmptyKey;
-                at += 2 * (size_t)t.width;
-            }
+    for (int w = 0; w < kWarps; ++w) {
+        const uint32_t v = s_count[w];
+        if (w < warp) before += v;
+        total += v;
+    }
+    if (threadIdx.x == 0 && total) s_base = atomicAdd(&c->shade_count, total);
+    __syncthreads();
+    if (!dirty) return;
+    uint32_t at = s_base + before;
+    unsigned long long* key = t.key + (size_t)(pos >> 16) * (size_t)t.width + (pos & 0xFFFFu);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) {
+        const bool has = keys[r] != kEmptyKey;
+        const unsigned m = __ballot_sync(0xFFFFFFFFu, has);
+        if (has) {
+            p.scratch.shade[at + (uint32_t)__popc(m & below)] = make_uint2(pos + ((uint32_t)(2 * r) << 16), (uint32_t)keys[r]);
+            key[(size_t)(2 * r) * (size_t)t.width] = kEmptyKey;  // for the next draw
         }
-#pragma unroll
-        for (int k = 0; k < kScanTiles; ++k)
-            if (dirty[k]) {
-#pragma unroll
-                for (int r = 0; r < 8; ++r) count += (uint32_t)__popc(__ballot_sync(0xFFFFFFFFu, keys[k][r] != kEmptyKey));
-            }
-        if (lane == 0) s_count[buf][warp] = count;
-        __syncthreads();
-        uint32_t before = 0, total = 0;
-#pragma unroll
-        for (int w = 0; w < kWarps; ++w) {
-            const uint32_t v = s_count[buf][w];
-            if (w < warp) before += v;
-            total += v;
+        at += (uint32_t)__popc(m);
+    }
+    if (lane == 0) {
+        t.tile_flag[tile] = 0u;
+        if (p.scratch.collect_stats && count) {
+            atomicAdd(&c->stat_tiles, 1ull);
+            atomicAdd(&c->stat_shaded, (unsigned long long)count);
         }
-        if (threadIdx.x == 0 && total) s_base[buf] = atomicAdd(&c->shade_count, total);
-        __syncthreads();
-        uint32_t at = s_base[buf] + before;
-#pragma unroll
-        for (int k = 0; k < kScanTiles; ++k) {
-            if (!dirty[k]) continue;
-            unsigned long long* key = t.key + (size_t)(pos[k] >> 16) * (size_t)t.width + (pos[k] & 0xFFFFu);
-#pragma unroll
-            for (int r = 0; r < 8; ++r) {
-                const bool has = keys[k][r] != kEmptyKey;
-                const unsigned m = __ballot_sync(0xFFFFFFFFu, has);
-                if (has) {
-                    p.scratch.shade[at + (uint32_t)__popc(m & below)] = make_uint2(pos[k] + ((uint32_t)(2 * r) << 16), (uint32_t)keys[k][r]);
-                    key[(size_t)(2 * r) * (size_t)t.width] = kEmptyKey;  // for the next draw
-                }
-                at += (uint32_t)__popc(m);
-            }
-            if (lane == 0) {
-                t.tile_flag[first + (uint32_t)(warp * kScanTiles + k)] = 0u;
-                if (p.scratch.collect_stats && count) atomicAdd(&c->stat_tiles, 1ull);
-            }
-        }
-        if (p.scratch.collect_stats && lane == 0) atomicAdd(&c->stat_shaded, (unsigned long long)count);
     }
 }
 
@@ -390,8 +375,7 @@ cudaError_t launch_shaded(const DrawParams& p, const LaunchConfig& cfg, cudaStre
     const uint32_t tiles = (uint32_t)(p.target.tiles_x * p.target.tiles_y);
     const bool scan = scan_pass(tiles, cfg.num_sms);
     if (scan) {
-        const unsigned scan_ctas = (tiles + kBlock / 32 * kScanTiles - 1) / (kBlock / 32 * kScanTiles);
-        e = launch_dependent(scan_kernel, scan_ctas, (unsigned)kBlock, stream, p);
+        e = launch_dependent(scan_kernel, grid_for(tiles, kBlock / 32, 0x7FFFFFFFu), (unsigned)kBlock, stream, p);
         if (e != cudaSuccess) return e;
         *launches += 1;
     }
