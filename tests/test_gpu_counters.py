@@ -1,5 +1,5 @@
-"""What the library counts and times: tiles with a covered pixel, the key scan's own time, and the launches of a
-batch."""
+"""What the library counts and times: tiles with a covered pixel, the key scan's own time, the launches of a
+batch, and work that repeats exactly when a batch is launched again."""
 import numpy as np
 import pytest
 
@@ -93,5 +93,24 @@ def test_launch_sets(form, count, sets):
     per = {api.BATCH_PHASED: 4, api.BATCH_PERSISTENT: 1, api.BATCH_BINNED: 3}[form]
     merges = 1 if count >= 128 and form != api.BATCH_PERSISTENT else 0
     assert ctx.profile()["kernel_launches"] - before == sets * per + merges
+    batch.close()
+    ctx.close()
+
+
+@pytest.mark.parametrize("count,scale", [(1, 0.1), (24, 0.1), (130, 0.05)])
+@pytest.mark.parametrize("form", [api.BATCH_PHASED, api.BATCH_PERSISTENT])
+def test_work_repeats(count, scale, form):
+    ctx = api.Context(0)
+    draws = api.batch_draws(ctx, W.batch_scenes(count=count, seed=11, tex_size=32, resolution_scale=scale))
+    ctx.batch_form = form
+    batch = api.Batch(ctx, draws)
+    ctx.stats(True)
+    ctx.stats()
+    batch.launch()
+    once = ctx.stats()
+    assert all(once[k] > 0 for k in ("triangles", "fragments", "tiles", "tested", "shaded"))
+    for _ in range(20):
+        batch.launch()
+    assert ctx.stats() == {k: 20 * v for k, v in once.items()}
     batch.close()
     ctx.close()
