@@ -105,7 +105,7 @@ __device__ int clip_plane(int plane, CV& v0, CV& v1, CV& v2, CV& v3) {
 // exact up to about 6 * 4 roundings of 2^-24 of the largest coordinates (1.5e-6), stays
 // positive and the plane keeps every triangle unchanged. A NaN or infinite coordinate fails
 // the comparison (and keeps the plane).
-__device__ __forceinline__ uint32_t idle_planes(const f4& c0, const f4& c1, const f4& c2) {
+static __device__ __noinline__ uint32_t idle_planes(const f4& c0, const f4& c1, const f4& c2) {
     const f4 c[3] = {c0, c1, c2};
     float mag = 0.0f;
 #pragma unroll
