@@ -674,8 +674,8 @@ axr_status axr_mesh_create(axr_context* ctx, const axr_mesh_desc* d, axr_mesh** 
     return AXR_OK;
 }
 
-// Above this many vertices axr_mesh_update computes the bounds on the device (five small
-// stream operations cost about as much as a host pass over 8k vertices).
+// Above this many vertices axr_mesh_update computes the bounds on the device (a second kernel
+// and an event cost about as much as a host pass over 8k vertices).
 constexpr uint32_t kHostBoundsMaxVertices = 8192;
 
 axr_status axr_mesh_update(axr_context* ctx, axr_mesh* m, const axr_mesh_desc* d) {

@@ -5,9 +5,10 @@
 // so the draws share nothing but the GPU, and one launch walks four phases over the
 // work units of all draws, separated by grid barriers:
 //   1. vertices   256-vertex units of every draw: screen cache + vertex-shader outputs
-//   2. faces      256-face units in draw order: clip, cull, setup, small-triangle raster;
-//                 large triangles go to one shared list with one item per 16x16 tile
-//   3. large      warps take items of the shared list (4 per atomic), any draw
+//   2. faces      units of faces in draw order (256; in the phased form up to 128): clip, cull, setup,
+//                 raster of the smaller boxes; large triangles go to one shared list with one
+//                 item per 16x16 tile
+//   3. large      warps take items of the shared list, strided over the grid, any draw
 //   4. tiles      tile units, one warp per 16x16 tile: a warp reads the tile's depth keys,
 //                 shades the winners (compacted across the warp through shared memory),
 //                 and writes the whole tile once. A draw that asks for a clear gets it
@@ -38,13 +39,13 @@ constexpr int kBatchMinBlocks = 3;  // 256 threads x 3 CTAs: at most 85 register
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;
 
 // Resident 128-thread CTAs per SM the phased face kernel is compiled for (8: at most 64
-// registers; its shared memory, 13 KB per CTA, allows more).
+// registers; its shared memory, 16.9 KB per CTA, allows 13).
 #ifndef AXR_FACE_MIN_BLOCKS
 #define AXR_FACE_MIN_BLOCKS 8
 #endif
 
 // Resident 256-thread CTAs per SM the phased tile kernel is compiled for (4: at most 64
-// registers; its shared memory, 36 KB per CTA, allows 6).
+// registers; its shared memory, 39.7 KB per CTA, allows 5).
 #ifndef AXR_TILE_MIN_BLOCKS
 #define AXR_TILE_MIN_BLOCKS 4
 #endif

@@ -102,10 +102,13 @@ inline uint32_t face_share(uint64_t faces, int num_sms) {
 }
 
 // Most pixels of a box that the face phase of a keyed batch of `faces` faces rasterises where no
-// limit was set or tuned: with few CTAs, those with large boxes outlast the others,
-// while the large-triangle pass spreads such boxes over all SMs (20 small draws, 30k faces: 63
-// us at 64 pixels, 73 at 256; 30 mixed draws, 320k faces: 159 us at 96, 180 at 256; 512 mixed
-// draws, 5.4M faces, with their PNG files: 5.91 ms at 64, 5.50 at 256).
+// limit was set or tuned: with few CTAs, those with large boxes outlast the others, while the large-triangle
+// pass spreads such boxes over all SMs. The lines lie at 4 and 64 CTAs of faces per SM (78k and 1.2M faces);
+// the draws' resolution moves the best limit as well, so they are compromises that the
+// autotuner betters. A step in us at limits of 64 / 96 / 256, phased: 90k faces 81 / 88 / 92, 326k 161 / 157 /
+// 172, 660k 379 / 362 / 340, at a quarter of the resolution 86 / 86 / 94, 1.2M 747 / 721 / 678, at a quarter
+// 143 / 141 / 145, 5.4M 3,223 / 3,156 / 2,883. Persistent: 90k 216 / 208 / 217, 326k 466 / 455 / 471, 660k 908 /
+// 880 / 857, at a quarter 284 / 283 / 293, 1.2M 1,764 / 1,700 / 1,601, 5.4M 7,130 / 6,949 / 6,461.
 inline int32_t face_pixels(uint64_t faces, int num_sms) {
     const uint64_t ctas = faces / kPhasedFaceUnit;
     return ctas < 4ull * (uint64_t)num_sms ? 64 : ctas < 64ull * (uint64_t)num_sms ? 96 : INT32_MAX;

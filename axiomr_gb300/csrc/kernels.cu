@@ -17,7 +17,7 @@
 //                    clip volume go to a list
 //   clip_kernel      one thread per listed face: the exact clipper, its output triangles
 //                    rasterised or queued as above; not launched when the mesh's bounding sphere
-//                    shows that no face can be clipped
+//                    shows that no face can be clipped (never left out of a recorded draw)
 //   large_kernel     warps take tile work items and evaluate 256 pixels each, 8 per lane
 //   tile_kernel      a CTA per flagged tile: its covered pixels (non-empty depth keys) are
 //                    listed and their keys reset, then one thread per covered pixel re-derives

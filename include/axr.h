@@ -174,10 +174,13 @@ axr_status axr_mesh_counts(const axr_mesh* mesh, uint32_t* vertices, uint32_t* f
 axr_status axr_mesh_create(axr_context* ctx, const axr_mesh_desc* desc, axr_mesh** out);
 /* Re-upload vertex attributes and indices of an existing mesh with the same counts,
  * asynchronously on the context stream (host buffers must stay valid until then;
- * pinned memory from axr_host_alloc makes the copies truly asynchronous). The mesh's
- * bounding sphere, used to plan batches, is recomputed from the new positions (on the
- * device for meshes above 8,192 vertices). Do not update a mesh while another context
- * plans or draws with it. */
+ * pinned memory from axr_host_alloc makes the copies truly asynchronous; arrays that all lie
+ * wholly in pinned memory, 16-byte aligned, are read from there by a kernel). The mesh's
+ * bounding sphere, used to plan batches and to leave the clip pass out of draws that
+ * need none, is recomputed from the new positions (on the
+ * device for meshes above 8,192 vertices). An update recorded into a graph reads the host
+ * buffers at every replay; the mesh's bounds then serve planning only. Do not update a mesh
+ * while another context plans or draws with it. */
 axr_status axr_mesh_update(axr_context* ctx, axr_mesh* mesh, const axr_mesh_desc* desc);
 void axr_mesh_destroy(axr_context* ctx, axr_mesh* mesh);
 
@@ -557,7 +560,8 @@ const char* axr_server_last_error(axr_server* srv);
 
 /* ------------------------------------------------------------------ CUDA graphs
  * Record the draws issued on the context between begin and end into a CUDA graph and
- * replay it. Per-draw scratch must be reserved (axr_reserve) and batches planned
+ * replay it. Cameras, shaders and model matrices are those of the recording; a replay draws
+ * the vertices it finds on the device. Per-draw scratch must be reserved (axr_reserve) and batches planned
  * (axr_batch_create) beforehand. */
 typedef struct axr_graph axr_graph;
 axr_status axr_graph_begin(axr_context* ctx);
