@@ -39,13 +39,13 @@ constexpr int kBatchMinBlocks = 3;  // 256 threads x 3 CTAs: at most 85 register
 constexpr unsigned long long kBarrierTimeoutNs = 2000000000ull;
 
 // Resident 128-thread CTAs per SM the phased face kernel is compiled for (8: at most 64
-// registers; its shared memory, 16.9 KB per CTA, allows 13).
+// registers; its shared memory, 16.9 KB per CTA, allows 9 and more).
 #ifndef AXR_FACE_MIN_BLOCKS
 #define AXR_FACE_MIN_BLOCKS 8
 #endif
 
 // Resident 256-thread CTAs per SM the phased tile kernel is compiled for (4: at most 64
-// registers; its shared memory, 39.7 KB per CTA, allows 5).
+// registers; its shared memory, 39.7 KB per CTA, allows 5 at most).
 #ifndef AXR_TILE_MIN_BLOCKS
 #define AXR_TILE_MIN_BLOCKS 4
 #endif
