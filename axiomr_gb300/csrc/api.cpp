@@ -228,7 +228,7 @@ axr_status check_mesh_desc(axr_context* ctx, const axr_mesh_desc* d) {
 }
 
 // The device's address of an array that the GPU may read in place (readable_in_place); NULL for anything
-// else. The range comes from the driver, which knows each allocation's and registration's extent.
+// else. The range comes from CUDA's driver, which knows each allocation's and registration's extent.
 template <class T>
 const T* pinned(const T* p, size_t bytes) {
     static std::once_flag once;
